@@ -104,9 +104,10 @@ void assign_tiles(Geometry& G, int target_tile_voxels) {
   for (int t = 0; t < G.n_tiles; t++) G.tile_c0[t] = G.rows[(size_t)t * tr].r0;
   G.ctrl_tiles.resize(nD);
   for (int c = 0; c < nD; c++) {
-    int a = (int)(std::lower_bound(G.tile_c0.begin(), G.tile_c0.end(), c - 2) - G.tile_c0.begin());
-    int b = (int)(std::upper_bound(G.tile_c0.begin(), G.tile_c0.end(), c) - G.tile_c0.begin());
-    G.ctrl_tiles[c] = make_int2(a, b);
+    auto first_at_least = [&](int r) {
+      return (int)(std::lower_bound(G.tile_c0.begin(), G.tile_c0.end(), r) - G.tile_c0.begin());
+    };
+    G.ctrl_tiles[c] = make_int4(first_at_least(c - 2), first_at_least(c - 1), first_at_least(c), first_at_least(c + 1));
   }
 }
 
@@ -333,7 +334,7 @@ fa_status retile(fa_reference* R, int target_tile_voxels) {
   cudaStream_t s = R->stream;
   FA_CU(cudaMemcpyAsync(R->tile_c0_dev, R->G.tile_c0.data(), R->G.tile_c0.size() * sizeof(int),
                         cudaMemcpyHostToDevice, s));
-  FA_CU(cudaMemcpyAsync(R->ctrl_dev, R->G.ctrl_tiles.data(), R->G.ctrl_tiles.size() * sizeof(int2),
+  FA_CU(cudaMemcpyAsync(R->ctrl_dev, R->G.ctrl_tiles.data(), R->G.ctrl_tiles.size() * sizeof(int4),
                         cudaMemcpyHostToDevice, s));
   FA_CU(cudaMemcpyAsync(R->dev, &R->host, sizeof(RefDev), cudaMemcpyHostToDevice, s));
   FA_CU(cudaStreamSynchronize(s));
@@ -544,7 +545,7 @@ fa_status reference_setup(fa_reference* R, const float* src, bool src_device) {
   h.tune_mb_small = 2;
   RowDesc* rows;
   int* tile_c0;
-  int2* ctrl;
+  int4* ctrl;
   float *ref32, *gx, *gy, *gz;
   double *Hd, *Hl, *tparts, *scan_dev;
   FA_TRY(dalloc_t(ctx, G.rows.size(), &rows, R->allocs));
@@ -567,7 +568,7 @@ fa_status reference_setup(fa_reference* R, const float* src, bool src_device) {
   cudaStream_t s = R->stream;
   FA_CU(cudaMemcpyAsync(rows, G.rows.data(), G.rows.size() * sizeof(RowDesc), cudaMemcpyHostToDevice, s));
   FA_CU(cudaMemcpyAsync(tile_c0, G.tile_c0.data(), G.tile_c0.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-  FA_CU(cudaMemcpyAsync(ctrl, G.ctrl_tiles.data(), G.ctrl_tiles.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
+  FA_CU(cudaMemcpyAsync(ctrl, G.ctrl_tiles.data(), G.ctrl_tiles.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
   FA_CU(cudaMemcpyAsync(ref32, src, (size_t)N * sizeof(float), src_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
   FA_CU(fa::launch_sobel(ref32, R->nz, R->ny, R->nx, gx, gy, gz, s));
   h.rows = rows;
@@ -1715,7 +1716,7 @@ extern "C" fa_status fa_test_tr_subproblem(fa_context* ctx, int nD, int n_dim, c
   if ((st = dalloc_t(ctx, hl.size(), &dHl, tmp)) != FA_OK) return done(st);
   if ((st = dalloc_t(ctx, (size_t)P, &dg, tmp)) != FA_OK) return done(st);
   if ((st = dalloc_t(ctx, (size_t)P, &dp, tmp)) != FA_OK) return done(st);
-  if ((st = dalloc_t(ctx, (size_t)P * (2 * n_dim) + 3 * (size_t)P, &work, tmp)) != FA_OK) return done(st);
+  if ((st = dalloc_t(ctx, 2 * ((size_t)P * (2 * n_dim)) + 4 * (size_t)P, &work, tmp)) != FA_OK) return done(st);
   if ((st = dalloc_t(ctx, 1, &db, tmp)) != FA_OK) return done(st);
   cudaError_t e = cudaMemcpy(dHd, hd.data(), hd.size() * sizeof(double), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dHl, hl.data(), hl.size() * sizeof(double), cudaMemcpyHostToDevice);

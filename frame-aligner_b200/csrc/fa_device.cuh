@@ -122,51 +122,75 @@ __device__ __forceinline__ float sample(const FT* __restrict__ fr, long long fpl
 
 constexpr int kWin = 5;  // control points [c0-1, c0+4) cover every interval a tile can touch
 
-// f = sum over tiles (thread-strided runs, then a fixed tree); g[c] = sum over the tiles listed in
-// ctrl_tiles[c], in tile order.
-__device__ __forceinline__ void reduce_partials(const RefDev& R, const double* __restrict__ parts, double* f_out, double* g_out) {
-  __shared__ double sf[kSolveThreads];
-  double acc = 0.0;
-  for (int t = threadIdx.x; t < R.n_tiles; t += blockDim.x) acc += parts[(long long)t * kPartialDoubles];
-  sf[threadIdx.x] = acc;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sf[threadIdx.x] += sf[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *f_out = sf[0];
-  const int nd = R.n_dim;
-  for (int i = threadIdx.x; i < R.P; i += blockDim.x) {
-    const int c = i / nd, k = i % nd;
-    const int2 tr = R.ctrl_tiles[c];
-    double a = 0.0;
-#pragma unroll 8
-    for (int t = tr.x; t < tr.y; t++) {
-      const double* pt = parts + (long long)t * kPartialDoubles;
-      const int s = c - R.tile_c0[t];
-      const double v = (s >= 0 && s < 3) ? pt[2 + s * 3 + k] : 0.0;
-      a += v;
+// f = sum over tiles (kReduceRuns strided runs, then a fixed tree); g[i] = sum over the tiles that hold
+// parameter i, in tile order. The first kReduceRuns threads of the block take f, the others g. What
+// bounds it is the latency of the loads, which no sum depends on: every thread has kReduceDepth of
+// them in flight, and the slot of a control point in a tile follows from the three bounds of
+// ctrl_tiles instead of a load per tile. f_out (shared memory) is valid, and g_out written, after the
+// closing barrier.
+constexpr int kReduceDepth = 16;
+__device__ __forceinline__ void reduce_partials(const RefDev& R, const double* __restrict__ parts, double* f_out,
+                                                double* g_out) {
+  __shared__ double sf[kReduceRuns];
+  const int tid = threadIdx.x;
+  if (tid < kReduceRuns) {
+    double acc = 0.0;
+    for (int t = tid; t < R.n_tiles; t += kReduceRuns * kReduceDepth) {
+      double v[kReduceDepth];
+#pragma unroll
+      for (int u = 0; u < kReduceDepth; u++) {
+        const int tt = t + u * kReduceRuns;
+        v[u] = tt < R.n_tiles ? __ldcg(parts + (long long)tt * kPartialDoubles) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kReduceDepth; u++) acc += v[u];  // + 0.0 leaves a sum that started at 0.0 as it is
     }
-    g_out[i] = a;
+    sf[tid] = acc;
+  } else {
+    const int nd = R.n_dim;
+    for (int i = tid - kReduceRuns; i < R.P; i += blockDim.x - kReduceRuns) {
+      const int c = i / nd, k = i - c * nd;
+      const int4 tr = R.ctrl_tiles[c];
+      double a = 0.0;
+      for (int t = tr.x; t < tr.w; t += kReduceDepth) {
+        double v[kReduceDepth];
+#pragma unroll
+        for (int u = 0; u < kReduceDepth; u++) {
+          const int tt = t + u;
+          const int s = tt < tr.y ? 2 : (tt < tr.z ? 1 : 0);
+          v[u] = tt < tr.w ? __ldcg(parts + (long long)tt * kPartialDoubles + 2 + s * 3 + k) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kReduceDepth; u++) a += v[u];
+      }
+      g_out[i] = a;
+    }
+  }
+  __syncthreads();
+  if (tid < 32) {  // the tree: run t takes run t + w, w = 64, 32, ..., 1
+    double a = (sf[tid] + sf[tid + 64]) + (sf[tid + 32] + sf[tid + 96]);
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) a += __shfl_down_sync(0xffffffffu, a, w);
+    if (tid == 0) *f_out = a;
   }
   __syncthreads();
 }
 
-// Control-point parameters (kDParamF4 float4 per control point) of the trial point D = x + p, from
-// job.x and job.p; control points k = t0, t0 + stride, ...
-__device__ __forceinline__ void write_trial_dparams(const Job& job, const RefDev& R, int t0, int stride) {
-  const int nd = R.n_dim;
-  for (int k = t0; k < R.nD; k += stride) {
+// Control-point parameters (kDParamF4 float4 per control point) of the trial point D = x + p; control
+// points k = t0, t0 + stride, ...
+__device__ __forceinline__ void write_trial_dparams(float4* dparams, const double* x, const double* p, int nD, int nd,
+                                                    int t0, int stride) {
+  for (int k = t0; k < nD; k += stride) {
     double d[3], dn[3];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
-      d[c] = c < nd ? job.x[k * nd + c] + job.p[k * nd + c] : 0.0;
-      dn[c] = (c < nd && k + 1 < R.nD) ? job.x[(k + 1) * nd + c] + job.p[(k + 1) * nd + c] : d[c];
+      d[c] = c < nd ? x[k * nd + c] + p[k * nd + c] : 0.0;
+      dn[c] = (c < nd && k + 1 < nD) ? x[(k + 1) * nd + c] + p[(k + 1) * nd + c] : d[c];
     }
     const double f0 = floor(d[0]), f1 = floor(d[1]), f2 = floor(d[2]);
-    job.dparams[k * kDParamF4 + 0] = make_float4((float)f0, (float)f1, (float)f2, 0.f);
-    job.dparams[k * kDParamF4 + 1] = make_float4((float)(d[0] - f0), (float)(d[1] - f1), (float)(d[2] - f2), 0.f);
-    job.dparams[k * kDParamF4 + 2] =
-        make_float4((float)(dn[0] - d[0]), (float)(dn[1] - d[1]), (float)(dn[2] - d[2]), 0.f);
+    dparams[k * kDParamF4 + 0] = make_float4((float)f0, (float)f1, (float)f2, 0.f);
+    dparams[k * kDParamF4 + 1] = make_float4((float)(d[0] - f0), (float)(d[1] - f1), (float)(d[2] - f2), 0.f);
+    dparams[k * kDParamF4 + 2] = make_float4((float)(dn[0] - d[0]), (float)(dn[1] - d[1]), (float)(dn[2] - d[2]), 0.f);
   }
 }
 

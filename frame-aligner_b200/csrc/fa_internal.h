@@ -95,7 +95,9 @@ struct RefDev {
   int tune_mb_small;   // the same for launches of one or a few frames (single-frame, static-scratch, serving)
   const RowDesc* rows;
   const int* tile_c0;      // per tile: storage range index of its first voxel
-  const int2* ctrl_tiles;  // per control point: tiles [x, y) whose partial slots may hold it
+  // Per control point c the tiles whose partial sums hold it: its own slot is 2 in [x, y) (tiles that
+  // start at range c - 2), 1 in [y, z) and 0 in [z, w).
+  const int4* ctrl_tiles;
   const float* ref32;
   const float* gx32;
   const float* gy32;

@@ -474,7 +474,9 @@ cudaError_t launch_eval(const Job* jobs_dev, int n_jobs, int max_tiles, int n_di
 
 __global__ void __launch_bounds__(kSolveThreads) reduce_kernel(const Job* __restrict__ job) {
   const RefDev& R = *job->ref;
-  reduce_partials(R, job->partials, job->result, job->result + 1);
+  __shared__ double s_f;
+  reduce_partials(R, job->partials, &s_f, job->result + 1);
+  if (threadIdx.x == 0) job->result[0] = s_f;
 }
 
 cudaError_t launch_reduce(const Job* job_dev, const RefDev&, cudaStream_t s) {
@@ -613,7 +615,7 @@ __global__ void hessian_reduce_kernel(const RefDev* __restrict__ Rp, const doubl
   if (c >= R.nD) return;
   double d[NDIM * NDIM], l[NDIM * NDIM];
   for (int i = 0; i < NDIM * NDIM; i++) d[i] = l[i] = 0.0;
-  const int t0 = max(0, R.ctrl_tiles[c].x), t1 = R.ctrl_tiles[c].y;
+  const int t0 = R.ctrl_tiles[c].x, t1 = R.ctrl_tiles[c].w;
   for (int t = t0; t < t1; t++) {
     const int ct = R.tile_c0[t];
     for (int s = 0; s < 2; s++) {
@@ -686,7 +688,7 @@ __global__ void __launch_bounds__(1024) compact_kernel(const Job* __restrict__ j
       if (*S->warm_seq == S->warm_need) {
         const RefDev& R = *j.ref;
         for (int q = 0; q < R.P; q++) j.p[q] = S->warm[q] - j.x[q];
-        write_trial_dparams(j, R, 0, 1);
+        write_trial_dparams(j.dparams, j.x, j.p, R.nD, R.n_dim, 0, 1);
         S->phase = kPhaseStartLast;
         phase = kPhaseStartLast;
       }

@@ -9,7 +9,10 @@ namespace fa {
 
 constexpr int kEvalThreads = 256;
 constexpr int kEvalWarps = kEvalThreads / 32;
-constexpr int kSolveThreads = 128;
+// The reduction and solve CTAs: kReduceRuns threads sum f in as many strided runs, the others one
+// parameter each.
+constexpr int kReduceRuns = 128;
+constexpr int kSolveThreads = 256;
 
 // Exact float Sobel3d (Sobel3d.cpp:60-85) of an FP32 volume.
 cudaError_t launch_sobel(const float* m, int nz, int ny, int nx, float* gx, float* gy, float* gz,

@@ -53,7 +53,7 @@ struct Geometry {
   long long lmin;
   int tile_rows, n_tiles;
   std::vector<int> tile_c0;
-  std::vector<int2> ctrl_tiles;
+  std::vector<int4> ctrl_tiles;
 };
 
 }  // namespace fa_rt
@@ -74,7 +74,7 @@ struct fa_reference {
   fa_scan_params scan{};
   fa_rt::Geometry G;
   int* tile_c0_dev = nullptr;
-  int2* ctrl_dev = nullptr;
+  int4* ctrl_dev = nullptr;
   std::vector<double> hd, hl;  // host copies of the Hessian blocks (diagonal, sub-diagonal)
   fa::RefDev host{};
   fa::RefDev* dev = nullptr;

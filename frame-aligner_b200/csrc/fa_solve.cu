@@ -44,31 +44,48 @@ struct Band {
 // L_ij accumulates A_ij (+ lambda) minus L_ik L_jk over ascending k -- the previous block's columns
 // first, then the earlier columns of its own block -- which is the dense algorithm's order (its
 // other terms are exact zeros). inv[i] = 1 / L_ii; off-diagonal entries multiply by it.
+//
+// One thread runs this and the two substitutions below: each is a chain of dependent FP64 operations
+// whose order is fixed. What one block needs of the previous one stays in registers, and the next
+// block's matrix entries are loaded while the current block computes, so that the chain waits for
+// arithmetic only, not for a store and a load per row.
 template <int ND>
-__device__ int band_chol(const Band<ND>& B, double lambda, double* L, double* inv) {
+__device__ __forceinline__ int band_chol(const Band<ND>& B, double lambda, double* __restrict__ L,
+                                         double* __restrict__ inv) {
   constexpr int NN = ND * ND;
-  double C[ND][ND];   // L rows of block b, columns of block b-1
-  double Dg[ND][ND];  // L rows of block b, its own columns (lower triangle)
-  double Dp[ND][ND];  // previous block's own-column L (rows of block b-1)
+  double Dp[ND][ND];  // previous block's own-column L (rows of block b-1), lower triangle
+  double ip[ND];      // and its reciprocal diagonal
+  double hd[NN], hl[NN];
 #pragma unroll
-  for (int r = 0; r < ND; r++)
+  for (int i = 0; i < NN; i++) {
+    hd[i] = B.Hd[i];
+    hl[i] = 0.0;
+    Dp[i / ND][i % ND] = 0.0;
+  }
 #pragma unroll
-    for (int c = 0; c < ND; c++) Dp[r][c] = 0.0;
+  for (int r = 0; r < ND; r++) ip[r] = 0.0;
   for (int b = 0; b < B.nD; b++) {
-    const double* hd = B.Hd + b * NN;
-    const double* hl = B.Hl + b * NN;
-    const int i0 = b * ND;
-    if (b > 0) {
+    double hdn[NN], hln[NN];
+    if (b + 1 < B.nD) {
 #pragma unroll
-      for (int r = 0; r < ND; r++)
-#pragma unroll
-        for (int c = 0; c < ND; c++) {
-          double s = hl[r * ND + c];
-#pragma unroll
-          for (int k = 0; k < c; k++) s -= C[r][k] * Dp[c][k];
-          C[r][c] = s * inv[i0 - ND + c];
-        }
+      for (int i = 0; i < NN; i++) {
+        hdn[i] = B.Hd[(b + 1) * NN + i];
+        hln[i] = B.Hl[(b + 1) * NN + i];
+      }
     }
+    const int i0 = b * ND;
+    double C[ND][ND];   // L rows of block b, columns of block b-1
+    double Dg[ND][ND];  // L rows of block b, its own columns (lower triangle)
+    double ic[ND];
+#pragma unroll
+    for (int r = 0; r < ND; r++)
+#pragma unroll
+      for (int c = 0; c < ND; c++) {
+        double s = hl[r * ND + c];
+#pragma unroll
+        for (int k = 0; k < c; k++) s -= C[r][k] * Dp[c][k];
+        C[r][c] = b > 0 ? s * ip[c] : 0.0;
+      }
 #pragma unroll
     for (int r = 0; r < ND; r++) {
 #pragma unroll
@@ -84,9 +101,10 @@ __device__ int band_chol(const Band<ND>& B, double lambda, double* L, double* in
           if (!(s > 0.0)) return -1;
           const double d = sqrt(s);
           Dg[r][r] = d;
-          inv[i0 + r] = 1.0 / d;
+          ic[r] = 1.0 / d;
+          inv[i0 + r] = ic[r];
         } else {
-          Dg[r][c] = s * inv[i0 + c];
+          Dg[r][c] = s * ic[c];
         }
       }
     }
@@ -96,50 +114,136 @@ __device__ int band_chol(const Band<ND>& B, double lambda, double* L, double* in
       double* row = L + (i0 + r) * 2 * ND;
 #pragma unroll
       for (int c = 0; c < ND; c++) {
-        row[c] = b > 0 ? C[r][c] : 0.0;
+        row[c] = C[r][c];
         row[ND + c] = c <= r ? Dg[r][c] : 0.0;
         Dp[r][c] = c <= r ? Dg[r][c] : 0.0;
       }
+      ip[r] = ic[r];
+    }
+#pragma unroll
+    for (int i = 0; i < NN; i++) {
+      hd[i] = hdn[i];
+      hl[i] = hln[i];
     }
   }
   return 0;
 }
 
-// L y = b by block rows (ascending k per entry, as the dense forward substitution).
+// One block's rows of the factor, their reciprocal diagonal and right-hand side.
 template <int ND>
-__device__ void band_forward(const Band<ND>& B, const double* L, const double* inv, const double* b, double* y) {
-  for (int blk = 0; blk < B.nD; blk++) {
-    const int i0 = blk * ND;
+struct FwdBlock {
+  double c[ND][ND], d[ND][ND], inv[ND], b[ND];
+  __device__ __forceinline__ void load(const double* __restrict__ L, const double* __restrict__ iv,
+                                       const double* __restrict__ rhs, int blk) {
 #pragma unroll
     for (int r = 0; r < ND; r++) {
-      const double* row = L + (i0 + r) * 2 * ND;
-      double s = b[i0 + r];
+      const double* row = L + (blk * ND + r) * 2 * ND;
+#pragma unroll
+      for (int k = 0; k < ND; k++) c[r][k] = row[k];
+#pragma unroll
+      for (int k = 0; k < r; k++) d[r][k] = row[ND + k];
+      inv[r] = iv[blk * ND + r];
+      b[r] = rhs[blk * ND + r];
+    }
+  }
+};
+
+// L y = b by block rows (ascending k per entry, as the dense forward substitution). y may be b.
+template <int ND>
+__device__ __forceinline__ void band_forward(const Band<ND>& B, const double* __restrict__ L,
+                                             const double* __restrict__ inv, const double* b, double* y) {
+  double yp[ND];
+  FwdBlock<ND> A, N;
+  auto step = [&](const FwdBlock<ND>& f, int blk) {
+    double yc[ND];
+#pragma unroll
+    for (int r = 0; r < ND; r++) {
+      double s = f.b[r];
       if (blk > 0) {
 #pragma unroll
-        for (int k = 0; k < ND; k++) s -= row[k] * y[i0 - ND + k];
+        for (int k = 0; k < ND; k++) s -= f.c[r][k] * yp[k];
       }
 #pragma unroll
-      for (int k = 0; k < r; k++) s -= row[ND + k] * y[i0 + k];
-      y[i0 + r] = s * inv[i0 + r];
+      for (int k = 0; k < r; k++) s -= f.d[r][k] * yc[k];
+      yc[r] = s * f.inv[r];
+    }
+#pragma unroll
+    for (int r = 0; r < ND; r++) {
+      y[blk * ND + r] = yc[r];
+      yp[r] = yc[r];
+    }
+  };
+#pragma unroll
+  for (int r = 0; r < ND; r++) yp[r] = 0.0;
+  A.load(L, inv, b, 0);
+  for (int blk = 0; blk < B.nD; blk += 2) {
+    if (blk + 1 < B.nD) N.load(L, inv, b, blk + 1);
+    step(A, blk);
+    if (blk + 1 < B.nD) {
+      if (blk + 2 < B.nD) A.load(L, inv, b, blk + 2);
+      step(N, blk + 1);
     }
   }
 }
 
-// L^T x = y by block rows from the end (ascending k per entry, as the dense back substitution).
+// One block of the back substitution: its own columns below the diagonal, the next block's rows of
+// this block's columns, reciprocal diagonal and right-hand side.
 template <int ND>
-__device__ void band_backward(const Band<ND>& B, const double* L, const double* inv, const double* y, double* x) {
-  for (int blk = B.nD - 1; blk >= 0; blk--) {
-    const int i0 = blk * ND;
+struct BwdBlock {
+  double c[ND][ND], d[ND][ND], inv[ND], b[ND];  // c[k][r] = L(next block row k, column r), d[k][r] = L(row k, r)
+  __device__ __forceinline__ void load(const double* __restrict__ L, const double* __restrict__ iv,
+                                       const double* __restrict__ y, int blk, bool next) {
+#pragma unroll
+    for (int k = 0; k < ND; k++) {
+      const double* row = L + (blk * ND + k) * 2 * ND;
+#pragma unroll
+      for (int r = 0; r < k; r++) d[k][r] = row[ND + r];
+      if (next) {
+#pragma unroll
+        for (int r = 0; r < ND; r++) c[k][r] = row[ND * 2 * ND + r];
+      }
+      inv[k] = iv[blk * ND + k];
+      b[k] = y[blk * ND + k];
+    }
+  }
+};
+
+// L^T x = y by block rows from the end (ascending k per entry, as the dense back substitution). x may
+// be y.
+template <int ND>
+__device__ __forceinline__ void band_backward(const Band<ND>& B, const double* __restrict__ L,
+                                              const double* __restrict__ inv, const double* y, double* x) {
+  double xn[ND];
+  BwdBlock<ND> A, N;
+  const int last = B.nD - 1;
+  auto step = [&](const BwdBlock<ND>& f, int blk) {
+    double xc[ND];
 #pragma unroll
     for (int r = ND - 1; r >= 0; r--) {
-      double s = y[i0 + r];
+      double s = f.b[r];
 #pragma unroll
-      for (int k = r + 1; k < ND; k++) s -= L[(i0 + k) * 2 * ND + ND + r] * x[i0 + k];
-      if (blk + 1 < B.nD) {
+      for (int k = r + 1; k < ND; k++) s -= f.d[k][r] * xc[k];
+      if (blk < last) {
 #pragma unroll
-        for (int k = 0; k < ND; k++) s -= L[(i0 + ND + k) * 2 * ND + r] * x[i0 + ND + k];
+        for (int k = 0; k < ND; k++) s -= f.c[k][r] * xn[k];
       }
-      x[i0 + r] = s * inv[i0 + r];
+      xc[r] = s * f.inv[r];
+    }
+#pragma unroll
+    for (int r = 0; r < ND; r++) {
+      x[blk * ND + r] = xc[r];
+      xn[r] = xc[r];
+    }
+  };
+#pragma unroll
+  for (int r = 0; r < ND; r++) xn[r] = 0.0;
+  A.load(L, inv, y, last, false);
+  for (int blk = last; blk >= 0; blk -= 2) {
+    if (blk >= 1) N.load(L, inv, y, blk - 1, true);
+    step(A, blk);
+    if (blk >= 1) {
+      if (blk >= 2) A.load(L, inv, y, blk - 2, true);
+      step(N, blk - 1);
     }
   }
 }
@@ -257,302 +361,483 @@ __device__ double predicted(const Band<ND>& B, const double* g, const double* p)
   return -(gp + 0.5 * pHp);
 }
 
-// Start a new trust-region iteration if the stop rule allows it. Returns false when done.
-template <int ND>
-__device__ bool loop_top(FrameState* S, const Band<ND>& B, const double* g, double* p, double* work) {
-  if (S->max_iter > 0 && S->iter >= S->max_iter) {
-    S->hit_max = 1;
-    return false;
+// ------------------------------------------------------------------ the whole block ---------------
+//
+// What a step needs one thread for is the chain of the two substitutions (3 and up to 7 dependent FP64
+// operations a row); everything else is per parameter. The sums whose rounding the algorithm fixes (the
+// norms and the predicted reduction) only feed comparisons: they are formed in parallel with an error
+// bound, and the ordered sum is taken by one thread only when the bound does not decide the
+// comparison. The steps taken are those of the ordered sums, bit for bit.
+
+// How far a sum over P parameters may lie from the ordered one, relative to the sum of magnitudes
+// (each order is within P * 2^-53 of the exact sum).
+__device__ __forceinline__ double sum_tol(int P) { return 1e-12 + P * 1e-15; }
+
+// Sums of up to three values over the block; every thread gets them. red: 3 doubles per warp, shared.
+template <int N>
+__device__ __forceinline__ void block_sums(double (&v)[N], double* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+  __syncthreads();  // earlier readers of red are done; the callers' shared stores are visible after the next
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < N; i++) red[w * 3 + i] = v[i];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    double a = 0.0;
+    for (int k = 0; k < nw; k++) a += red[k * 3 + i];
+    v[i] = a;
   }
-  if (S->have_prev && fabs(S->f - S->f_prev) < kMinDelta) return false;
-  S->have_prev = 1;
-  S->f_prev = S->f;
-  S->iter++;
-  S->boundary = subproblem(B, g, S->radius, 0.1, 20, p, work);
-  return true;
 }
 
-}  // namespace
+// subproblem by the whole block (g visible to every thread; p visible to every thread on return). An
+// interior step -- the first factorisation's (lambda = 0) step inside the radius -- takes the two
+// substitutions with the reference's cached factor; anything else goes to subproblem on one thread.
+// flag: one int, shared.
+template <int ND>
+__device__ __forceinline__ int subproblem_block(const Band<ND>& B, const double* g, double radius, double eps,
+                                                int max_iter, double* p, double* work, double* red, int* flag) {
+  const int P = B.P;
+  double* y = work + P * 2 * ND + P;
+  double* rhs = y + P;
+  double gg[1] = {0.0};
+  for (int i = threadIdx.x; i < P; i += blockDim.x) {
+    rhs[i] = -g[i];
+    gg[0] += g[i] * g[i];
+  }
+  block_sums(gg, red);
+  if (gg[0] == 0.0) {  // squares are not negative: the ordered norm is zero exactly when this sum is
+    for (int i = threadIdx.x; i < P; i += blockDim.x) p[i] = 0.0;
+    __syncthreads();
+    return 0;
+  }
+  if (B.L0 != nullptr && B.chol0_ok != 0 && max_iter > 0) {
+    if (threadIdx.x == 0) {
+      band_forward<ND>(B, B.L0, B.inv0, rhs, y);
+      band_backward<ND>(B, B.L0, B.inv0, y, p);
+    }
+    __syncthreads();
+    double pp[1] = {0.0};
+    for (int i = threadIdx.x; i < P; i += blockDim.x) pp[0] += p[i] * p[i];
+    block_sums(pp, red);
+    if (pp[0] < radius * radius * (1.0 - 4.0 * sum_tol(P))) return 0;  // |p| <= radius for certain
+  }
+  if (threadIdx.x == 0) *flag = subproblem<ND>(B, g, radius, eps, max_iter, p, work);
+  __syncthreads();
+  const int r = *flag;
+  __syncthreads();
+  return r;
+}
 
-// Doubles of shared memory one frame's solve uses when staged: Hessian blocks, band factor,
-// 1/L_ii, two work vectors, g and p, and a copy of the reference's cached factor of H (and its 1/L_ii),
-// which the serial chain of every interior step reads.
+// The ratio test of a trial point: measured reduction meas over the predicted reduction, as the ordered
+// sums decide it. Returns bits: 1 the solve ends, 2 rho < 1/4, 4 rho > 3/4, 8 rho > 0.
+__device__ __forceinline__ int ratio_bits(double pred, double meas) {
+  if (fabs(pred) <= fabs(meas) * kDblEps) return 1;
+  const double rho = meas / fabs(pred);
+  if (!isfinite(rho)) return 1;
+  return (rho < 0.25 ? 2 : 0) | (rho > 0.75 ? 4 : 0) | (rho > 0 ? 8 : 0);
+}
+
+template <int ND>
+__device__ __forceinline__ int ratio_block(const Band<ND>& B, const double* g, const double* p, double meas,
+                                           double* red, int* flag) {
+  constexpr int NN = ND * ND;
+  double v[3] = {0.0, 0.0, 0.0};  // g.p, p.H.p, the sum of their terms' magnitudes
+  for (int i = threadIdx.x; i < B.P; i += blockDim.x) {
+    const int b = i / ND, a = i - b * ND;
+    double s = 0, m = 0;
+    auto term = [&](double h, double q) {
+      s += h * q;
+      m += fabs(h * q);
+    };
+    if (b > 0) {
+#pragma unroll
+      for (int c = 0; c < ND; c++) term(B.Hl[b * NN + a * ND + c], p[(b - 1) * ND + c]);
+    }
+#pragma unroll
+    for (int c = 0; c < ND; c++) term(B.Hd[b * NN + a * ND + c], p[b * ND + c]);
+    if (b + 1 < B.nD) {
+#pragma unroll
+      for (int c = 0; c < ND; c++) term(B.Hl[(b + 1) * NN + c * ND + a], p[(b + 1) * ND + c]);
+    }
+    v[0] += g[i] * p[i];
+    v[1] += p[i] * s;
+    v[2] += fabs(g[i] * p[i]) + 0.5 * fabs(p[i]) * m;
+  }
+  block_sums(v, red);
+  const double pred = -(v[0] + 0.5 * v[1]), rel = sum_tol(B.P), tol = rel * v[2];
+  const double lo = fabs(pred) - tol, hi = fabs(pred) + tol;
+  if (lo > 0.0 && isfinite(hi) && isfinite(meas) && fabs(meas) > 1e-200 && fabs(meas) < 1e200 && hi < 1e200 &&
+      lo > 1e-200 && lo > 2.0 * fabs(meas) * kDblEps) {
+    // the ordered sum lies in [lo, hi]: decided when both ends give the same answer
+    const int b0 = ratio_bits(lo * (1.0 - rel), meas), b1 = ratio_bits(hi * (1.0 + rel), meas);
+    if (b0 == b1) return b0;
+  }
+  if (threadIdx.x == 0) *flag = ratio_bits(predicted<ND>(B, g, p), meas);
+  __syncthreads();
+  const int r = *flag;
+  __syncthreads();
+  return r;
+}
+
+// Doubles of shared memory one frame's solve uses when staged: Hessian blocks, g, p, x and the trial
+// gradient, band factor, 1/L_ii and two work vectors, and a copy of the reference's cached factor of H
+// and its 1/L_ii, which the chain of every interior step reads.
 __host__ __device__ inline long long solve_smem_doubles(int nD, int nd) {
   const long long P = (long long)nD * nd;
-  return 2LL * nD * nd * nd + 2 * (P * 2 * nd) + 6 * P;
+  return 2LL * nD * nd * nd + 2 * (P * 2 * nd) + 8 * P;
 }
 
-// The trust-region state machine for one frame after a fused pass at its trial point (thread 0).
+// The trust-region state machine for one frame after a fused pass at its trial point, by the whole
+// block. S (shared) is the frame's state; gt the gradient at the trial point, in p the rigid point's
+// gradient in the paired start.
 template <int ND>
-__device__ void state_step(const Job& job, FrameState* S, const RefDev& R, const double* Hd, const double* Hl,
-                           const double* L0, const double* inv0, double* gv, double* pv, double* work, double ft,
-                           double ft2) {
-  const int P = R.P, nd = ND;
-  Band<ND> B{Hd, Hl, R.nD, P, R.h_inf, R.h_mindiag, L0, inv0, R.chol0_ok};
-  double* x = job.x;
-  double* g = gv;
-  double* p = pv;
-  const double* gt = job.gt;
-  bool go_top = false, done = false;
+__device__ __forceinline__ void state_step(FrameState& S, const Band<ND>& B, double* x, double* g, double* p,
+                                           const double* gt, double* work, double ft, double ft2, double* red,
+                                           int* flag) {
+  const int P = B.P, t0 = threadIdx.x, nt = blockDim.x;
+  const bool lead = threadIdx.x == 0;
+  const int phase = S.phase;
+  const bool warm = S.use_warm && S.warm != nullptr;
+  bool go_top = false, done = false, top = false;
   int next = kPhaseTrial;
-  S->evaluations++;
-  switch (S->phase) {
+  const double f0 = S.f, f_start = S.f_start;
+  double radius = S.radius, f = f0;
+  int evaluations = S.evaluations + 1, accepted = S.accepted;
+  double f_zero = f_start;
+  __syncthreads();  // every thread has read the state
+  switch (phase) {
     case kPhaseStartZero: {
-      S->f_start = ft;
-      for (int i = 0; i < P; i++) g[i] = gt[i];
+      f_zero = ft;
+      for (int i = t0; i < P; i += nt) g[i] = gt[i];
       bool rigid = false;
-      for (int c = 0; c < nd; c++) rigid = rigid || (S->rigid[c] != 0.0);
+#pragma unroll
+      for (int c = 0; c < ND; c++) rigid = rigid || (S.rigid[c] != 0.0);
       if (rigid) {
-        for (int k = 0; k < R.nD; k++)
-          for (int c = 0; c < nd; c++) p[k * nd + c] = S->rigid[c];
+        for (int i = t0; i < P; i += nt) p[i] = S.rigid[i % ND];
         next = kPhaseStartRigid;
       } else {
-        S->f = ft;
-        if (S->use_warm && S->warm != nullptr) {
+        f = ft;
+        if (warm)
           next = kPhaseWaitWarm;
-        } else {
+        else
           go_top = true;
-        }
       }
       break;
     }
     case kPhaseStartPair: {
       // Both cold starting points from one pass: ft, gt at zero; ft2 and (in p) its gradient at the
       // rigid shift. The same choice as kPhaseStartZero followed by kPhaseStartRigid.
-      S->evaluations++;
-      S->f_start = ft;
+      evaluations++;
+      f_zero = ft;
       if (ft2 < ft) {
-        for (int k = 0; k < R.nD; k++)
-          for (int c = 0; c < nd; c++) {
-            x[k * nd + c] = S->rigid[c];
-            g[k * nd + c] = p[k * nd + c];
-          }
-        S->f = ft2;
+        for (int i = t0; i < P; i += nt) {
+          x[i] = S.rigid[i % ND];
+          g[i] = p[i];
+        }
+        f = ft2;
       } else {
-        for (int i = 0; i < P; i++) g[i] = gt[i];
-        S->f = ft;
+        for (int i = t0; i < P; i += nt) g[i] = gt[i];
+        f = ft;
       }
-      if (S->use_warm && S->warm != nullptr) {
+      if (warm)
         next = kPhaseWaitWarm;
-      } else {
+      else
         go_top = true;
-      }
       break;
     }
     case kPhaseStartRigid: {
       // Starting points {0, 0, rigid}: std::min_element keeps the first minimum
       // (FrameWarpAligner.cpp:194-198).
-      if (ft < S->f_start) {
-        for (int i = 0; i < P; i++) {
+      if (ft < f_start) {
+        for (int i = t0; i < P; i += nt) {
           x[i] = p[i];
           g[i] = gt[i];
         }
-        S->f = ft;
+        f = ft;
       } else {
-        S->f = S->f_start;
+        f = f_start;
       }
-      if (S->use_warm && S->warm != nullptr) {
-        // the warm start waits (out of the passes) until the earlier frame's solution is written;
-        // the compact pass then sets p = warm - x and the trial point
+      // a warm start waits (out of the passes) until the earlier frame's solution is written; the
+      // compact pass then sets p = warm - x and the trial point
+      if (warm)
         next = kPhaseWaitWarm;
-      } else {
+      else
         go_top = true;
-      }
       break;
     }
     case kPhaseStartLast: {
       // Warm start: the previous frame's solution as a fourth starting point after {0, 0, rigid};
       // only a strictly smaller value replaces the current start (first minimum kept). The trial
       // point was x + (warm - x), and that is the point taken.
-      if (ft < S->f) {
-        for (int i = 0; i < P; i++) {
+      if (ft < f0) {
+        for (int i = t0; i < P; i += nt) {
           x[i] = x[i] + p[i];
           g[i] = gt[i];
         }
-        S->f = ft;
+        f = ft;
       }
       go_top = true;
       break;
     }
     case kPhaseTrial: {
-      const double pred = predicted(B, g, p);
-      const double meas = S->f - ft;
-      if (fabs(pred) <= fabs(meas) * kDblEps) {
+      const int r = ratio_block<ND>(B, g, p, f0 - ft, red, flag);
+      if (r & 1) {
         done = true;
         break;
       }
-      const double rho = meas / fabs(pred);
-      if (!isfinite(rho)) {
-        done = true;
-        break;
-      }
-      if (rho < 0.25) {
-        S->radius *= 0.25;
-        if (S->radius <= kRadius0 * kDblEps) {
+      if (r & 2) {
+        radius *= 0.25;
+        if (radius <= kRadius0 * kDblEps) {
           done = true;
           break;
         }
-      } else if (rho > 0.75 && S->boundary) {
-        S->radius = 2 * S->radius < kRadiusMax ? 2 * S->radius : kRadiusMax;
+      } else if ((r & 4) && S.boundary) {
+        radius = 2 * radius < kRadiusMax ? 2 * radius : kRadiusMax;
       }
-      if (rho > 0) {
-        for (int i = 0; i < P; i++) {
+      if (r & 8) {
+        for (int i = t0; i < P; i += nt) {
           x[i] = x[i] + p[i];
           g[i] = gt[i];
         }
-        S->f = ft;
-        S->accepted++;
+        f = ft;
+        accepted++;
       }
-      if (!loop_top(S, B, g, p, work)) done = true;
+      top = true;
       break;
     }
     default:
       done = true;
   }
+  __syncthreads();  // x, g, p as this phase leaves them
+  int iter = S.iter, have_prev = S.have_prev, hit_max = S.hit_max, boundary = S.boundary;
+  double f_prev = S.f_prev;
   if (go_top) {
-    for (int i = 0; i < P; i++) p[i] = 0.0;
-    S->radius = kRadius0;
-    S->iter = 0;
-    S->have_prev = 0;
-    if (!loop_top(S, B, g, p, work)) done = true;
+    radius = kRadius0;
+    iter = 0;
+    have_prev = 0;
+    for (int i = t0; i < P; i += nt) p[i] = 0.0;
+    __syncthreads();
   }
-  S->phase = done ? kPhaseDone : next;
+  if (go_top || top) {
+    // a new trust-region iteration, if the stop rules allow it
+    if (S.max_iter > 0 && iter >= S.max_iter) {
+      hit_max = 1;
+      done = true;
+    } else if (have_prev && fabs(f - f_prev) < kMinDelta) {
+      done = true;
+    } else {
+      have_prev = 1;
+      f_prev = f;
+      iter++;
+      boundary = subproblem_block<ND>(B, g, radius, 0.1, 20, p, work, red, flag);
+    }
   }
+  __syncthreads();  // every thread is done with the old state
+  if (lead) {
+    S.f = f;
+    S.f_start = f_zero;
+    S.f_prev = f_prev;
+    S.radius = radius;
+    S.iter = iter;
+    S.accepted = accepted;
+    S.evaluations = evaluations;
+    S.have_prev = have_prev;
+    S.boundary = boundary;
+    S.hit_max = hit_max;
+    S.phase = done ? kPhaseDone : next;
+  }
+  __syncthreads();
+}
 
-__global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const Job* __restrict__ jobs, int smem_cap_doubles,
+static_assert(sizeof(Job) % 8 == 0 && sizeof(FrameState) % 8 == 0 && sizeof(RefDev) % 8 == 0, "copied by words");
+template <typename T>
+__device__ __forceinline__ void copy_words(T* dst, const T* src) {
+  for (int i = threadIdx.x; i < (int)(sizeof(T) / 8); i += blockDim.x)
+    reinterpret_cast<unsigned long long*>(dst)[i] = __ldcg(reinterpret_cast<const unsigned long long*>(src) + i);
+}
+
+// One trust-region step of one frame per CTA. The step is latency: a few rounds of dependent loads
+// (job, then reference and state, then everything they point at, brought into shared memory when it
+// fits), the tile reduction, and the chain of two substitutions; a pass over the frame takes
+// longer only for volumes. The chain was the whole step before it ran from registers with its loads
+// ahead of it and without the ordered norms (mean over the steps of a solve, before -> after: 22.9 ->
+// 9.2 us for a 512 x 512 plane with nD = 32, 58 -> 21 us for 512 x 512 x 16 with nD = 32, 261 -> 90 us
+// for 1024 x 1024 x 64 with nD = 64).
+template <int ND, bool STAGED>
+__global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const Job* __restrict__ jobs,
                                                                  const int* __restrict__ active,
                                                                  const int* __restrict__ n_active) {
   extern __shared__ double s_dyn[];
+  __shared__ Job job;
+  __shared__ RefDev R;
+  __shared__ FrameState S;
+  __shared__ double s_f, s_f2, s_red[3 * (kSolveThreads / 32)];
+  __shared__ int s_flag;
   if (active != nullptr && (int)blockIdx.x >= *n_active) return;
-  const Job& job = jobs[active != nullptr ? active[blockIdx.x] : blockIdx.x];
-  FrameState* S = job.state;
-  if (S->phase == kPhaseDone || S->phase == kPhaseWaitWarm) return;
-  const RefDev& R = *job.ref;
-  __shared__ double s_f, s_f2;
-  reduce_partials(R, job.partials, &s_f, job.gt);
-  // paired start: the rigid point's sums, its gradient into p (free until the first step)
-  const bool pair = S->phase == kPhaseStartPair;
-  if (pair) reduce_partials(R, job.partials2, &s_f2, job.p);
+  copy_words(&job, jobs + (active != nullptr ? active[blockIdx.x] : blockIdx.x));
   __syncthreads();
-  // Stage the Hessian blocks, g and p in shared memory when they fit; otherwise work in global.
-  const int nn = R.n_dim * R.n_dim;
-  const bool staged = solve_smem_doubles(R.nD, R.n_dim) <= smem_cap_doubles;
-  const double* Hd = R.Hd;
-  const double* Hl = R.Hl;
-  double* work = job.work;
-  double* gv = job.g;
-  double* pv = job.p;
-  const double* L0 = R.L0;
-  const double* inv0 = R.inv0;
-  if (staged) {
+  copy_words(&S, job.state);
+  copy_words(&R, job.ref);
+  __syncthreads();
+  if (S.phase == kPhaseDone || S.phase == kPhaseWaitWarm) return;
+  const bool pair = S.phase == kPhaseStartPair;
+  const int nD = R.nD, P = R.P, nn = ND * ND;
+  const bool cached = R.L0 != nullptr;
+  Band<ND> B{R.Hd, R.Hl, nD, P, R.h_inf, R.h_mindiag, R.L0, R.inv0, R.chol0_ok};
+  double *x = job.x, *g = job.g, *p = job.p, *gt = job.gt, *work = job.work;
+  if constexpr (STAGED) {
     double* sHd = s_dyn;
-    double* sHl = sHd + R.nD * nn;
-    double* sg = sHl + R.nD * nn;
-    double* sp = sg + R.P;
-    for (int i = threadIdx.x; i < R.nD * nn; i += blockDim.x) {
+    double* sHl = sHd + nD * nn;
+    x = sHl + nD * nn;
+    g = x + P;
+    p = g + P;
+    gt = p + P;
+    work = gt + P;
+    double* sL0 = work + P * 2 * ND + 3 * P;
+    double* sinv0 = sL0 + P * 2 * ND;
+    for (int i = threadIdx.x; i < nD * nn; i += blockDim.x) {
       sHd[i] = R.Hd[i];
       sHl[i] = R.Hl[i];
     }
-    for (int i = threadIdx.x; i < R.P; i += blockDim.x) {
-      sg[i] = job.g[i];
-      sp[i] = job.p[i];
-    }
-    Hd = sHd;
-    Hl = sHl;
-    gv = sg;
-    pv = sp;
-    work = sp + R.P;
-    if (R.L0 != nullptr) {  // after the subproblem's work area (factor, 1/L_ii, two vectors)
-      double* sL0 = work + R.P * 2 * R.n_dim + 3 * R.P;
-      double* sinv0 = sL0 + R.P * 2 * R.n_dim;
-      for (int i = threadIdx.x; i < R.P * 2 * R.n_dim; i += blockDim.x) sL0[i] = R.L0[i];
-      for (int i = threadIdx.x; i < R.P; i += blockDim.x) sinv0[i] = R.inv0[i];
-      L0 = sL0;
-      inv0 = sinv0;
-    }
-    __syncthreads();
-  }
-  const int P = R.P;
-  if (threadIdx.x == 0) {
-    if (R.n_dim == 3)
-      state_step<3>(job, S, R, Hd, Hl, L0, inv0, gv, pv, work, s_f, pair ? s_f2 : 0.0);
-    else
-      state_step<2>(job, S, R, Hd, Hl, L0, inv0, gv, pv, work, s_f, pair ? s_f2 : 0.0);
-  }
-  __syncthreads();
-  if (staged) {
     for (int i = threadIdx.x; i < P; i += blockDim.x) {
-      job.g[i] = gv[i];
-      job.p[i] = pv[i];
+      x[i] = job.x[i];
+      g[i] = job.g[i];
+      p[i] = job.p[i];
     }
-    __syncthreads();
+    B.Hd = sHd;
+    B.Hl = sHl;
+    if (cached) {
+      for (int i = threadIdx.x; i < P * 2 * ND; i += blockDim.x) sL0[i] = R.L0[i];
+      for (int i = threadIdx.x; i < P; i += blockDim.x) sinv0[i] = R.inv0[i];
+      B.L0 = sL0;
+      B.inv0 = sinv0;
+    }
+    if (pair) __syncthreads();  // p is loaded before the rigid point's gradient replaces it
   }
-  if (S->phase == kPhaseDone) {
+  reduce_partials(R, job.partials, &s_f, gt);
+  // paired start: the rigid point's sums, its gradient into p (free until the first step)
+  if (pair) reduce_partials(R, job.partials2, &s_f2, p);
+  state_step<ND>(S, B, x, g, p, gt, work, s_f, pair ? s_f2 : 0.0, s_red, &s_flag);
+  if constexpr (STAGED) {
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+      job.x[i] = x[i];
+      job.g[i] = g[i];
+      job.p[i] = p[i];
+    }
+  }
+  for (int i = threadIdx.x; i < (int)(sizeof(FrameState) / 8); i += blockDim.x)
+    reinterpret_cast<unsigned long long*>(job.state)[i] = reinterpret_cast<const unsigned long long*>(&S)[i];
+  if (S.phase == kPhaseDone) {
     // Finished in this step: report the state and parameters, and keep them as the warm start.
     if (job.report != nullptr) {
-      if (threadIdx.x == 0) *static_cast<FrameState*>(job.report) = *S;
+      if (threadIdx.x == 0) *static_cast<FrameState*>(job.report) = S;
       double* xr = reinterpret_cast<double*>(static_cast<char*>(job.report) + kReportHeaderBytes);
-      for (int i = threadIdx.x; i < P; i += blockDim.x) xr[i] = job.x[i];
+      for (int i = threadIdx.x; i < P; i += blockDim.x) xr[i] = x[i];
     }
-    if (S->warm != nullptr) {
-      for (int i = threadIdx.x; i < P; i += blockDim.x) S->warm[i] = job.x[i];
-      if (threadIdx.x == 0 && S->warm_seq != nullptr) *S->warm_seq = S->seq;  // read by later launches
+    if (S.warm != nullptr) {
+      for (int i = threadIdx.x; i < P; i += blockDim.x) S.warm[i] = x[i];
+      if (threadIdx.x == 0 && S.warm_seq != nullptr) *S.warm_seq = S.seq;  // read by later launches
     }
     return;
   }
-  if (S->phase == kPhaseWaitWarm) return;
+  if (S.phase == kPhaseWaitWarm) return;
   // Next trial point D = x + p, as the fused pass's control-point parameters.
-  write_trial_dparams(job, R, threadIdx.x, blockDim.x);
+  write_trial_dparams(job.dparams, x, p, nD, ND, threadIdx.x, blockDim.x);
 }
+
+}  // namespace
+
+namespace {
+template <int ND>
+cudaError_t launch_solve_nd(const Job* jobs_dev, int n_jobs, int max_nD, cudaStream_t s, const int* active,
+                            const int* n_active) {
+  constexpr long long kCapBytes = 200 * 1024;
+  const long long need = solve_smem_doubles(max_nD, ND) * (long long)sizeof(double);
+  if (need > kCapBytes) {  // every frame of the launch works in global memory
+    solve_kernel<ND, false><<<n_jobs, kSolveThreads, 0, s>>>(jobs_dev, active, n_active);
+    return cudaGetLastError();
+  }
+  if (need > 40 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(solve_kernel<ND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+    if (e != cudaSuccess) return e;
+  }
+  solve_kernel<ND, true><<<n_jobs, kSolveThreads, (size_t)need, s>>>(jobs_dev, active, n_active);
+  return cudaGetLastError();
+}
+}  // namespace
 
 cudaError_t launch_solve(const Job* jobs_dev, int n_jobs, int max_nD, int n_dim, cudaStream_t s, const int* active,
                          const int* n_active) {
-  constexpr long long kCapBytes = 200 * 1024;
-  long long need = solve_smem_doubles(max_nD, n_dim) * (long long)sizeof(double);
-  int smem = need <= kCapBytes ? (int)need : 0;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
-  solve_kernel<<<n_jobs, kSolveThreads, smem, s>>>(jobs_dev, smem / (int)sizeof(double), active, n_active);
-  return cudaGetLastError();
+  return n_dim == 3 ? launch_solve_nd<3>(jobs_dev, n_jobs, max_nD, s, active, n_active)
+                    : launch_solve_nd<2>(jobs_dev, n_jobs, max_nD, s, active, n_active);
 }
 
-__global__ void chol0_kernel(const double* Hd, const double* Hl, int nD, int nd, double* L0, double* inv0, int* ok) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (nd == 3) {
-    Band<3> B{Hd, Hl, nD, nD * 3, 0.0, 0.0};
-    *ok = band_chol(B, 0.0, L0, inv0) == 0;
-  } else {
-    Band<2> B{Hd, Hl, nD, nD * 2, 0.0, 0.0};
-    *ok = band_chol(B, 0.0, L0, inv0) == 0;
+// The factor of H itself, once per reference: one block brings the blocks of H into shared memory (when
+// they fit) for the chain that one thread runs.
+template <int ND>
+__global__ void __launch_bounds__(128) chol0_kernel(const double* Hd, const double* Hl, int nD, double* L0, double* inv0,
+                                                    int* ok, int staged) {
+  extern __shared__ double s_dyn[];
+  constexpr int NN = ND * ND;
+  Band<ND> B{Hd, Hl, nD, nD * ND, 0.0, 0.0};
+  if (staged) {
+    for (int i = threadIdx.x; i < nD * NN; i += blockDim.x) {
+      s_dyn[i] = Hd[i];
+      s_dyn[nD * NN + i] = Hl[i];
+    }
+    __syncthreads();
+    B.Hd = s_dyn;
+    B.Hl = s_dyn + nD * NN;
   }
+  if (threadIdx.x == 0) *ok = band_chol<ND>(B, 0.0, L0, inv0) == 0;
 }
 
 cudaError_t launch_chol0(const double* Hd, const double* Hl, int nD, int nd, double* L0, double* inv0, int* ok,
                          cudaStream_t s) {
-  chol0_kernel<<<1, 32, 0, s>>>(Hd, Hl, nD, nd, L0, inv0, ok);
+  const size_t bytes = (size_t)2 * nD * nd * nd * sizeof(double);
+  const int staged = bytes <= 48 * 1024;
+  if (nd == 3)
+    chol0_kernel<3><<<1, 128, staged ? bytes : 0, s>>>(Hd, Hl, nD, L0, inv0, ok, staged);
+  else
+    chol0_kernel<2><<<1, 128, staged ? bytes : 0, s>>>(Hd, Hl, nD, L0, inv0, ok, staged);
   return cudaGetLastError();
 }
 
-__global__ void test_subproblem_kernel(const double* Hd, const double* Hl, int nD, int nd, double hinf,
-                                       double mindiag, const double* g, double radius, double* p, int* boundary,
-                                       double* work) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  // work: P*(2*nd) + 3*P doubles
-  if (nd == 3) {
-    Band<3> B{Hd, Hl, nD, nD * 3, hinf, mindiag};
-    *boundary = subproblem(B, g, radius, 0.1, 20, p, work);
-  } else {
-    Band<2> B{Hd, Hl, nD, nD * 2, hinf, mindiag};
-    *boundary = subproblem(B, g, radius, 0.1, 20, p, work);
-  }
+// The subproblem of one frame on given H, g and radius, with the cached factor as the solver has it.
+// work: P * (2 * nd) + 3 * P doubles, then the cached factor and its reciprocal diagonal, P * (2 * nd)
+// + P doubles.
+template <int ND>
+__global__ void __launch_bounds__(kSolveThreads) test_subproblem_kernel(const double* Hd, const double* Hl, int nD,
+                                                                        double hinf, double mindiag, const double* g,
+                                                                        double radius, double* p, int* boundary,
+                                                                        double* work) {
+  __shared__ double s_red[3 * (kSolveThreads / 32)];
+  __shared__ int s_flag, s_ok;
+  const int P = nD * ND;
+  double* L0 = work + P * 2 * ND + 3 * P;
+  double* inv0 = L0 + P * 2 * ND;
+  Band<ND> B{Hd, Hl, nD, P, hinf, mindiag};
+  if (threadIdx.x == 0) s_ok = band_chol<ND>(B, 0.0, L0, inv0) == 0;
+  __syncthreads();
+  B.L0 = L0;
+  B.inv0 = inv0;
+  B.chol0_ok = s_ok;
+  const int b = subproblem_block<ND>(B, g, radius, 0.1, 20, p, work, s_red, &s_flag);
+  if (threadIdx.x == 0) *boundary = b;
 }
 
 cudaError_t launch_test_subproblem(const double* Hd, const double* Hl, int nD, int nd, double hinf, double mindiag,
                                    const double* g, double radius, double* p_out, int* boundary_out, double* work,
                                    cudaStream_t s) {
-  test_subproblem_kernel<<<1, 32, 0, s>>>(Hd, Hl, nD, nd, hinf, mindiag, g, radius, p_out, boundary_out, work);
+  if (nd == 3)
+    test_subproblem_kernel<3><<<1, kSolveThreads, 0, s>>>(Hd, Hl, nD, hinf, mindiag, g, radius, p_out, boundary_out, work);
+  else
+    test_subproblem_kernel<2><<<1, kSolveThreads, 0, s>>>(Hd, Hl, nD, hinf, mindiag, g, radius, p_out, boundary_out, work);
   return cudaGetLastError();
 }
 
