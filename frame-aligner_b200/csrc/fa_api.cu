@@ -1,6 +1,8 @@
 // fa_api.cu -- host runtime behind the C ABI (include/fa_b200.h): device memory under a budget,
 // reference set-up (exact scan geometry, Sobel, Hessian), frame slots, fused evaluations, the
 // single-frame and batched trust-region drivers, and the phase correlator.
+#include <limits.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -469,8 +471,9 @@ fa_status autotune(fa_reference* R) {
       // register budgets under which the kernel spills more than a few values are not candidates
       if (mb != mbs[0] && fa::eval4_active_local_bytes(R->n_dim, kind, mixed, mb) > 128) continue;
       auto launch = [&]() {
-        return fa::launch_eval4_active(jobs_dev, list, cnt, prefix, (long long)K * R->G.n_tiles, R->n_dim, kind, mixed,
-                                       mb, mb * sms, s);
+        // (the one-warp-per-tile form, whatever the count: the other has no budget to choose)
+        const long long items = (long long)K * R->G.n_tiles;
+        return fa::launch_eval4_active(jobs_dev, list, cnt, prefix, LLONG_MAX, items, R->n_dim, kind, mixed, mb, mb * sms, s);
       };
       double per_frame[2] = {0.0, 0.0};  // K frames, one frame
       for (int c = 0; c < 2; c++) {
@@ -1100,7 +1103,7 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
   const bool vec4_all = vec4;
   std::vector<Job> jobs(n);
   // most work items of one pass: a frame in the paired start phase has two items per tile
-  long long most_items = 0;
+  long long most_items = 0, least_items = LLONG_MAX;  // least: one frame left
   for (int i = 0; i < n; i++) {
     fa_frame* F = frames[i];
     if (!peak_start) FA_TRY(init_solve(F, rigid_shifts ? rigid_shifts + 3 * i : nullptr, max_iterations, vec4_all));
@@ -1110,6 +1113,7 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     max_tiles = std::max(max_tiles, F->ref->G.n_tiles);
     max_nD = std::max(max_nD, F->ref->nD);
     most_items += (long long)F->ref->G.n_tiles * (vec4_all ? 2 : 1);
+    least_items = std::min<long long>(least_items, F->ref->G.n_tiles);
   }
   // host-made initial states went on every frame's stream: one wait per stream (the copies are done then)
   if (!peak_start)
@@ -1151,7 +1155,7 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
   const int max_rounds = (max_steps + kGraphIters - 1) / kGraphIters;
   // the register budget tuned for launches of many frames, or of a few
   const int mb = n >= kManyFrames ? R0->host.tune_mb : R0->host.tune_mb_small;
-  const long long key[7] = {n, most_items, max_nD, (vec4 ? 1 : 0) + 2 * frames[0]->kind, mb, 0, max_rounds};
+  const long long key[7] = {n, most_items, max_nD, (vec4 ? 1 : 0) + 2 * frames[0]->kind, mb, least_items, max_rounds};
   const bool reuse = bc->exec && bc->frames.size() == (size_t)n &&
                      std::equal(bc->frames.begin(), bc->frames.end(), frames) && std::equal(key, key + 7, bc->key);
   if (!reuse) {
@@ -1176,7 +1180,7 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     if (e == cudaSuccess) {
       for (int it = 0; it < kGraphIters && e == cudaSuccess; it++) {
         if (vec4)
-          e = fa::launch_eval4_active(bc->jobs_dev, bc->d_list, bc->d_active, bc->d_prefix, most_items, R0->n_dim,
+          e = fa::launch_eval4_active(bc->jobs_dev, bc->d_list, bc->d_active, bc->d_prefix, least_items, most_items, R0->n_dim,
                                       frames[0]->kind, R0->prec == FA_PREC_MIXED, mb, mb * sms, s);
         else
           e = fa::launch_eval(bc->jobs_dev, n, max_tiles, R0->n_dim, frames[0]->kind, R0->prec == FA_PREC_MIXED, s,

@@ -56,10 +56,12 @@ cudaError_t launch_eval(const Job* jobs_dev, int n_jobs, int max_tiles, int n_di
 
 // Persistent fused pass over the compacted active list: grid CTAs walk the (active[a], tile) items,
 // item = tile_prefix[a] + tile for a < *n_active, so frames of different sizes share one launch
-// (rows must be multiples of 4). most_items bounds the grid.
+// (rows must be multiples of 4). A pass of few items gives each a CTA, one of many each a warp; which it
+// is follows on the device, and least_items (the smallest frame's tiles) and most_items bound what a
+// launch can meet.
 cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const int* n_active, const int* tile_prefix,
-                                long long most_items, int n_dim, int frame_kind, bool ref_bf16, int mb, int grid,
-                                cudaStream_t s);
+                                long long least_items, long long most_items, int n_dim, int frame_kind, bool ref_bf16,
+                                int mb, int grid, cudaStream_t s);
 
 // Thread-local (spill) bytes of that kernel's instantiation for a register budget of mb CTAs per SM.
 size_t eval4_active_local_bytes(int n_dim, int frame_kind, bool ref_bf16, int mb);

@@ -18,6 +18,8 @@
 // on the device (out of the passes) until frame k-d has written its solution to the warm-start ring
 // entry stamped with k-d's sequence number, and continues from that fourth starting point; results
 // therefore do not depend on arrival timing either.
+#include <limits.h>
+
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -130,7 +132,7 @@ struct SrvClass {
   cudaEvent_t ev = nullptr;
   bool running = false;
   int in_solve = 0;
-  int max_nD = 0, max_tiles = 0, mb = 2, grid_mult = 2;
+  int max_nD = 0, max_tiles = 0, min_tiles = INT_MAX, mb = 2, grid_mult = 2;
   long long tuned_for = -1;  // N of the acquisition whose tuning the class uses
   std::vector<Alloc> allocs;
 };
@@ -275,6 +277,7 @@ fa_status attach(fa_server* S, SrvAcq* q) {
   C->acqs.push_back(q);
   C->max_nD = std::max(C->max_nD, R->nD);
   C->max_tiles = std::max(C->max_tiles, R->G.n_tiles);
+  C->min_tiles = std::min(C->min_tiles, R->G.n_tiles);
   if (R->N > C->tuned_for) {  // the largest volume's register budget tuned for launches of a few frames
     C->tuned_for = R->N;
     C->mb = R->host.tune_mb_small;
@@ -302,7 +305,8 @@ fa_status class_capture(fa_server* S, SrvClass* C) {
       e = fa::launch_compact(C->jobs_dev, C->cap, C->list, n_active, C->prefix, C->busy, done_list, n_done, s);
       if (e == cudaSuccess) {
         if (C->vec4)
-          e = fa::launch_eval4_active(C->jobs_dev, C->list, n_active, C->prefix, 2LL * C->cap * C->max_tiles,
+          e = fa::launch_eval4_active(C->jobs_dev, C->list, n_active, C->prefix, C->min_tiles,
+                                      2LL * C->cap * C->max_tiles,
                                       C->n_dim, C->kind, C->bf16, C->mb, C->grid_mult * S->sms, s);
         else
           e = fa::launch_eval(C->jobs_dev, C->cap, C->max_tiles, C->n_dim, C->kind, C->bf16, s, false);
