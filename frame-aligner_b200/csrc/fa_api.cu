@@ -1001,17 +1001,17 @@ fa_status finish_solve_enqueue(fa_frame* F, cudaStream_t s) {
   return FA_OK;
 }
 
-// D (and the statistics) from the copies finish_solve_enqueue queued, once they completed.
-void finish_solve_read(fa_frame* F, double* D_out, fa_align_stats* stats) {
-  fa_reference* R = F->ref;
+// D (and the statistics) of a solved frame from its parameters and state in host memory.
+void finish_solve_read(const fa_frame* F, const double* x, const fa::FrameState& S, double* D_out,
+                       fa_align_stats* stats) {
+  const fa_reference* R = F->ref;
   const int nd = R->n_dim;
   for (int k = 0; k < R->nD; k++) {
-    D_out[3 * k] = F->h_x[k * nd];
-    D_out[3 * k + 1] = F->h_x[k * nd + 1];
-    D_out[3 * k + 2] = nd == 3 ? F->h_x[k * nd + 2] : 0.0;
+    D_out[3 * k] = x[k * nd];
+    D_out[3 * k + 1] = x[k * nd + 1];
+    D_out[3 * k + 2] = nd == 3 ? x[k * nd + 2] : 0.0;
   }
   if (stats) {
-    const fa::FrameState& S = *F->h_state;
     stats->iterations = S.iter;
     stats->evaluations = S.evaluations;
     stats->accepted = S.accepted;
@@ -1024,7 +1024,7 @@ void finish_solve_read(fa_frame* F, double* D_out, fa_align_stats* stats) {
 fa_status finish_solve(fa_frame* F, double* D_out, fa_align_stats* stats) {
   FA_TRY(finish_solve_enqueue(F, F->stream));
   FA_CU(cudaStreamSynchronize(F->stream));
-  finish_solve_read(F, D_out, stats);
+  finish_solve_read(F, F->h_x, *F->h_state, D_out, stats);
   return FA_OK;
 }
 
@@ -1071,16 +1071,17 @@ struct PeakStart {
   cudaEvent_t ready;
 };
 
-// Queues a batched solve of n frames on frames[0]'s stream: the starting states, one launch of the
-// cached solve graph, and the copies of every frame's x and state into its pinned buffers; the
-// caller's align_batch_finish waits for them. frame_data (optional) replaces each frame's own device
+// Queues a batched solve of n frames on frames[0]'s stream: the starting states and one launch of the
+// cached solve graph, whose steps write every finished frame's state and x to host-mapped memory; the
+// caller's align_batch_finish waits for it. frame_data (optional) replaces each frame's own device
 // data pointer for this call. bc keeps the buffers and the graph for the next call on the same
 // frames. With `peak_start` the rigid starts come from device peaks (rigid_shifts is ignored) and the
 // states are set up on the device, so the host neither waits for the peaks nor copies a state.
 //
-// The graph holds one while-conditional node whose body is kGraphIters x (fused pass, solve step,
-// active-list compaction) and a loop-control kernel: the body repeats on the device until no frame is
-// active or the iteration limit is reached, with no host round trip between rounds.
+// The graph holds one while-conditional node whose body is kGraphIters x (fused pass, solve step): the
+// last CTA of a step builds the next active list, the last step also controls the loop, and the body
+// repeats on the device until no frame is active or the iteration limit is reached, with no host round
+// trip between rounds.
 fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigid_shifts, int max_iterations,
                               const void* const* frame_data, BatchCache* bc, const PeakStart* peak_start) {
   if (!frames || n <= 0 || !bc) return fail(FA_ERR_BAD_ARG, "bad arguments");
@@ -1096,7 +1097,30 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
   fa_context* ctx = R0->ctx;
   FA_CU(cudaSetDevice(ctx->device));
   cudaStream_t s = frames[0]->stream;
-  int max_tiles = 0, max_nD = 0;
+  int max_tiles = 0, max_nD = 0, max_P = 0;
+  for (int i = 0; i < n; i++) max_P = std::max(max_P, frames[i]->ref->P);
+  const size_t out_bytes = batch_report_offset(n, max_P);
+  if (bc->cap < n || bc->out_bytes < out_bytes) {
+    FA_CU(cudaStreamSynchronize(s));
+    batch_cache_release(ctx, bc);
+    FA_TRY(dalloc_t(ctx, (size_t)n, &bc->jobs_dev, bc->allocs));
+    FA_TRY(dalloc_t(ctx, 4, &bc->d_active, bc->allocs));
+    FA_TRY(dalloc_t(ctx, 2 * (size_t)n, &bc->d_list, bc->allocs));
+    FA_TRY(dalloc_t(ctx, (size_t)n + 1, &bc->d_prefix, bc->allocs));
+    void* hp = nullptr;
+    if (cudaHostAlloc(&hp, out_bytes, cudaHostAllocMapped) != cudaSuccess) {
+      cudaGetLastError();
+      batch_cache_release(ctx, bc);
+      return fail(FA_ERR_OOM, "cudaHostAlloc failed");
+    }
+    bc->h_out = static_cast<char*>(hp);
+    bc->out_bytes = out_bytes;
+    void* dp = nullptr;
+    FA_CU(cudaHostGetDevicePointer(&dp, hp, 0));
+    bc->d_out = static_cast<char*>(dp);
+    FA_CU(cudaMemsetAsync(bc->d_active, 0, 4 * sizeof(int), s));
+    bc->cap = n;
+  }
   bool vec4 = true;
   for (int i = 0; i < n; i++) vec4 = vec4 && (frames[i]->ref->nx % 4 == 0);
   // the persistent pass evaluates both cold starting points of a frame in its first launch
@@ -1110,6 +1134,8 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     jobs[i] = F->job;
     jobs[i].state = F->state;
     if (frame_data) jobs[i].frame = frame_data[i];
+    jobs[i].report = bc->d_out + batch_report_offset(i, max_P);
+    reinterpret_cast<fa::FrameState*>(bc->h_out + batch_report_offset(i, max_P))->phase = -1;  // not reported
     max_tiles = std::max(max_tiles, F->ref->G.n_tiles);
     max_nD = std::max(max_nD, F->ref->nD);
     most_items += (long long)F->ref->G.n_tiles * (vec4_all ? 2 : 1);
@@ -1118,19 +1144,6 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
   // host-made initial states went on every frame's stream: one wait per stream (the copies are done then)
   if (!peak_start)
     for (int i = 0; i < n; i++) FA_CU(cudaStreamSynchronize(frames[i]->stream));
-  if (bc->cap < n) {
-    FA_CU(cudaStreamSynchronize(s));
-    batch_cache_release(ctx, bc);
-    FA_TRY(dalloc_t(ctx, (size_t)n, &bc->jobs_dev, bc->allocs));
-    FA_TRY(dalloc_t(ctx, 2, &bc->d_active, bc->allocs));  // [0] active frames, [1] rounds of the loop
-    FA_TRY(dalloc_t(ctx, (size_t)n, &bc->d_list, bc->allocs));
-    FA_TRY(dalloc_t(ctx, (size_t)n + 1, &bc->d_prefix, bc->allocs));
-    if (cudaMallocHost(&bc->h_rounds, sizeof(int)) != cudaSuccess) {
-      bc->h_rounds = nullptr;
-      return fail(FA_ERR_OOM, "cudaMallocHost failed");
-    }
-    bc->cap = n;
-  }
   // The job table goes up before any wait on the peaks (a copy from pageable memory may wait for the
   // stream); then the device-side start when the peaks are on the device, and the first active list
   // from the states.
@@ -1142,17 +1155,28 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
                                     peak_start->cnz, peak_start->binning, max_iterations, vec4_all, s);
     g_launches += 1;
   }
-  if (e == cudaSuccess)
-    e = fa::launch_compact(bc->jobs_dev, n, bc->d_list, bc->d_active, bc->d_prefix, nullptr, nullptr, nullptr, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(bc->d_active + 1, 0, sizeof(int), s);
+  // each round runs kGraphIters iterations; the host loop this replaces stopped after max + 4 steps
+  constexpr int kGraphIters = 4;
+  static_assert(kGraphIters % 2 == 0, "the steps alternate between two lists");
+  const int max_steps = (max_iterations > 0 ? max_iterations : 100) + 4;
+  const int max_rounds = (max_steps + kGraphIters - 1) / kGraphIters;
+  *reinterpret_cast<int*>(bc->h_out) = 0;
+  auto list_out = [&](int which) {
+    fa::ActiveOut o{};
+    o.n_jobs = n;
+    o.active = bc->d_list + (size_t)which * bc->cap;
+    o.n_active = bc->d_active + which;
+    o.prefix = bc->d_prefix;
+    o.rounds = bc->d_active + 2;
+    o.rounds_host = reinterpret_cast<int*>(bc->d_out);
+    o.max_rounds = max_rounds;
+    return o;
+  };
+  if (e == cudaSuccess) e = fa::launch_compact(bc->jobs_dev, list_out(0), s);
   g_launches += 1;
   if (e != cudaSuccess) return fail(FA_ERR_CUDA, std::string("batch start: ") + cudaGetErrorString(e));
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  constexpr int kGraphIters = 4;
-  // each round runs kGraphIters iterations; the host loop this replaces stopped after max + 4 steps
-  const int max_steps = (max_iterations > 0 ? max_iterations : 100) + 4;
-  const int max_rounds = (max_steps + kGraphIters - 1) / kGraphIters;
   // the register budget tuned for launches of many frames, or of a few
   const int mb = n >= kManyFrames ? R0->host.tune_mb : R0->host.tune_mb_small;
   const long long key[7] = {n, most_items, max_nD, (vec4 ? 1 : 0) + 2 * frames[0]->kind, mb, least_items, max_rounds};
@@ -1179,17 +1203,19 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
       for (int it = 0; it < kGraphIters && e == cudaSuccess; it++) {
+        const fa::ActiveOut in = list_out(it & 1);
+        fa::ActiveOut out = list_out(1 - (it & 1));
+        out.loop = loop;
         if (vec4)
-          e = fa::launch_eval4_active(bc->jobs_dev, bc->d_list, bc->d_active, bc->d_prefix, least_items, most_items, R0->n_dim,
-                                      frames[0]->kind, R0->prec == FA_PREC_MIXED, mb, mb * sms, s);
+          e = fa::launch_eval4_active(bc->jobs_dev, in.active, in.n_active, in.prefix, least_items, most_items,
+                                      R0->n_dim, frames[0]->kind, R0->prec == FA_PREC_MIXED, mb, mb * sms, s);
         else
           e = fa::launch_eval(bc->jobs_dev, n, max_tiles, R0->n_dim, frames[0]->kind, R0->prec == FA_PREC_MIXED, s,
                               false);
-        if (e == cudaSuccess) e = fa::launch_solve(bc->jobs_dev, n, max_nD, R0->n_dim, s);
         if (e == cudaSuccess)
-          e = fa::launch_compact(bc->jobs_dev, n, bc->d_list, bc->d_active, bc->d_prefix, nullptr, nullptr, nullptr, s);
+          e = fa::launch_solve(bc->jobs_dev, n, max_nD, R0->n_dim, s, in.active, in.n_active, &out,
+                               reinterpret_cast<unsigned*>(bc->d_active + 3), it == kGraphIters - 1);
       }
-      if (e == cudaSuccess) e = fa::launch_loop_control(loop, bc->d_active, bc->d_active + 1, max_rounds, s);
       cudaGraph_t captured = nullptr;
       const cudaError_t e2 = cudaStreamEndCapture(s, &captured);
       if (e == cudaSuccess) e = e2;
@@ -1204,12 +1230,8 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     std::copy(key, key + 7, bc->key);
   }
   e = cudaGraphLaunch(bc->exec, s);
-  // the rounds that ran, for the launch count
-  if (e == cudaSuccess) e = cudaMemcpyAsync(bc->h_rounds, bc->d_active + 1, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return fail(FA_ERR_CUDA, std::string("batch solve: ") + cudaGetErrorString(e));
-  bc->per_round = 3 * kGraphIters + 1;
-  // every frame's x and state in one batch of copies on the solve's stream
-  for (int i = 0; i < n; i++) FA_TRY(finish_solve_enqueue(frames[i], s));
+  bc->per_round = 2 * kGraphIters;
   return FA_OK;
 }
 
@@ -1217,11 +1239,22 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
 fa_status align_batch_finish(fa_frame* const* frames, int n, const BatchCache* bc, double* D_out,
                              fa_align_stats* stats) {
   if (cudaStreamSynchronize(frames[0]->stream) != cudaSuccess) return fail(FA_ERR_CUDA, "batch solve failed");
-  g_launches += (long long)*bc->h_rounds * bc->per_round;
+  g_launches += (long long)*reinterpret_cast<const int*>(bc->h_out) * bc->per_round;
+  int max_P = 0;
+  for (int i = 0; i < n; i++) max_P = std::max(max_P, frames[i]->ref->P);
   for (int i = 0; i < n; i++) {
     fa_frame* F = frames[i];
-    finish_solve_read(F, D_out + (size_t)i * 3 * F->ref->nD, stats ? stats + i : nullptr);
+    double* D = D_out + (size_t)i * 3 * F->ref->nD;
+    const char* rep = bc->h_out + batch_report_offset(i, max_P);
+    const fa::FrameState& S = *reinterpret_cast<const fa::FrameState*>(rep);
     F->have_last = false;
+    if (S.phase != fa::kPhaseDone) {  // the loop's limit came first: where the solve stands
+      FA_TRY(finish_solve_enqueue(F, frames[0]->stream));
+      FA_CU(cudaStreamSynchronize(frames[0]->stream));
+      finish_solve_read(F, F->h_x, *F->h_state, D, stats ? stats + i : nullptr);
+      continue;
+    }
+    finish_solve_read(F, reinterpret_cast<const double*>(rep + fa::kReportHeaderBytes), S, D, stats ? stats + i : nullptr);
   }
   return FA_OK;
 }
@@ -1256,8 +1289,9 @@ void batch_cache_release(fa_context* ctx, BatchCache* c) {
   if (c->exec) cudaGraphExecDestroy(c->exec);
   c->exec = nullptr;
   c->frames.clear();
-  if (c->h_rounds) cudaFreeHost(c->h_rounds);
-  c->h_rounds = nullptr;
+  if (c->h_out) cudaFreeHost(c->h_out);
+  c->h_out = c->d_out = nullptr;
+  c->out_bytes = 0;
   dfree_all(ctx, c->allocs);
   c->jobs_dev = nullptr;
   c->d_active = c->d_list = c->d_prefix = nullptr;

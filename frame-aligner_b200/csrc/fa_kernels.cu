@@ -661,112 +661,14 @@ cudaError_t launch_hessian(const RefDev* ref_dev, const RefDev& R, const double*
 
 // ------------------------------------------------------------------ batched-solve bookkeeping ----
 
-// One block of 1024 threads scans the job table in chunks: ballots give each warp's active / done
-// counts, a shuffle scan the tile prefix inside a warp, and thread 0 the per-warp offsets.
-__global__ void __launch_bounds__(1024) compact_kernel(const Job* __restrict__ jobs, int n, int* __restrict__ active,
-                                                       int* __restrict__ n_active, int* __restrict__ tile_prefix,
-                                                       int* __restrict__ busy, int* __restrict__ done_list,
-                                                       int* __restrict__ n_done) {
-  __shared__ int s_act[32], s_tiles[32], s_done[32];
-  __shared__ int base_a, base_t, base_d, tot_a, tot_t, tot_d;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (threadIdx.x == 0) {
-    base_a = 0;
-    base_t = 0;
-    base_d = busy != nullptr ? *n_done : 0;
-  }
-  __syncthreads();
-  const unsigned lt = (1u << lane) - 1u;
-  for (int c = 0; c < n; c += blockDim.x) {
-    const int i = c + threadIdx.x;
-    int phase = i < n ? jobs[i].state->phase : (int)kPhaseDone;
-    if (phase == kPhaseWaitWarm) {
-      // Resume a frame waiting for its warm start once the earlier frame's solution is written (by a
-      // finished solve launch): the fourth starting point x + (warm - x).
-      const Job& j = jobs[i];
-      FrameState* S = j.state;
-      if (*S->warm_seq == S->warm_need) {
-        const RefDev& R = *j.ref;
-        for (int q = 0; q < R.P; q++) j.p[q] = S->warm[q] - j.x[q];
-        write_trial_dparams(j.dparams, j.x, j.p, R.nD, R.n_dim, 0, 1);
-        S->phase = kPhaseStartLast;
-        phase = kPhaseStartLast;
-      }
-    }
-    const bool act = i < n && phase != kPhaseDone && phase != kPhaseWaitWarm;
-    const bool fin = i < n && busy != nullptr && phase == kPhaseDone && busy[i] != 0;
-    const int tiles = act ? jobs[i].ref->n_tiles * (phase == kPhaseStartPair ? 2 : 1) : 0;
-    int incl = tiles;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const unsigned ma = __ballot_sync(0xffffffffu, act), md = __ballot_sync(0xffffffffu, fin);
-    if (lane == 31) s_tiles[w] = incl;
-    if (lane == 0) {
-      s_act[w] = __popc(ma);
-      s_done[w] = __popc(md);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int a = 0, t = 0, d = 0;
-      for (int k = 0; k < nw; k++) {
-        const int va = s_act[k], vt = s_tiles[k], vd = s_done[k];
-        s_act[k] = a;
-        s_tiles[k] = t;
-        s_done[k] = d;
-        a += va;
-        t += vt;
-        d += vd;
-      }
-      tot_a = a;
-      tot_t = t;
-      tot_d = d;
-    }
-    __syncthreads();
-    if (act) {
-      const int pos = base_a + s_act[w] + __popc(ma & lt);
-      active[pos] = i;
-      tile_prefix[pos] = base_t + s_tiles[w] + incl - tiles;
-    }
-    if (fin) {
-      done_list[base_d + s_done[w] + __popc(md & lt)] = i;
-      busy[i] = 0;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      base_a += tot_a;
-      base_t += tot_t;
-      base_d += tot_d;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    *n_active = base_a;
-    tile_prefix[base_a] = base_t;
-    if (busy != nullptr) *n_done = base_d;
-  }
+// The first list of a solve or of a server's graph launch (later ones come from the solve steps).
+__global__ void __launch_bounds__(256) compact_kernel(const Job* __restrict__ jobs, ActiveOut out) {
+  if (threadIdx.x == 0 && out.rounds != nullptr) *out.rounds = 0;
+  compact_block(jobs, out);
 }
 
-cudaError_t launch_compact(const Job* jobs_dev, int n_jobs, int* active, int* n_active, int* tile_prefix, int* busy,
-                           int* done_list, int* n_done, cudaStream_t s) {
-  compact_kernel<<<1, 1024, 0, s>>>(jobs_dev, n_jobs, active, n_active, tile_prefix, busy, done_list, n_done);
-  return cudaGetLastError();
-}
-
-// Last node of the body of a batched solve's device-side loop: counts the rounds and repeats the body
-// while a frame is still active and fewer than max_rounds rounds ran.
-__global__ void loop_control_kernel(cudaGraphConditionalHandle h, const int* __restrict__ n_active,
-                                    int* __restrict__ rounds, int max_rounds) {
-  const int r = *rounds + 1;
-  *rounds = r;
-  cudaGraphSetConditional(h, *n_active > 0 && r < max_rounds ? 1u : 0u);
-}
-
-cudaError_t launch_loop_control(cudaGraphConditionalHandle h, const int* n_active, int* rounds, int max_rounds,
-                                cudaStream_t s) {
-  loop_control_kernel<<<1, 1, 0, s>>>(h, n_active, rounds, max_rounds);
+cudaError_t launch_compact(const Job* jobs_dev, const ActiveOut& out, cudaStream_t s) {
+  compact_kernel<<<1, 256, 0, s>>>(jobs_dev, out);
   return cudaGetLastError();
 }
 

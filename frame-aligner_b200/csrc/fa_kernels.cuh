@@ -66,21 +66,28 @@ cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const in
 // Thread-local (spill) bytes of that kernel's instantiation for a register budget of mb CTAs per SM.
 size_t eval4_active_local_bytes(int n_dim, int frame_kind, bool ref_bf16, int mb);
 
-// Rebuilds the active list of a job table (frames not done, ascending index), the exclusive prefix
-// sum of their tile counts (tile_prefix[*n_active] = items of the next fused pass), and, when busy is
-// non-null, appends frames that are done and still busy to done_list[*n_done...] and clears busy.
-cudaError_t launch_compact(const Job* jobs_dev, int n_jobs, int* active, int* n_active, int* tile_prefix, int* busy,
-                           int* done_list, int* n_done, cudaStream_t s);
+// Where the active list of a job table goes (frames not done and not waiting, ascending index): the list,
+// its length, the exclusive prefix sum of the frames' tile counts (prefix[*n_active] = items of the next
+// fused pass) and, when busy is non-null, frames that are done and still busy appended to
+// done_list[*n_done ...] (busy is cleared). A frame waiting for a warm start that has been written is
+// resumed. In a device-side loop (rounds non-null) the list that ends a round also counts it and repeats
+// the loop while a frame is active and fewer than max_rounds rounds ran.
+struct ActiveOut {
+  int n_jobs;
+  int *active, *n_active, *prefix;
+  int *busy, *done_list, *n_done;
+  int* rounds;          // device counter, set to zero by launch_compact
+  int* rounds_host;     // host-mapped copy
+  int max_rounds;
+  cudaGraphConditionalHandle loop;
+};
+cudaError_t launch_compact(const Job* jobs_dev, const ActiveOut& out, cudaStream_t s);
 
-// Initialises the solve state of n frames (zero start, optional rigid and warm starts) and marks them busy.
-// Loop control inside a while-conditional graph body: ++*rounds, and the body repeats while
-// *n_active > 0 and *rounds < max_rounds.
-cudaError_t launch_loop_control(cudaGraphConditionalHandle h, const int* n_active, int* rounds, int max_rounds,
-                                cudaStream_t s);
 // Zero / paired start of n jobs from phase-correlation peak indices in device memory (correlator
 // dims cnz x cny x cnx, x and y scaled by the binning).
 cudaError_t launch_activate_peaks(const Job* jobs_dev, int n, const long long* peaks, int cnx, int cny, int cnz,
                                   int binning, int max_iter, bool pair, cudaStream_t s);
+// Initialises the solve state of n frames (zero start, optional rigid and warm starts) and marks them busy.
 cudaError_t launch_activate(const Job* jobs_dev, const Activation* recs, int n, int* busy, cudaStream_t s);
 
 // Reduces one job's tile partials into result = [f, g(P)] (deterministic order).
@@ -94,9 +101,13 @@ cudaError_t launch_warp(const RefDev* ref_dev, const RefDev& ref_host, const voi
 // One trust-region step for each job (grid = n_jobs): reduce partials, advance the state machine,
 // solve the next subproblem, write the next trial point's dparams. With an active list, block b
 // serves jobs[active[b]] for b < *n_active. max_nD / n_dim size the shared-memory staging (frames
-// above about 200 KB work in global memory).
+// above about 200 KB work in global memory). With `next`, the last CTA to finish builds the next active
+// list there (its list and length must not be `active` and `n_active`, which the launch's other CTAs may
+// still read; `finished` counts them and is zero between launches), and with end_of_round it also
+// controls the loop.
 cudaError_t launch_solve(const Job* jobs_dev, int n_jobs, int max_nD, int n_dim, cudaStream_t s,
-                         const int* active = nullptr, const int* n_active = nullptr);
+                         const int* active = nullptr, const int* n_active = nullptr, const ActiveOut* next = nullptr,
+                         unsigned* finished = nullptr, bool end_of_round = false);
 
 // Test hook: the device trust-region subproblem on given dense H (P x P) and g.
 // The band Cholesky factor of H (lambda = 0) into L0 (nD * nd rows of 2 * nd) and inv0 (nD * nd); *ok

@@ -149,16 +149,24 @@ namespace fa_rt {
 struct BatchCache {
   std::vector<Alloc> allocs;
   fa::Job* jobs_dev = nullptr;
-  int* d_active = nullptr;  // [0] active frames, [1] rounds of the device-side loop
-  int* d_list = nullptr;
+  int* d_active = nullptr;  // [0], [1] active frames of the two lists, [2] rounds of the loop, [3] finished CTAs
+  int* d_list = nullptr;    // two lists of cap entries: a step reads one and builds the other
   int* d_prefix = nullptr;
-  int* h_rounds = nullptr;  // pinned: rounds the last solve ran
+  // host-mapped memory the solve steps write: the rounds of the last solve, then one report per frame
+  char* h_out = nullptr;
+  char* d_out = nullptr;    // its device address
+  size_t out_bytes = 0;
   int per_round = 0;        // kernel launches per round
   int cap = 0;
   cudaGraphExec_t exec = nullptr;
   std::vector<fa_frame*> frames;  // the frames the graph was captured for
   long long key[7] = {0, 0, 0, 0, 0, 0, 0};
 };
+// Report i of a batch whose frames have at most P parameters.
+constexpr size_t kBatchOutHeader = 64;
+inline size_t batch_report_offset(int i, int P) {
+  return kBatchOutHeader + (size_t)i * ((fa::kReportHeaderBytes + (size_t)P * sizeof(double) + 63) / 64 * 64);
+}
 // Frees the cache's buffers and graph (after the caller's streams are idle).
 void batch_cache_release(fa_context* ctx, BatchCache* c);
 

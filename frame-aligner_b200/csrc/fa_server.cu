@@ -118,6 +118,7 @@ struct SrvClass {
   int* prefix = nullptr;              // cap + 1
   int* busy = nullptr;
   int* counts = nullptr;              // [n_active, n_done, done list (cap)]
+  int* next = nullptr;                // [n_active of the second list, CTAs finished]
   int* h_counts = nullptr;            // pinned copy, written by the graph's last node
   fa::Activation* d_act = nullptr;
   fa::Activation* h_act = nullptr;    // pinned
@@ -224,10 +225,11 @@ fa_status class_create_impl(fa_server* S, SrvClass* C) {
   fa_context* ctx = S->ctx;
   const int cap = C->cap;
   FA_TRY(dalloc_t(ctx, (size_t)cap, &C->jobs_dev, C->allocs));
-  FA_TRY(dalloc_t(ctx, (size_t)cap, &C->list, C->allocs));
+  FA_TRY(dalloc_t(ctx, 2 * (size_t)cap, &C->list, C->allocs));
   FA_TRY(dalloc_t(ctx, (size_t)cap + 1, &C->prefix, C->allocs));
   FA_TRY(dalloc_t(ctx, (size_t)cap, &C->busy, C->allocs));
   FA_TRY(dalloc_t(ctx, (size_t)cap + 2, &C->counts, C->allocs));
+  FA_TRY(dalloc_t(ctx, 2, &C->next, C->allocs));
   FA_TRY(dalloc_t(ctx, (size_t)cap, &C->d_act, C->allocs));
   FA_TRY(dalloc_t(ctx, 1, &C->dummy, C->allocs));
   if (cudaMallocHost(&C->h_jobs, (size_t)cap * sizeof(Job)) != cudaSuccess ||
@@ -247,6 +249,7 @@ fa_status class_create_impl(fa_server* S, SrvClass* C) {
   FA_CU(cudaMemcpyAsync(C->jobs_dev, C->h_jobs, (size_t)cap * sizeof(Job), cudaMemcpyHostToDevice, C->stream));
   FA_CU(cudaMemsetAsync(C->busy, 0, (size_t)cap * sizeof(int), C->stream));
   FA_CU(cudaMemsetAsync(C->counts, 0, (size_t)(cap + 2) * sizeof(int), C->stream));
+  FA_CU(cudaMemsetAsync(C->next, 0, 2 * sizeof(int), C->stream));
   FA_CU(cudaStreamSynchronize(C->stream));
   return FA_OK;
 }
@@ -287,34 +290,42 @@ fa_status attach(fa_server* S, SrvAcq* q) {
   return FA_OK;
 }
 
-// Graph of one launch: iterations_per_launch x (compact, fused pass, step), a final compact, and
-// the copy of the counts and done list to pinned host memory.
+// Graph of one launch: the active list, iterations_per_launch x (fused pass, step that also builds the
+// next list), and the copy of the counts and done list to pinned host memory.
 fa_status class_capture(fa_server* S, SrvClass* C) {
   if (C->exec) cudaGraphExecDestroy(C->exec);
   if (C->graph) cudaGraphDestroy(C->graph);
   C->exec = nullptr;
   C->graph = nullptr;
   cudaStream_t s = C->stream;
-  int* n_active = C->counts;
-  int* n_done = C->counts + 1;
-  int* done_list = C->counts + 2;
+  // the steps alternate between two lists; the list before the first step is list 0
+  auto list_out = [&](int which) {
+    fa::ActiveOut o{};
+    o.n_jobs = C->cap;
+    o.active = C->list + (size_t)which * C->cap;
+    o.n_active = which ? C->next : C->counts;
+    o.prefix = C->prefix;
+    o.busy = C->busy;
+    o.done_list = C->counts + 2;
+    o.n_done = C->counts + 1;
+    return o;
+  };
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    e = cudaMemsetAsync(n_done, 0, sizeof(int), s);
+    e = cudaMemsetAsync(C->counts + 1, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = fa::launch_compact(C->jobs_dev, list_out(0), s);
     for (int it = 0; it < S->cfg.iterations_per_launch && e == cudaSuccess; it++) {
-      e = fa::launch_compact(C->jobs_dev, C->cap, C->list, n_active, C->prefix, C->busy, done_list, n_done, s);
-      if (e == cudaSuccess) {
-        if (C->vec4)
-          e = fa::launch_eval4_active(C->jobs_dev, C->list, n_active, C->prefix, C->min_tiles,
-                                      2LL * C->cap * C->max_tiles,
-                                      C->n_dim, C->kind, C->bf16, C->mb, C->grid_mult * S->sms, s);
-        else
-          e = fa::launch_eval(C->jobs_dev, C->cap, C->max_tiles, C->n_dim, C->kind, C->bf16, s, false);
-      }
-      if (e == cudaSuccess) e = fa::launch_solve(C->jobs_dev, C->cap, C->max_nD, C->n_dim, s, C->list, n_active);
+      const fa::ActiveOut in = list_out(it & 1), out = list_out(1 - (it & 1));
+      if (C->vec4)
+        e = fa::launch_eval4_active(C->jobs_dev, in.active, in.n_active, in.prefix, C->min_tiles,
+                                    2LL * C->cap * C->max_tiles, C->n_dim, C->kind, C->bf16, C->mb,
+                                    C->grid_mult * S->sms, s);
+      else
+        e = fa::launch_eval(C->jobs_dev, C->cap, C->max_tiles, C->n_dim, C->kind, C->bf16, s, false);
+      if (e == cudaSuccess)
+        e = fa::launch_solve(C->jobs_dev, C->cap, C->max_nD, C->n_dim, s, in.active, in.n_active, &out,
+                             reinterpret_cast<unsigned*>(C->next + 1), false);
     }
-    if (e == cudaSuccess)
-      e = fa::launch_compact(C->jobs_dev, C->cap, C->list, n_active, C->prefix, C->busy, done_list, n_done, s);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(C->h_counts, C->counts, (size_t)(C->cap + 2) * sizeof(int), cudaMemcpyDeviceToHost, s);
     cudaError_t e2 = cudaStreamEndCapture(s, &C->graph);
@@ -566,7 +577,7 @@ fa_status class_launch(fa_server* S, SrvClass* C, bool* launched) {
     g_launches += 1;
   }
   FA_CU(cudaGraphLaunch(C->exec, C->stream));
-  g_launches += 3 * S->cfg.iterations_per_launch + 1;
+  g_launches += 2 * S->cfg.iterations_per_launch + 1;
   FA_CU(cudaEventRecord(C->ev, C->stream));
   FA_CU(cudaLaunchHostFunc(C->stream, wake_worker, S));
   C->in_solve += n_act;
