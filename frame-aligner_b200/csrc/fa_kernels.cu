@@ -1,6 +1,6 @@
 // fa_kernels.cu -- sm_100a kernels of the warper path.
 //
-//   sobel_tiled_kernel  Sobel3d (FrameAligner/Sobel3d.cpp:8-85), bit-exact float arithmetic
+//   sobel_kernel    Sobel3d (FrameAligner/Sobel3d.cpp:8-85), bit-exact float arithmetic
 //   hessian_*       computeSteepestDecentImages + computeHessian (FrameWarper.cpp:296-395)
 //   eval_kernel     fused warpImageInterpolated + computeErrorImage + computeJacobian
 //                   (FrameWarper.cpp:4-69,147-176): one HBM pass per frame evaluation
@@ -17,92 +17,176 @@ namespace fa {
 
 // ------------------------------------------------------------------ Sobel3d ----------------------
 
-// One separable pass at position i of an axis of length n (Sobel3d.cpp:8-58): interior
-// f0*G(i-1) + f1*G(i) + f2*G(i+1); edges e1 = {e1a*G(0) + e1b*G(1)}, e2 = {e2a*G(n-1) + e2b*G(n-2)}.
-// Float products and sums are rounded one by one (no FMA), as in the reference build.
-template <typename G>
-__device__ __forceinline__ float pass(int i, int n, bool copy_if_single, const float* f, const float* e1,
-                                      const float* e2, G get) {
-  if (n == 1 && copy_if_single) return get(i);
-  if (i == 0) return __fadd_rn(__fmul_rn(e1[0], get(0)), __fmul_rn(e1[1], get(1)));
-  if (i == n - 1) return __fadd_rn(__fmul_rn(e2[0], get(n - 1)), __fmul_rn(e2[1], get(n - 2)));
-  return __fadd_rn(__fadd_rn(__fmul_rn(f[0], get(i - 1)), __fmul_rn(f[1], get(i))), __fmul_rn(f[2], get(i + 1)));
+// One separable pass (Sobel3d.cpp:8-58) at a position of an axis from its neighbours: interior
+// f0*lo + f1*mid + f2*hi; first of the axis e1a*mid + e1b*hi; last e2a*mid + e2b*lo. Float products and
+// sums are rounded one by one (no FMA), as in the reference build. EDGE false: interior for certain.
+struct AxisPos {
+  bool first, last;
+};
+template <bool EDGE>
+__device__ __forceinline__ float pass3(AxisPos q, float lo, float mid, float hi, float f0, float f1, float f2, float e1a,
+                                       float e1b, float e2a, float e2b) {
+  float r = __fadd_rn(__fadd_rn(__fmul_rn(f0, lo), __fmul_rn(f1, mid)), __fmul_rn(f2, hi));
+  if (EDGE) {
+    if (q.first)
+      r = __fadd_rn(__fmul_rn(e1a, mid), __fmul_rn(e1b, hi));
+    else if (q.last)
+      r = __fadd_rn(__fmul_rn(e2a, mid), __fmul_rn(e2b, lo));
+  }
+  return r;
+}
+template <bool EDGE>
+__device__ __forceinline__ float smooth3(AxisPos q, float lo, float mid, float hi) {
+  return pass3<EDGE>(q, lo, mid, hi, 1.0f / 4.0f, 2.0f / 4.0f, 1.0f / 4.0f, 2.0f / 3.0f, 2.0f / 3.0f, 2.0f / 3.0f, 2.0f / 3.0f);
+}
+template <bool EDGE>
+__device__ __forceinline__ float diff3(AxisPos q, float lo, float mid, float hi) {
+  return pass3<EDGE>(q, lo, mid, hi, -0.5f, 0.0f, 0.5f, -0.5f, 0.5f, 0.5f, -0.5f);
 }
 
-// Sobel3d (Sobel3d.cpp:60-85) with each separable pass computed once per voxel: a CTA takes a tile of
-// kSbZ x kSbY x kSbX outputs, loads the reference over the tile plus a one-voxel halo (clipped to the
-// volume) into shared memory and forms the intermediate images there -- a = Sx(m) and a' = Sy(m) on
-// the halo, then b = Sy(a), c = Sz(a), b' = Sz(a'), then gz = Dz(b), gy = Dy(c), gx = Dx(b'). Every
-// value is produced by `pass` with the global index along its axis, so the edge rules apply at the
-// volume's faces and every product and sum is rounded in the reference's order: gx = Dx(Sz(Sy(m))),
-// gy = Dy(Sz(Sx(m))), gz = Dz(Sy(Sx(m))) (Sobel3d.cpp:73-84), bit for bit.
-constexpr int kSbX = 32, kSbY = 8, kSbZ = 4;
-constexpr int kSbHX = kSbX + 2, kSbHY = kSbY + 2, kSbHZ = kSbZ + 2;
-constexpr int kSbVol = kSbHX * kSbHY * kSbHZ;
+// Sobel3d (Sobel3d.cpp:60-85), gx = Dx(Sz(Sy(m))), gy = Dy(Sz(Sx(m))), gz = Dz(Sy(Sx(m))) (:73-84), bit
+// for bit: every value is formed by pass3 with its global position, so the edge rules apply at the
+// volume's faces and every product and sum is rounded in the reference's order. A thread marches along
+// z at one (x, y): of each plane it reads the 3 x 3 neighbourhood (nine loads, the cache serves eight) and
+// keeps Sx of the three rows, Sy of the three columns and Sy(Sx) for three planes, from which the plane in
+// the middle follows. With QUAD (nx a multiple of 4, so that a group of four voxels is four lanes) the
+// BF16 groups of RefDev::q16 are written in the same pass: four lanes exchange so that each writes one
+// quantity of the group.
+// HBM-bound in principle (4 B in, 12 or 20 B out per voxel: 15 us for 512 x 512 x 16 at the copy rate);
+// with the groups 40 us there, by instruction issue (131 + 39 us before: passes through shared memory with
+// a division per element and step, then a conversion of its own; the edge rules cost another 30 us
+// where no column of a CTA is at a face, so those CTAs take a march without them).
+constexpr int kSobX = 32, kSobY = 8;
 
-__global__ void __launch_bounds__(256) sobel_tiled_kernel(const float* __restrict__ m, int nz, int ny, int nx,
-                                                          float* __restrict__ gx, float* __restrict__ gy,
-                                                          float* __restrict__ gz) {
-  __shared__ float sM[kSbVol];   // m, later b
-  __shared__ float sA[kSbVol];   // a = Sx(m)
-  __shared__ float sA2[kSbVol];  // a' = Sy(m)
-  __shared__ float sC[kSbVol];   // c = Sz(a)
-  __shared__ float sB2[kSbVol];  // b' = Sz(a')
-  const float sm[3] = {1.0f / 4.0f, 2.0f / 4.0f, 1.0f / 4.0f};
-  const float se[2] = {2.0f / 3.0f, 2.0f / 3.0f};
-  const float dm[3] = {-0.5f, 0.0f, 0.5f};
-  const float de1[2] = {-0.5f, 0.5f};
-  const float de2[2] = {0.5f, -0.5f};
-  const int x0 = blockIdx.x * kSbX, y0 = blockIdx.y * kSbY, z0 = blockIdx.z * kSbZ;
-  // local index of global (z, y, x): origin at (z0 - 1, y0 - 1, x0 - 1)
-  auto L = [&](int z, int y, int x) { return ((z - z0 + 1) * kSbHY + (y - y0 + 1)) * kSbHX + (x - x0 + 1); };
-  // a range [lo, hi) of global positions along an axis, clipped to the volume
-  const int hz0 = max(z0 - 1, 0), hz1 = min(z0 + kSbZ + 1, nz), tz1 = min(z0 + kSbZ, nz);
-  const int hy0 = max(y0 - 1, 0), hy1 = min(y0 + kSbY + 1, ny), ty1 = min(y0 + kSbY, ny);
-  const int hx0 = max(x0 - 1, 0), hx1 = min(x0 + kSbX + 1, nx), tx1 = min(x0 + kSbX, nx);
-  // run f(z, y, x) over a box
-  auto box = [&](int za, int zb, int ya, int yb, int xa, int xb, auto f) {
-    const int wx = xb - xa, wy = yb - ya, n = (zb - za) * wy * wx;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const int x = xa + i % wx, r = i / wx;
-      f(za + r / wy, ya + r % wy, x);
-    }
+// The march of one CTA; EDGE: some of its columns are at a face along x or y.
+template <bool QUAD, bool EDGE>
+__device__ __forceinline__ void sobel_march(const float* __restrict__ m, int nz, int ny, int nx, int zc,
+                                            float* __restrict__ gx, float* __restrict__ gy, float* __restrict__ gz,
+                                            __nv_bfloat16* __restrict__ q16) {
+  const int x = blockIdx.x * kSobX + threadIdx.x, y = blockIdx.y * kSobY + threadIdx.y;
+  const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, nz);
+  if (y >= ny) return;  // whole warps: a warp is one row
+  const bool in = x < nx;
+  const int xc = min(x, nx - 1);
+  const int xs[3] = {max(xc - 1, 0), xc, min(xc + 1, nx - 1)};
+  const int ys[3] = {max(y - 1, 0), y, min(y + 1, ny - 1)};
+  const AxisPos px{xc == 0, xc == nx - 1}, py{y == 0, y == ny - 1};  // a clamped neighbour is never used
+  const int plane = ny * nx;  // fewer than 2^31 voxels
+  float A[3][3], A2[3][3], B[3];  // [plane][row]: Sx(m); [plane][column]: Sy(m); [plane]: Sy(Sx(m))
+  float mid[3];                   // the reference itself
+  auto load = [&](int z, float* a, float* a2, float& b, float& v) {
+    const float* p = m + min(max(z, 0), nz - 1) * plane;
+    float w[3][3];
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) w[j][i] = __ldg(p + ys[j] * nx + xs[i]);
+#pragma unroll
+    for (int j = 0; j < 3; j++) a[j] = smooth3<EDGE>(px, w[j][0], w[j][1], w[j][2]);
+#pragma unroll
+    for (int i = 0; i < 3; i++) a2[i] = smooth3<EDGE>(py, w[0][i], w[1][i], w[2][i]);
+    b = smooth3<EDGE>(py, a[0], a[1], a[2]);
+    v = w[1][1];
   };
-  box(hz0, hz1, hy0, hy1, hx0, hx1,
-      [&](int z, int y, int x) { sM[L(z, y, x)] = __ldg(m + ((long long)z * ny + y) * nx + x); });
-  __syncthreads();
-  // a = Sx(m) on (halo z, halo y, tile x); a' = Sy(m) on (halo z, tile y, halo x)
-  box(hz0, hz1, hy0, hy1, x0, tx1, [&](int z, int y, int x) {
-    sA[L(z, y, x)] = pass(x, nx, false, sm, se, se, [&](int k) { return sM[L(z, y, k)]; });
-  });
-  box(hz0, hz1, y0, ty1, hx0, hx1, [&](int z, int y, int x) {
-    sA2[L(z, y, x)] = pass(y, ny, false, sm, se, se, [&](int k) { return sM[L(z, k, x)]; });
-  });
-  __syncthreads();
-  // b = Sy(a) on (halo z, tile y, tile x) into sM; c = Sz(a) on (tile z, halo y, tile x);
-  // b' = Sz(a') on (tile z, tile y, halo x)
-  box(hz0, hz1, y0, ty1, x0, tx1, [&](int z, int y, int x) {
-    sM[L(z, y, x)] = pass(y, ny, false, sm, se, se, [&](int k) { return sA[L(z, k, x)]; });
-  });
-  box(z0, tz1, hy0, hy1, x0, tx1, [&](int z, int y, int x) {
-    sC[L(z, y, x)] = pass(z, nz, true, sm, se, se, [&](int k) { return sA[L(k, y, x)]; });
-  });
-  box(z0, tz1, y0, ty1, hx0, hx1, [&](int z, int y, int x) {
-    sB2[L(z, y, x)] = pass(z, nz, true, sm, se, se, [&](int k) { return sA2[L(k, y, x)]; });
-  });
-  __syncthreads();
-  box(z0, tz1, y0, ty1, x0, tx1, [&](int z, int y, int x) {
-    const long long p = ((long long)z * ny + y) * nx + x;
-    gz[p] = pass(z, nz, true, dm, de1, de2, [&](int k) { return sM[L(k, y, x)]; });
-    gy[p] = pass(y, ny, false, dm, de1, de2, [&](int k) { return sC[L(z, k, x)]; });
-    gx[p] = pass(x, nx, false, dm, de1, de2, [&](int k) { return sB2[L(z, y, k)]; });
-  });
+  load(z0 - 1, A[0], A2[0], B[0], mid[0]);
+  load(z0, A[1], A2[1], B[1], mid[1]);
+#pragma unroll 1
+  for (int z = z0; z < z1; z++) {
+    load(z + 1, A[2], A2[2], B[2], mid[2]);
+    float c[3], b2[3], g[3];
+    if (nz > 1 && z > 0 && z < nz - 1) {
+      const AxisPos pz{false, false};
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        c[i] = smooth3<false>(pz, A[0][i], A[1][i], A[2][i]);
+        b2[i] = smooth3<false>(pz, A2[0][i], A2[1][i], A2[2][i]);
+      }
+      g[2] = diff3<false>(pz, B[0], B[1], B[2]);
+    } else {  // a single plane is copied by the z passes
+      const AxisPos pz{z == 0, z == nz - 1};
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        c[i] = nz == 1 ? A[1][i] : smooth3<true>(pz, A[0][i], A[1][i], A[2][i]);
+        b2[i] = nz == 1 ? A2[1][i] : smooth3<true>(pz, A2[0][i], A2[1][i], A2[2][i]);
+      }
+      g[2] = nz == 1 ? B[1] : diff3<true>(pz, B[0], B[1], B[2]);
+    }
+    g[0] = diff3<EDGE>(px, b2[0], b2[1], b2[2]);
+    g[1] = diff3<EDGE>(py, c[0], c[1], c[2]);
+    const int p = z * plane + y * nx + x;
+    if (in) {
+      gx[p] = g[0];
+      gy[p] = g[1];
+      gz[p] = g[2];
+    }
+    if (QUAD) {
+      // four lanes hold a group of four voxels, four quantities each; lane j has to hold quantity j of the
+      // four: a 4 x 4 transpose in two exchanges
+      const int j = threadIdx.x & 3;
+      float q[4] = {mid[1], g[0], g[1], g[2]};
+      const bool odd = j & 1, high = j & 2;
+      const float s0 = __shfl_xor_sync(0xffffffffu, odd ? q[0] : q[1], 1), s1 = __shfl_xor_sync(0xffffffffu, odd ? q[2] : q[3], 1);
+      if (odd) {
+        q[0] = s0;
+        q[2] = s1;
+      } else {
+        q[1] = s0;
+        q[3] = s1;
+      }
+      const float t0 = __shfl_xor_sync(0xffffffffu, high ? q[0] : q[2], 2), t1 = __shfl_xor_sync(0xffffffffu, high ? q[1] : q[3], 2);
+      if (high) {
+        q[0] = t0;
+        q[1] = t1;
+      } else {
+        q[2] = t0;
+        q[3] = t1;
+      }
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(q[0], q[1]), hi = __floats2bfloat162_rn(q[2], q[3]);
+      if (in)
+        *reinterpret_cast<uint2*>(q16 + (long long)(p >> 2) * 16 + j * 4) =
+            make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      A[0][i] = A[1][i];
+      A[1][i] = A[2][i];
+      A2[0][i] = A2[1][i];
+      A2[1][i] = A2[2][i];
+    }
+    B[0] = B[1];
+    B[1] = B[2];
+    mid[1] = mid[2];
+  }
 }
 
-cudaError_t launch_sobel(const float* m, int nz, int ny, int nx, float* gx, float* gy, float* gz, cudaStream_t s) {
-  const dim3 grid((nx + kSbX - 1) / kSbX, (ny + kSbY - 1) / kSbY, (nz + kSbZ - 1) / kSbZ);
-  sobel_tiled_kernel<<<grid, 256, 0, s>>>(m, nz, ny, nx, gx, gy, gz);
-  return cudaGetLastError();
+template <bool QUAD>
+__global__ void __launch_bounds__(kSobX * kSobY) sobel_kernel(const float* __restrict__ m, int nz, int ny, int nx,
+                                                             int zc, float* __restrict__ gx, float* __restrict__ gy,
+                                                             float* __restrict__ gz, __nv_bfloat16* __restrict__ q16) {
+  const bool edge = blockIdx.x == 0 || blockIdx.y == 0 || (int)(blockIdx.x + 1) * kSobX >= nx ||
+                    (int)(blockIdx.y + 1) * kSobY >= ny;
+  if (edge)
+    sobel_march<QUAD, true>(m, nz, ny, nx, zc, gx, gy, gz, q16);
+  else
+    sobel_march<QUAD, false>(m, nz, ny, nx, zc, gx, gy, gz, q16);
+}
+
+cudaError_t launch_sobel(const float* m, int nz, int ny, int nx, float* gx, float* gy, float* gz, __nv_bfloat16* q16,
+                         cudaStream_t s) {
+  // planes per CTA: the march pays two extra planes per chunk, a short one fills the GPU
+  const long long cols = (long long)((nx + kSobX - 1) / kSobX) * ((ny + kSobY - 1) / kSobY);
+  int zc = nz;
+  while (zc > 4 && cols * ((nz + zc - 1) / zc) < 148 * 8) zc = (zc + 1) / 2;
+  const dim3 grid((nx + kSobX - 1) / kSobX, (ny + kSobY - 1) / kSobY, (nz + zc - 1) / zc), block(kSobX, kSobY);
+  if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
+  if (q16 != nullptr && nx % 4 == 0) {
+    sobel_kernel<true><<<grid, block, 0, s>>>(m, nz, ny, nx, zc, gx, gy, gz, q16);
+    return cudaGetLastError();
+  }
+  sobel_kernel<false><<<grid, block, 0, s>>>(m, nz, ny, nx, zc, gx, gy, gz, nullptr);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && q16 != nullptr) e = launch_to_quad16(m, gx, gy, gz, (long long)nz * ny * nx, q16, s);
+  return e;
 }
 
 // ------------------------------------------------------------------ conversions ------------------
@@ -537,25 +621,47 @@ cudaError_t launch_warp(const RefDev* ref_dev, const RefDev& R, const void* fram
 // (FrameWarper.cpp:258-259, 319-342), over the voxels of the range that are not its last.
 constexpr int kHessTerms = 21;
 
+// The block tree of one CTA's 256 values of a term: run t takes run t + w, w = 128, 64, ..., 1, by one warp.
+__device__ __forceinline__ double tree256(const double* v, int lane) {
+  double a = ((v[lane] + v[lane + 128]) + (v[lane + 64] + v[lane + 192])) +
+             ((v[lane + 32] + v[lane + 160]) + (v[lane + 96] + v[lane + 224]));
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) a += __shfl_down_sync(0xffffffffu, a, w);
+  return a;
+}
+
+// What bounded it were the reductions, 21 block trees of eight barriers each, and the second slot's pass
+// over tiles that have only one range: the trees are now one warp's each after one barrier (the same
+// order), and an empty slot is written as zeros. 512 x 512 x 16: 134 -> 63 us, now the FP64 division and
+// the 21 conversions and sums of every voxel.
 template <int NDIM>
 __global__ void __launch_bounds__(256) hessian_tile_kernel(const RefDev* __restrict__ Rp, double pd, double ild,
                                                            double ifd, double stack, double* __restrict__ parts) {
   const RefDev& R = *Rp;
   const int tile = blockIdx.x;
   const int slot = blockIdx.y;
-  const int nx = R.nx, ny = R.ny;
+  const int nx = R.nx;
   const int row_begin = tile * R.tile_rows;
   const int row_end = min(row_begin + R.tile_rows, R.n_rows);
   const int c0 = R.tile_c0[tile];
   const double nDm1 = (double)(R.nD - 1);
   constexpr int NU = NDIM * (NDIM + 1) / 2;
-  double acc[2 * NU + NDIM * NDIM];
+  constexpr int kTerms = 2 * NU + NDIM * NDIM;
+  double* out = parts + ((long long)tile * 2 + slot) * kHessTerms;
+  if (slot == 1) {  // the ranges do not decrease: the tile has a second one if its last row reaches it
+    const RowDesc rl = R.rows[row_end - 1];
+    const int last = R.bidir ? rl.r0 + (rl.xr < nx ? 1 : 0) : rl.di0 + (rl.xdi < nx ? 1 : 0);
+    if (last == c0) {
+      if (threadIdx.x < kTerms) out[threadIdx.x] = 0.0;
+      return;
+    }
+  }
+  double acc[kTerms];
 #pragma unroll
-  for (int i = 0; i < 2 * NU + NDIM * NDIM; i++) acc[i] = 0.0;
+  for (int i = 0; i < kTerms; i++) acc[i] = 0.0;
   for (int row = row_begin; row < row_end; row++) {
     const RowDesc rd = R.rows[row];
-    const int z = row / ny;
-    const int y = row - z * ny;
+    const int z = rd.z, y = rd.y;
     const bool flip = R.bidir && (y & 1);
     for (int x = threadIdx.x; x < nx; x += blockDim.x) {
       const int r = R.bidir ? rd.r0 + (x >= rd.xr ? 1 : 0) : rd.di0 + (x >= rd.xdi ? 1 : 0);
@@ -591,58 +697,68 @@ __global__ void __launch_bounds__(256) hessian_tile_kernel(const RefDev* __restr
         for (int b = 0; b < NDIM; b++) acc[2 * NU + a * NDIM + b] += (double)__fmul_rn(v1[a], v0[b]);
     }
   }
-  __shared__ double sacc[256];
-  double* out = parts + ((long long)tile * 2 + slot) * kHessTerms;
-  for (int i = 0; i < 2 * NU + NDIM * NDIM; i++) {
-    sacc[threadIdx.x] = acc[i];
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-      if (threadIdx.x < w) sacc[threadIdx.x] += sacc[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[i] = sacc[0];
-    __syncthreads();
+  __shared__ double sacc[kTerms][256];
+#pragma unroll
+  for (int i = 0; i < kTerms; i++) sacc[i][threadIdx.x] = acc[i];
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int i = warp; i < kTerms; i += 8) {
+    const double a = tree256(sacc[i], lane);
+    if (lane == 0) out[i] = a;
   }
 }
 
-// Hd[c] = sum_t A(t, c - c0_t) + B(t, c - 1 - c0_t);  Hl[c] = sum_t C(t, c - 1 - c0_t).
+// Hd[c] = sum_t A(t, c - c0_t) + B(t, c - 1 - c0_t);  Hl[c] = sum_t C(t, c - 1 - c0_t), one thread per entry,
+// each in tile order (first the range c, then c - 1: at most one of a tile's two slots is either) with
+// the loads of eight tiles in flight (one thread per control point: 138 us for 32 of them, now 14).
 template <int NDIM>
-__global__ void hessian_reduce_kernel(const RefDev* __restrict__ Rp, const double* __restrict__ parts,
-                                      double* __restrict__ Hd, double* __restrict__ Hl) {
+__global__ void __launch_bounds__(64) hessian_reduce_kernel(const RefDev* __restrict__ Rp,
+                                                            const double* __restrict__ parts, double* __restrict__ Hd,
+                                                            double* __restrict__ Hl) {
   const RefDev& R = *Rp;
-  constexpr int NU = NDIM * (NDIM + 1) / 2;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= R.nD) return;
-  double d[NDIM * NDIM], l[NDIM * NDIM];
-  for (int i = 0; i < NDIM * NDIM; i++) d[i] = l[i] = 0.0;
-  const int t0 = R.ctrl_tiles[c].x, t1 = R.ctrl_tiles[c].w;
-  for (int t = t0; t < t1; t++) {
-    const int ct = R.tile_c0[t];
-    for (int s = 0; s < 2; s++) {
-      const double* pt = parts + ((long long)t * 2 + s) * kHessTerms;
-      const int r = ct + s;
-      if (r == c) {
-        int u = 0;
-        for (int a = 0; a < NDIM; a++)
-          for (int b = a; b < NDIM; b++, u++) {
-            d[a * NDIM + b] += pt[u];
-            if (a != b) d[b * NDIM + a] += pt[u];
-          }
-      }
-      if (r + 1 == c) {
-        int u = 0;
-        for (int a = 0; a < NDIM; a++)
-          for (int b = a; b < NDIM; b++, u++) {
-            d[a * NDIM + b] += pt[NU + u];
-            if (a != b) d[b * NDIM + a] += pt[NU + u];
-          }
-        for (int a = 0; a < NDIM * NDIM; a++) l[a] += pt[2 * NU + a];
+  constexpr int NU = NDIM * (NDIM + 1) / 2, NN = NDIM * NDIM;
+  const int c = blockIdx.x;
+  const int4 tr = R.ctrl_tiles[c];
+  if (threadIdx.x >= NU + NN) return;
+  const bool diag = threadIdx.x < NU;
+  const int i = diag ? threadIdx.x : threadIdx.x - NU;
+  double h = 0.0;
+  // tiles that start at range c - 2 hold range c - 1 in slot 1; at c - 1, range c - 1 in slot 0 and range c in
+  // slot 1; at c, range c in slot 0
+  constexpr int kDepth = 8;
+  for (int t = tr.x; t < tr.w; t += kDepth) {
+    double v[kDepth][2];
+#pragma unroll
+    for (int u = 0; u < kDepth; u++) {
+      const int tt = min(t + u, tr.w - 1);
+      const double* p0 = parts + (long long)tt * 2 * kHessTerms;
+      const double* p1 = p0 + kHessTerms;
+      if (diag) {
+        v[u][0] = tt < tr.y ? 0.0 : (tt < tr.z ? p0[NU + i] : p0[i]);
+        v[u][1] = tt < tr.y ? p1[NU + i] : (tt < tr.z ? p1[i] : 0.0);
+      } else {
+        v[u][0] = tt >= tr.y && tt < tr.z ? p0[2 * NU + i] : 0.0;
+        v[u][1] = tt < tr.y ? p1[2 * NU + i] : 0.0;
       }
     }
+#pragma unroll
+    for (int u = 0; u < kDepth; u++)
+      if (t + u < tr.w) {
+        h += v[u][0];
+        h += v[u][1];
+      }
   }
-  for (int i = 0; i < NDIM * NDIM; i++) {
-    Hd[c * NDIM * NDIM + i] = d[i];
-    Hl[c * NDIM * NDIM + i] = l[i];
+  if (diag) {
+    int a = 0, b = i;
+    while (b >= NDIM - a) {  // entry i of the upper triangle, row by row
+      b -= NDIM - a;
+      a++;
+    }
+    b += a;
+    Hd[c * NN + a * NDIM + b] = h;
+    Hd[c * NN + b * NDIM + a] = h;
+  } else {
+    Hl[c * NN + i] = h;
   }
 }
 
@@ -651,10 +767,10 @@ cudaError_t launch_hessian(const RefDev* ref_dev, const RefDev& R, const double*
   dim3 grid(R.n_tiles, 2);
   if (R.n_dim == 3) {
     hessian_tile_kernel<3><<<grid, 256, 0, s>>>(ref_dev, scan4[0], scan4[1], scan4[2], scan4[3], tile_parts);
-    hessian_reduce_kernel<3><<<(R.nD + 127) / 128, 128, 0, s>>>(ref_dev, tile_parts, Hd, Hl);
+    hessian_reduce_kernel<3><<<R.nD, 64, 0, s>>>(ref_dev, tile_parts, Hd, Hl);
   } else {
     hessian_tile_kernel<2><<<grid, 256, 0, s>>>(ref_dev, scan4[0], scan4[1], scan4[2], scan4[3], tile_parts);
-    hessian_reduce_kernel<2><<<(R.nD + 127) / 128, 128, 0, s>>>(ref_dev, tile_parts, Hd, Hl);
+    hessian_reduce_kernel<2><<<R.nD, 64, 0, s>>>(ref_dev, tile_parts, Hd, Hl);
   }
   return cudaGetLastError();
 }

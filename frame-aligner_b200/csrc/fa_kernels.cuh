@@ -14,8 +14,9 @@ constexpr int kEvalWarps = kEvalThreads / 32;
 constexpr int kReduceRuns = 128;
 constexpr int kSolveThreads = 256;
 
-// Exact float Sobel3d (Sobel3d.cpp:60-85) of an FP32 volume.
-cudaError_t launch_sobel(const float* m, int nz, int ny, int nx, float* gx, float* gy, float* gz,
+// Exact float Sobel3d (Sobel3d.cpp:60-85) of an FP32 volume; with q16 also the BF16 groups of
+// launch_to_quad16.
+cudaError_t launch_sobel(const float* m, int nz, int ny, int nx, float* gx, float* gy, float* gz, __nv_bfloat16* q16,
                          cudaStream_t s);
 
 // Per-tile Hessian partials (exact Df per voxel, FP32 products, FP64 sums) and their reduction
