@@ -411,9 +411,9 @@ fa_status autotune(fa_reference* R) {
   if (st == FA_OK) st = dalloc_t(ctx, (size_t)R->nD * fa::kDParamF4, &dp, tmp);
   if (st == FA_OK) st = dalloc_t(ctx, (size_t)K * R->G.n_rows * fa::kPartialDoubles, &parts, tmp);
   if (st == FA_OK) st = dalloc_t(ctx, (size_t)K, &jobs_dev, tmp);
-  if (st == FA_OK) st = dalloc_t(ctx, (size_t)K, &list, tmp);
+  if (st == FA_OK) st = dalloc_t(ctx, (size_t)K + fa::kListSlack, &list, tmp);
   if (st == FA_OK) st = dalloc_t(ctx, 1, &cnt, tmp);
-  if (st == FA_OK) st = dalloc_t(ctx, (size_t)K + 1, &prefix, tmp);
+  if (st == FA_OK) st = dalloc_t(ctx, (size_t)K + 1 + fa::kListSlack, &prefix, tmp);
   if (st != FA_OK) return done(st);
   cudaStream_t s = R->stream;
   void* interior = static_cast<char*>(frame) + ((long long)hz * plane + (long long)fa::kHaloY * pitch + fa::kHaloX) * esz;
@@ -435,7 +435,6 @@ fa_status autotune(fa_reference* R) {
   std::vector<int> all(K);
   for (int i = 0; i < K; i++) {
     Job j{};
-    j.ref = R->dev;
     j.frame = static_cast<char*>(interior) + (size_t)i * elems * esz;
     j.fplane = plane;
     j.fpitch = pitch;
@@ -470,7 +469,9 @@ fa_status autotune(fa_reference* R) {
     const int target = targets[ti];
     if (retile(R, target) != FA_OK) break;
     for (int i = 0; i <= K; i++) hprefix[i] = i * R->G.n_tiles;
-    e = cudaMemcpyAsync(prefix, hprefix.data(), (K + 1) * sizeof(int), cudaMemcpyHostToDevice, s);
+    for (Job& j : jobs) j.R = R->host;  // this tile size's tables
+    e = cudaMemcpyAsync(jobs_dev, jobs.data(), K * sizeof(Job), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(prefix, hprefix.data(), (K + 1) * sizeof(int), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) break;
     for (int mi = 0; mi < 3; mi++) {
@@ -784,7 +785,7 @@ fa_status frame_alloc(fa_reference* R, int kind, fa_frame** out) {
   const long long origin = (long long)hz * plane + (long long)fa::kHaloY * pitch + fa::kHaloX;
   F->data = static_cast<char*>(data) + origin * esz;  // voxel (0, 0, 0)
   Job& j = F->job;
-  j.ref = R->dev;
+  j.R = R->host;
   j.frame = F->data;
   j.fplane = plane;
   j.fpitch = pitch;
@@ -1109,8 +1110,8 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     batch_cache_release(ctx, bc);
     FA_TRY(dalloc_t(ctx, (size_t)n, &bc->jobs_dev, bc->allocs));
     FA_TRY(dalloc_t(ctx, 4, &bc->d_active, bc->allocs));
-    FA_TRY(dalloc_t(ctx, 2 * (size_t)n, &bc->d_list, bc->allocs));
-    FA_TRY(dalloc_t(ctx, (size_t)n + 1, &bc->d_prefix, bc->allocs));
+    FA_TRY(dalloc_t(ctx, 2 * (size_t)n + fa::kListSlack, &bc->d_list, bc->allocs));
+    FA_TRY(dalloc_t(ctx, 2 * (size_t)n + 1 + fa::kListSlack, &bc->d_prefix, bc->allocs));
     void* hp = nullptr;
     if (cudaHostAlloc(&hp, out_bytes, cudaHostAllocMapped) != cudaSuccess) {
       cudaGetLastError();
@@ -1171,6 +1172,7 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     o.active = bc->d_list + (size_t)which * bc->cap;
     o.n_active = bc->d_active + which;
     o.prefix = bc->d_prefix;
+    o.items = bc->d_prefix + bc->cap + 1;
     o.rounds = bc->d_active + 2;
     o.rounds_host = reinterpret_cast<int*>(bc->d_out);
     o.max_rounds = max_rounds;
@@ -2228,11 +2230,10 @@ extern "C" fa_status fa_profile_eval(fa_frame* const* frames, int n, const doubl
 
 namespace fa {
 
-fa_status static_eval_prepare(const fa_reference* R, const double* D, const RefDev** dev, const RefDev** host, int* nD,
-                              int* n_dim, bool* mixed, int* device) {
+fa_status static_eval_prepare(const fa_reference* R, const double* D, const RefDev** host, int* nD, int* n_dim,
+                              bool* mixed, int* device) {
   if (!finite_all(D, (size_t)R->nD * 3)) return fail(FA_ERR_BAD_ARG, "D has non-finite entries");
   *device = R->ctx->device;
-  *dev = R->dev;
   *host = &R->host;
   *nD = R->nD;
   *n_dim = R->n_dim;

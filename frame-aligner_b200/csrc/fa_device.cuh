@@ -207,44 +207,36 @@ __device__ __forceinline__ void write_const_dparams(float4* dp, int nD, int nd, 
   }
 }
 
-// Rebuilds the active list of a job table by one block (see ActiveOut): ballots give each warp's active /
-// done counts, a shuffle scan the tile prefix inside a warp, and one thread the per-warp offsets. States
-// are read past the L1 cache: other CTAs of the same launch may have written them.
-__device__ __forceinline__ void compact_block(const Job* __restrict__ jobs, const ActiveOut& out) {
+// An active list by one block from n entries in order: get(i) gives an entry's job, its items in the next
+// pass (0: not active) and whether it goes to the done list; between(c) runs on the whole block after the
+// entries of a chunk were read. Ballots give each warp's active / done counts, a shuffle scan the tile
+// prefix inside a warp, and one thread the per-warp offsets.
+struct ListEntry {
+  int job, items;
+  bool fin;
+};
+template <class Get, class Between>
+__device__ __forceinline__ void list_block(int n, const ActiveOut& out, Get get, Between between) {
   __shared__ int s_act[32], s_tiles[32], s_done[32];
   __shared__ int base_a, base_t, base_d, tot_a, tot_t, tot_d;
-  __shared__ int s_resume[256], n_resume;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (threadIdx.x == 0) {
     base_a = 0;
     base_t = 0;
     base_d = out.busy != nullptr ? *out.n_done : 0;
-    n_resume = 0;
   }
   __syncthreads();
   const unsigned lt = (1u << lane) - 1u;
-  for (int c = 0; c < out.n_jobs; c += blockDim.x) {  // (at most 256 threads: s_resume)
+  for (int c = 0; c < n; c += blockDim.x) {
     const int i = c + threadIdx.x;
-    int phase = i < out.n_jobs ? __ldcg(&jobs[i].state->phase) : (int)kPhaseDone;
-    if (phase == kPhaseWaitWarm) {
-      // Resume a frame waiting for its warm start once the earlier frame's solution is written (by a
-      // finished solve step): the fourth starting point x + (warm - x), set by the whole block below.
-      const FrameState* S = jobs[i].state;
-      if (__ldcg(S->warm_seq) == __ldcg(&S->warm_need)) {
-        s_resume[atomicAdd(&n_resume, 1)] = i;
-        phase = kPhaseStartLast;
-      }
-    }
-    const bool act = i < out.n_jobs && phase != kPhaseDone && phase != kPhaseWaitWarm;
-    const bool fin = i < out.n_jobs && out.busy != nullptr && phase == kPhaseDone && out.busy[i] != 0;
-    const int tiles = act ? jobs[i].ref->n_tiles * (phase == kPhaseStartPair ? 2 : 1) : 0;
-    int incl = tiles;
+    const ListEntry e = i < n ? get(i) : ListEntry{0, 0, false};
+    int incl = e.items;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int v = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += v;
     }
-    const unsigned ma = __ballot_sync(0xffffffffu, act), md = __ballot_sync(0xffffffffu, fin);
+    const unsigned ma = __ballot_sync(0xffffffffu, e.items > 0), md = __ballot_sync(0xffffffffu, e.fin);
     if (lane == 31) s_tiles[w] = incl;
     if (lane == 0) {
       s_act[w] = __popc(ma);
@@ -267,31 +259,21 @@ __device__ __forceinline__ void compact_block(const Job* __restrict__ jobs, cons
       tot_d = d;
     }
     __syncthreads();
-    if (act) {
+    if (e.items > 0) {
       const int pos = base_a + s_act[w] + __popc(ma & lt);
-      out.active[pos] = i;
-      out.prefix[pos] = base_t + s_tiles[w] + incl - tiles;
+      out.active[pos] = e.job;
+      out.prefix[pos] = base_t + s_tiles[w] + incl - e.items;
     }
-    if (fin) {
-      out.done_list[base_d + s_done[w] + __popc(md & lt)] = i;
-      out.busy[i] = 0;
+    if (e.fin) {
+      out.done_list[base_d + s_done[w] + __popc(md & lt)] = e.job;
+      out.busy[e.job] = 0;
     }
-    for (int r = 0; r < n_resume; r++) {
-      const Job& j = jobs[s_resume[r]];
-      const RefDev& R = *j.ref;
-      FrameState* S = j.state;
-      const double* warm = S->warm;
-      for (int q = threadIdx.x; q < R.P; q += blockDim.x) j.p[q] = __ldcg(warm + q) - __ldcg(j.x + q);
-      __syncthreads();
-      write_trial_dparams(j.dparams, j.x, j.p, R.nD, R.n_dim, threadIdx.x, blockDim.x);
-      if (threadIdx.x == 0) S->phase = kPhaseStartLast;
-    }
+    between();
     __syncthreads();
     if (threadIdx.x == 0) {
       base_a += tot_a;
       base_t += tot_t;
       base_d += tot_d;
-      n_resume = 0;
     }
     __syncthreads();
   }
@@ -300,6 +282,45 @@ __device__ __forceinline__ void compact_block(const Job* __restrict__ jobs, cons
     out.prefix[base_a] = base_t;
     if (out.busy != nullptr) *out.n_done = base_d;
   }
+}
+
+// The active list of a whole job table (see ActiveOut), at most 256 threads. States are read past the L1
+// cache: other CTAs of the same launch may have written them.
+__device__ __forceinline__ void compact_block(const Job* __restrict__ jobs, const ActiveOut& out) {
+  __shared__ int s_resume[256], n_resume;
+  if (threadIdx.x == 0) n_resume = 0;
+  __syncthreads();
+  list_block(
+      out.n_jobs, out,
+      [&](int i) {
+        int phase = __ldcg(&jobs[i].state->phase);
+        if (phase == kPhaseWaitWarm) {
+          // Resume a frame waiting for its warm start once the earlier frame's solution is written (by a
+          // finished solve step): the fourth starting point x + (warm - x), set by the whole block below.
+          const FrameState* S = jobs[i].state;
+          if (__ldcg(S->warm_seq) == __ldcg(&S->warm_need)) {
+            s_resume[atomicAdd(&n_resume, 1)] = i;
+            phase = kPhaseStartLast;
+          }
+        }
+        const bool act = phase != kPhaseDone && phase != kPhaseWaitWarm;
+        return ListEntry{i, act ? jobs[i].R.n_tiles * (phase == kPhaseStartPair ? 2 : 1) : 0,
+                         out.busy != nullptr && phase == kPhaseDone && out.busy[i] != 0};
+      },
+      [&]() {
+        for (int r = 0; r < n_resume; r++) {
+          const Job& j = jobs[s_resume[r]];
+          const RefDev& R = j.R;
+          FrameState* S = j.state;
+          const double* warm = S->warm;
+          for (int q = threadIdx.x; q < R.P; q += blockDim.x) j.p[q] = __ldcg(warm + q) - __ldcg(j.x + q);
+          __syncthreads();
+          write_trial_dparams(j.dparams, j.x, j.p, R.nD, R.n_dim, threadIdx.x, blockDim.x);
+          if (threadIdx.x == 0) S->phase = kPhaseStartLast;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) n_resume = 0;
+      });
 }
 
 }  // namespace fa

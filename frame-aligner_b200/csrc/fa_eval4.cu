@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(kEvalThreads, MB) eval4_kernel(const Job* __re
   __shared__ float sg[kEvalWarps][9 * 32];
   const Job& job = jobs[blockIdx.y];
   if (job.state != nullptr && (job.state->phase == kPhaseDone || job.state->phase == kPhaseWaitWarm)) return;
-  const RefDev& R = *job.ref;
+  const RefDev& R = job.R;
   const int warp = threadIdx.x >> 5;
   const int tile = blockIdx.x * kEvalWarps + warp;
   if (tile >= R.n_tiles) return;
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval4_cta_kernel(const Job* _
   auto& sm = *reinterpret_cast<CtaTileSmem<NDIM, RT>*>(s_cta);
   const Job& job = jobs[blockIdx.y];
   if (job.state != nullptr && (job.state->phase == kPhaseDone || job.state->phase == kPhaseWaitWarm)) return;
-  const RefDev& R = *job.ref;
+  const RefDev& R = job.R;
   if ((int)blockIdx.x >= R.n_tiles) return;
   eval4_tile_cta<NDIM, FT, RT>(job, R, blockIdx.x, sm, job.dparams, job.partials);
 }
@@ -922,7 +922,7 @@ __device__ __forceinline__ ActiveItem active_item(const Job* __restrict__ jobs, 
       hi = mid - 1;
   }
   ActiveItem it{&jobs[active[a]], item - tile_prefix[a], false};
-  const int n_tiles = it.job->ref->n_tiles;
+  const int n_tiles = it.job->R.n_tiles;
   it.second = it.tile >= n_tiles;
   if (it.second) it.tile -= n_tiles;
   return it;
@@ -948,7 +948,7 @@ __global__ void __launch_bounds__(kEvalThreads, MB) eval4_active_kernel(const Jo
   for (int item = blockIdx.x * kEvalWarps + warp; item < n_items; item += stride) {
     const ActiveItem it = active_item(jobs, active, tile_prefix, na, item, a);
     const Job& job = *it.job;
-    eval4_tile<NDIM, FT, RT, kPipe<FT, RT, MB>>(job, *job.ref, it.tile, sD[warp], sp[warp], sg[warp],
+    eval4_tile<NDIM, FT, RT, kPipe<FT, RT, MB>>(job, job.R, it.tile, sD[warp], sp[warp], sg[warp],
                                                 it.second ? job.dparams2 : job.dparams,
                                                 it.second ? job.partials2 : job.partials);
   }
@@ -961,14 +961,25 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval4_active_cta_kernel(const
                                                                         const int* __restrict__ tile_prefix, int few) {
   extern __shared__ float4 s_cta[];
   auto& sm = *reinterpret_cast<CtaTileSmem<NDIM, RT>*>(s_cta);
-  const int na = *n_active;
-  const int n_items = tile_prefix[na];
+  // (the lists have room for kListSlack entries more than jobs, so these loads need not wait for na)
+  const int lane = threadIdx.x & 31;
+  const int na = *n_active, prefix_l = tile_prefix[lane], active_l = active[lane];
+  const int n_items = na < 32 ? __shfl_sync(0xffffffffu, prefix_l, na) : tile_prefix[na];
   if (n_items > few) return;
   int a = 0;
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const ActiveItem it = active_item(jobs, active, tile_prefix, na, item, a);
+    ActiveItem it;
+    if (na <= 32) {  // one look at the list instead of a search through it
+      a = __popc(__ballot_sync(0xffffffffu, lane < na && prefix_l <= item)) - 1;
+      it.job = &jobs[__shfl_sync(0xffffffffu, active_l, a)];
+      it.tile = item - __shfl_sync(0xffffffffu, prefix_l, a);
+      it.second = it.tile >= it.job->R.n_tiles;
+      if (it.second) it.tile -= it.job->R.n_tiles;
+    } else {
+      it = active_item(jobs, active, tile_prefix, na, item, a);
+    }
     const Job& job = *it.job;
-    eval4_tile_cta<NDIM, FT, RT>(job, *job.ref, it.tile, sm, it.second ? job.dparams2 : job.dparams,
+    eval4_tile_cta<NDIM, FT, RT>(job, job.R, it.tile, sm, it.second ? job.dparams2 : job.dparams,
                                  it.second ? job.partials2 : job.partials);
   }
 }

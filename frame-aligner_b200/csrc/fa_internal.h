@@ -154,7 +154,7 @@ constexpr int kHaloY = 2;
 constexpr int kHaloZ = 2;  // planes, for volumes with nz > 1
 
 struct Job {
-  const RefDev* ref;      // device pointer
+  RefDev R;               // the frame's reference (a copy: one dependent load fewer in every kernel)
   const void* frame;      // device pointer to voxel (0, 0, 0); FrameKind storage
   long long fplane;       // elements between planes of the frame
   int fpitch;             // elements between rows of the frame

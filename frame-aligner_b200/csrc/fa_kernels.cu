@@ -426,7 +426,7 @@ template <int NDIM, typename FT, typename RT>
 __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const Job* __restrict__ jobs) {
   const Job& job = jobs[blockIdx.y];
   if (job.state != nullptr && (job.state->phase == kPhaseDone || job.state->phase == kPhaseWaitWarm)) return;
-  const RefDev& R = *job.ref;
+  const RefDev& R = job.R;
   const int tile = blockIdx.x;
   if (tile >= R.n_tiles) return;
   const int nx = R.nx, ny = R.ny, nz = R.nz;
@@ -557,7 +557,7 @@ cudaError_t launch_eval(const Job* jobs_dev, int n_jobs, int max_tiles, int n_di
 // ------------------------------------------------------------------ reductions -------------------
 
 __global__ void __launch_bounds__(kSolveThreads) reduce_kernel(const Job* __restrict__ job) {
-  const RefDev& R = *job->ref;
+  const RefDev& R = job->R;
   __shared__ double s_f;
   reduce_partials(R, job->partials, &s_f, job->result + 1);
   if (threadIdx.x == 0) job->result[0] = s_f;
@@ -792,7 +792,7 @@ cudaError_t launch_compact(const Job* jobs_dev, const ActiveOut& out, cudaStream
 __global__ void activate_kernel(const Job* __restrict__ jobs, const Activation* __restrict__ recs, int* busy) {
   const Activation r = recs[blockIdx.x];
   const Job& j = jobs[r.job];
-  const RefDev& R = *j.ref;
+  const RefDev& R = j.R;
   for (int i = threadIdx.x; i < R.P; i += blockDim.x) {
     j.x[i] = 0.0;
     j.g[i] = 0.0;
@@ -832,7 +832,7 @@ __global__ void activate_kernel(const Job* __restrict__ jobs, const Activation* 
 __global__ void activate_peaks_kernel(const Job* __restrict__ jobs, const long long* __restrict__ peaks, int cnx,
                                       int cny, int cnz, int binning, int max_iter, int pair) {
   const Job& j = jobs[blockIdx.x];
-  const RefDev& R = *j.ref;
+  const RefDev& R = j.R;
   const long long idx = peaks[blockIdx.x];
   long long x = idx % cnx, y = (idx / cnx) % cny, z = idx / ((long long)cnx * cny);
   if (x > cnx / 2) x -= cnx;

@@ -73,10 +73,12 @@ size_t eval4_active_local_bytes(int n_dim, int frame_kind, bool ref_bf16, int mb
 // done_list[*n_done ...] (busy is cleared). A frame waiting for a warm start that has been written is
 // resumed. In a device-side loop (rounds non-null) the list that ends a round also counts it and repeats
 // the loop while a frame is active and fewer than max_rounds rounds ran.
+constexpr int kListSlack = 32;  // entries that active and prefix have room for beyond n_jobs (+ 1)
 struct ActiveOut {
   int n_jobs;
   int *active, *n_active, *prefix;
   int *busy, *done_list, *n_done;
+  int* items;           // tables without busy flags: a step's CTA b leaves its frame's next item count here
   int* rounds;          // device counter, set to zero by launch_compact
   int* rounds_host;     // host-mapped copy
   int max_rounds;

@@ -23,7 +23,10 @@ constexpr size_t kStaticScratchBytes = size_t(2) << 20;  // 2 MiB
 
 // Host code never dereferences this name: it is a host-side stand-in for the device array. The
 // device address comes from cudaGetSymbolAddress below.
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+// The job descriptor has a block of its own in front of the scratch that the size limit counts.
+constexpr size_t kJobBytes = 1024;
+static_assert(sizeof(fa::Job) <= kJobBytes, "job descriptor");
+static __device__ __align__(256) unsigned char g_static_scratch[kJobBytes + kStaticScratchBytes];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
@@ -35,8 +38,8 @@ size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
 // Internal accessors into fa_api.cu (the reference layout is private to the runtime).
 namespace fa {
-fa_status static_eval_prepare(const fa_reference* ref, const double* D, const RefDev** dev, const RefDev** host, int* nD,
-                              int* n_dim, bool* mixed, int* device);
+fa_status static_eval_prepare(const fa_reference* ref, const double* D, const RefDev** host, int* nD, int* n_dim,
+                              bool* mixed, int* device);
 fa_status static_eval_fail(fa_status s, const char* msg);
 void static_eval_dparams(const double* D, int nD, int n_dim, float4* out);
 void static_eval_count_launches(int n);
@@ -44,20 +47,20 @@ void static_eval_count_launches(int n);
 
 extern "C" fa_status fa_get_error_jacobian_static(const fa_reference* ref, const void* frame_device, fa_dtype dtype,
                                                   const double* D, double* f, double* jac) {
-  const fa::RefDev* dev = nullptr;
   const fa::RefDev* host = nullptr;
   int nD = 0, n_dim = 0;
   bool mixed = false;
   int device = 0;
   if (!ref || !frame_device || !D || !f || !jac) return fa::static_eval_fail(FA_ERR_BAD_ARG, "NULL argument");
-  fa_status st = fa::static_eval_prepare(ref, D, &dev, &host, &nD, &n_dim, &mixed, &device);
+  fa_status st = fa::static_eval_prepare(ref, D, &host, &nD, &n_dim, &mixed, &device);
   if (st != FA_OK) return st;
   if (dtype != (mixed ? FA_F16 : FA_F32))
     return fa::static_eval_fail(FA_ERR_BAD_ARG, mixed ? "a mixed-precision reference needs FA_F16 frames"
                                                       : "an FP32 reference needs FA_F32 frames");
-  // Layout inside the array: Job | dparams (nD*3 float4) | result (1+P doubles) | tile partials.
+  // Layout inside the array: Job | dparams (nD*3 float4) | result (1+P doubles) | tile partials. The limit
+  // counts 256 bytes for the job.
   const int P = nD * n_dim;
-  const size_t off_dp = align256(sizeof(fa::Job));
+  const size_t off_dp = 256;
   const size_t off_res = off_dp + align256((size_t)nD * fa::kDParamF4 * sizeof(float4));
   const size_t off_parts = off_res + align256((size_t)(1 + P) * sizeof(double));
   const size_t need = off_parts + (size_t)host->n_tiles * fa::kPartialDoubles * sizeof(double);
@@ -93,14 +96,15 @@ extern "C" fa_status fa_get_error_jacobian_static(const fa_reference* ref, const
     base = static_cast<char*>(g_addr[device]);
   }
   fa::Job job{};
-  job.ref = dev;
+  job.R = *host;
   job.frame = frame_device;
   job.fplane = (long long)host->nx * host->ny;  // the caller's dense frame, no halo
   job.fpitch = host->nx;
   job.fpad = 0;
-  job.dparams = reinterpret_cast<float4*>(base + off_dp);
-  job.result = reinterpret_cast<double*>(base + off_res);
-  job.partials = reinterpret_cast<double*>(base + off_parts);
+  char* scratch = base + kJobBytes - 256;
+  job.dparams = reinterpret_cast<float4*>(scratch + off_dp);
+  job.result = reinterpret_cast<double*>(scratch + off_res);
+  job.partials = reinterpret_cast<double*>(scratch + off_parts);
   job.state = nullptr;
   // Every scratch word the kernels read is written earlier in this call (the job, the parameters,
   // each tile's partials, the result), so nothing needs clearing between calls. Host staging uses a

@@ -151,7 +151,7 @@ struct BatchCache {
   fa::Job* jobs_dev = nullptr;
   int* d_active = nullptr;  // [0], [1] active frames of the two lists, [2] rounds of the loop, [3] finished CTAs
   int* d_list = nullptr;    // two lists of cap entries: a step reads one and builds the other
-  int* d_prefix = nullptr;
+  int* d_prefix = nullptr;  // cap + 1 entries, then cap entries for the steps' items
   // host-mapped memory the solve steps write: the rounds of the last solve, then one report per frame
   char* h_out = nullptr;
   char* d_out = nullptr;    // its device address

@@ -225,8 +225,8 @@ fa_status class_create_impl(fa_server* S, SrvClass* C) {
   fa_context* ctx = S->ctx;
   const int cap = C->cap;
   FA_TRY(dalloc_t(ctx, (size_t)cap, &C->jobs_dev, C->allocs));
-  FA_TRY(dalloc_t(ctx, 2 * (size_t)cap, &C->list, C->allocs));
-  FA_TRY(dalloc_t(ctx, (size_t)cap + 1, &C->prefix, C->allocs));
+  FA_TRY(dalloc_t(ctx, 2 * (size_t)cap + fa::kListSlack, &C->list, C->allocs));
+  FA_TRY(dalloc_t(ctx, (size_t)cap + 1 + fa::kListSlack, &C->prefix, C->allocs));
   FA_TRY(dalloc_t(ctx, (size_t)cap, &C->busy, C->allocs));
   FA_TRY(dalloc_t(ctx, (size_t)cap + 2, &C->counts, C->allocs));
   FA_TRY(dalloc_t(ctx, 2, &C->next, C->allocs));

@@ -654,14 +654,15 @@ __device__ __forceinline__ void state_step(FrameState& S, const Band<ND>& B, dou
   __syncthreads();
 }
 
-static_assert(sizeof(Job) % 8 == 0 && sizeof(FrameState) % 8 == 0 && sizeof(RefDev) % 8 == 0, "copied by words");
+static_assert(sizeof(Job) % 8 == 0 && sizeof(FrameState) % 8 == 0, "copied by words");
 template <typename T>
 __device__ __forceinline__ void copy_words(T* dst, const T* src) {
   for (int i = threadIdx.x; i < (int)(sizeof(T) / 8); i += blockDim.x)
     reinterpret_cast<unsigned long long*>(dst)[i] = __ldcg(reinterpret_cast<const unsigned long long*>(src) + i);
 }
 
-// One trust-region step of one frame per CTA. The step is latency: a few rounds of dependent loads
+// One trust-region step of one frame per CTA; returns the frame's items in the next fused pass (0: done or
+// waiting). The step is latency: a few rounds of dependent loads
 // (job, then reference and state, then everything they point at, brought into shared memory when it
 // fits), the tile reduction, and the chain of two substitutions; a pass over the frame takes
 // longer only for volumes. The chain was the whole step before it ran from registers with its loads
@@ -669,18 +670,17 @@ __device__ __forceinline__ void copy_words(T* dst, const T* src) {
 // 9.2 us for a 512 x 512 plane with nD = 32, 58 -> 21 us for 512 x 512 x 16 with nD = 32, 261 -> 90 us
 // for 1024 x 1024 x 64 with nD = 64).
 template <int ND, bool STAGED>
-__device__ __forceinline__ void solve_step(const Job* job_src, double* s_dyn) {
+__device__ __forceinline__ int solve_step(const Job* job_src, double* s_dyn) {
   __shared__ Job job;
-  __shared__ RefDev R;
   __shared__ FrameState S;
   __shared__ double s_f, s_f2, s_red[3 * (kSolveThreads / 32)];
   __shared__ int s_flag;
   copy_words(&job, job_src);
   __syncthreads();
   copy_words(&S, job.state);
-  copy_words(&R, job.ref);
   __syncthreads();
-  if (S.phase == kPhaseDone || S.phase == kPhaseWaitWarm) return;
+  const RefDev& R = job.R;
+  if (S.phase == kPhaseDone || S.phase == kPhaseWaitWarm) return 0;
   const bool pair = S.phase == kPhaseStartPair;
   const int nD = R.nD, P = R.P, nn = ND * ND;
   const bool cached = R.L0 != nullptr;
@@ -739,11 +739,12 @@ __device__ __forceinline__ void solve_step(const Job* job_src, double* s_dyn) {
       for (int i = threadIdx.x; i < P; i += blockDim.x) S.warm[i] = x[i];
       if (threadIdx.x == 0 && S.warm_seq != nullptr) *S.warm_seq = S.seq;  // read by later launches
     }
-    return;
+    return 0;
   }
-  if (S.phase == kPhaseWaitWarm) return;
+  if (S.phase == kPhaseWaitWarm) return 0;
   // Next trial point D = x + p, as the fused pass's control-point parameters.
   write_trial_dparams(job.dparams, x, p, nD, ND, threadIdx.x, blockDim.x);
+  return R.n_tiles;
 }
 
 // The CTA that finishes last builds the next active list: one launch per iteration fewer than a
@@ -755,24 +756,37 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const Job* __re
                                                                  unsigned* finished, int end_of_round) {
   extern __shared__ double s_dyn[];
   __shared__ bool s_last;
-  int na = 1;
+  int na = 1, mine = blockIdx.x;
   if (active != nullptr) {
     na = *n_active;
+    mine = active[blockIdx.x];  // within the list's room, whatever its length
     // with no frame active one CTA still ends the round
     if ((int)blockIdx.x >= (finished != nullptr ? max(na, 1) : na)) return;
   }
-  if (na > 0) solve_step<ND, STAGED>(jobs + (active != nullptr ? active[blockIdx.x] : blockIdx.x), s_dyn);
+  const int items = na > 0 ? solve_step<ND, STAGED>(jobs + mine, s_dyn) : 0;
   if (finished == nullptr) return;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();  // the step's writes before the count
-    s_last = atomicAdd(finished, 1u) == (unsigned)max(na, 1) - 1u;
-    if (s_last) *finished = 0u;
-    __threadfence();
+  if (na > 1 || next.busy != nullptr) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (next.items != nullptr) next.items[blockIdx.x] = items;
+      __threadfence();  // the step's writes before the count
+      s_last = atomicAdd(finished, 1u) == (unsigned)max(na, 1) - 1u;
+      if (s_last) *finished = 0u;
+      __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    if (next.busy != nullptr)
+      compact_block(jobs, next);
+    else  // frames only leave a list without busy flags
+      list_block(
+          na, next, [&](int i) { return ListEntry{active[i], __ldcg(next.items + i), false}; }, [] {});
+  } else if (threadIdx.x == 0) {  // the list of one frame, or none
+    *next.n_active = items > 0 ? 1 : 0;
+    next.active[0] = mine;
+    next.prefix[0] = 0;
+    next.prefix[1] = items;
   }
-  __syncthreads();
-  if (!s_last) return;
-  compact_block(jobs, next);
   if (end_of_round && threadIdx.x == 0) {
     const int r = *next.rounds + 1;
     *next.rounds = r;
