@@ -1051,7 +1051,8 @@ extern "C" fa_status fa_align_frame(fa_frame* F, const double* rigid_shift, int 
   for (int step = 0; step < max_steps && phase != fa::kPhaseDone; step++) {
     FA_CU(fa::launch_eval(F->job_dev, 1, R->G.n_tiles, R->n_dim, F->kind, R->prec == FA_PREC_MIXED, F->stream,
                           R->nx % 4 == 0, R->host.tune_mb_small));
-    FA_CU(fa::launch_solve(F->job_dev, 1, R->nD, R->n_dim, F->stream));
+    FA_CU(fa::launch_solve(F->job_dev, 1, R->nD, R->n_dim, F->stream, nullptr, nullptr, nullptr, nullptr, false,
+                           R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles)));
     g_launches += 2;
     FA_CU(cudaMemcpyAsync(&F->h_state->phase, &F->state->phase, sizeof(int), cudaMemcpyDeviceToHost, F->stream));
     FA_CU(cudaStreamSynchronize(F->stream));
@@ -1208,6 +1209,7 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     }
     if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
+      const bool early = vec4 && fa::eval4_few_only(most_items);
       for (int it = 0; it < kGraphIters && e == cudaSuccess; it++) {
         const fa::ActiveOut in = list_out(it & 1);
         fa::ActiveOut out = list_out(1 - (it & 1));
@@ -1220,7 +1222,7 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
                               false);
         if (e == cudaSuccess)
           e = fa::launch_solve(bc->jobs_dev, n, max_nD, R0->n_dim, s, in.active, in.n_active, &out,
-                               reinterpret_cast<unsigned*>(bc->d_active + 3), it == kGraphIters - 1);
+                               reinterpret_cast<unsigned*>(bc->d_active + 3), it == kGraphIters - 1, early);
       }
       cudaGraph_t captured = nullptr;
       const cudaError_t e2 = cudaStreamEndCapture(s, &captured);

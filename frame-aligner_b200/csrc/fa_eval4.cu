@@ -897,6 +897,8 @@ template <int NDIM, typename FT, typename RT>
 __global__ void __launch_bounds__(kEvalThreads, 2) eval4_cta_kernel(const Job* __restrict__ jobs) {
   extern __shared__ float4 s_cta[];
   auto& sm = *reinterpret_cast<CtaTileSmem<NDIM, RT>*>(s_cta);
+  cudaGridDependencySynchronize();            // the step before this pass
+  cudaTriggerProgrammaticLaunchCompletion();  // the one after it may come in and wait for this pass's end
   const Job& job = jobs[blockIdx.y];
   if (job.state != nullptr && (job.state->phase == kPhaseDone || job.state->phase == kPhaseWaitWarm)) return;
   const RefDev& R = job.R;
@@ -961,6 +963,8 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval4_active_cta_kernel(const
                                                                         const int* __restrict__ tile_prefix, int few) {
   extern __shared__ float4 s_cta[];
   auto& sm = *reinterpret_cast<CtaTileSmem<NDIM, RT>*>(s_cta);
+  cudaGridDependencySynchronize();            // the step before this pass
+  cudaTriggerProgrammaticLaunchCompletion();  // the one after it may come in and wait for this pass's end
   // (the lists have room for kListSlack entries more than jobs, so these loads need not wait for na)
   const int lane = threadIdx.x & 31;
   const int na = *n_active, prefix_l = tile_prefix[lane], active_l = active[lane];
@@ -991,6 +995,8 @@ inline cudaError_t dispatch_mb(int mb, Fn&& f) {
   return f(std::integral_constant<int, 2>{});
 }
 
+bool eval4_few_only(long long most_items) { return most_items <= kCtaTiles; }
+
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
   return bytes <= 48 * 1024 ? cudaSuccess
@@ -1006,8 +1012,7 @@ cudaError_t launch_eval4(const Job* jobs_dev, int n_jobs, int max_tiles, int n_d
       auto kernel = eval4_cta_kernel<C::nd, typename C::F, typename C::R>;
       const cudaError_t e = allow_smem(kernel, smem);
       if (e != cudaSuccess) return e;
-      kernel<<<dim3(max_tiles, n_jobs), kEvalThreads, smem, s>>>(jobs_dev);
-      return cudaGetLastError();
+      return launch_early(kernel, dim3(max_tiles, n_jobs), dim3(kEvalThreads), smem, s, true, jobs_dev);
     });
   const dim3 grid((max_tiles + kEvalWarps - 1) / kEvalWarps, n_jobs);
   return dispatch_cfg(n_dim, frame_kind, ref_bf16, [&](auto c) {
@@ -1046,8 +1051,8 @@ cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const in
       auto kernel = eval4_active_cta_kernel<C::nd, typename C::F, typename C::R>;
       cudaError_t e = allow_smem(kernel, smem);
       if (e != cudaSuccess) return e;
-      kernel<<<(int)std::max<long long>(1, ctas), kEvalThreads, smem, s>>>(jobs_dev, active, n_active, tile_prefix, kCtaTiles);
-      e = cudaGetLastError();
+      e = launch_early(kernel, dim3((unsigned)std::max<long long>(1, ctas)), dim3(kEvalThreads), smem, s, !many, jobs_dev,
+                       active, n_active, tile_prefix, (int)kCtaTiles);
       if (e != cudaSuccess || !many) return e;
     }
     const long long most_ctas = (most_items + kEvalWarps - 1) / kEvalWarps;

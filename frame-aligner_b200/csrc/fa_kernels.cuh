@@ -64,6 +64,10 @@ cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const in
                                 long long least_items, long long most_items, int n_dim, int frame_kind, bool ref_bf16,
                                 int mb, int grid, cudaStream_t s);
 
+// Whether every pass of a solve of at most most_items items takes the form for few tiles: then its passes
+// and steps may overlap (the `early` of launch_solve).
+bool eval4_few_only(long long most_items);
+
 // Thread-local (spill) bytes of that kernel's instantiation for a register budget of mb CTAs per SM.
 size_t eval4_active_local_bytes(int n_dim, int frame_kind, bool ref_bf16, int mb);
 
@@ -73,6 +77,25 @@ size_t eval4_active_local_bytes(int n_dim, int frame_kind, bool ref_bf16, int mb
 // done_list[*n_done ...] (busy is cleared). A frame waiting for a warm start that has been written is
 // resumed. In a device-side loop (rounds non-null) the list that ends a round also counts it and repeats
 // the loop while a frame is active and fewer than max_rounds rounds ran.
+// Launches whose kernels may start while their predecessor on the stream still runs (programmatic
+// dependent launch): the kernel itself waits (cudaGridDependencySynchronize) before it touches what the
+// predecessor writes. Used where an iteration is short; a kernel that waits early holds its SMs.
+template <typename... P, typename... A>
+inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool early,
+                                A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 constexpr int kListSlack = 32;  // entries that active and prefix have room for beyond n_jobs (+ 1)
 struct ActiveOut {
   int n_jobs;
@@ -107,10 +130,10 @@ cudaError_t launch_warp(const RefDev* ref_dev, const RefDev& ref_host, const voi
 // above about 200 KB work in global memory). With `next`, the last CTA to finish builds the next active
 // list there (its list and length must not be `active` and `n_active`, which the launch's other CTAs may
 // still read; `finished` counts them and is zero between launches), and with end_of_round it also
-// controls the loop.
+// controls the loop. early: the launch directly after a few-tile pass may start before the pass ends.
 cudaError_t launch_solve(const Job* jobs_dev, int n_jobs, int max_nD, int n_dim, cudaStream_t s,
                          const int* active = nullptr, const int* n_active = nullptr, const ActiveOut* next = nullptr,
-                         unsigned* finished = nullptr, bool end_of_round = false);
+                         unsigned* finished = nullptr, bool end_of_round = false, bool early = false);
 
 // Test hook: the device trust-region subproblem on given dense H (P x P) and g.
 // The band Cholesky factor of H (lambda = 0) into L0 (nD * nd rows of 2 * nd) and inv0 (nD * nd); *ok

@@ -123,6 +123,7 @@ struct SrvClass {
   fa::Activation* d_act = nullptr;
   fa::Activation* h_act = nullptr;    // pinned
   fa::FrameState* dummy = nullptr;    // phase Done, for unused entries
+  int bound = 1;                      // table entries the graph covers (all in use lie below)
   std::vector<SrvSlot*> owner;
   std::vector<int> free_idx;
   std::vector<SrvAcq*> acqs;
@@ -298,10 +299,12 @@ fa_status class_capture(fa_server* S, SrvClass* C) {
   C->exec = nullptr;
   C->graph = nullptr;
   cudaStream_t s = C->stream;
+  const long long most_items = 2LL * C->bound * C->max_tiles;
+  const bool early = C->vec4 && fa::eval4_few_only(most_items);
   // the steps alternate between two lists; the list before the first step is list 0
   auto list_out = [&](int which) {
     fa::ActiveOut o{};
-    o.n_jobs = C->cap;
+    o.n_jobs = C->bound;
     o.active = C->list + (size_t)which * C->cap;
     o.n_active = which ? C->next : C->counts;
     o.prefix = C->prefix;
@@ -318,13 +321,13 @@ fa_status class_capture(fa_server* S, SrvClass* C) {
       const fa::ActiveOut in = list_out(it & 1), out = list_out(1 - (it & 1));
       if (C->vec4)
         e = fa::launch_eval4_active(C->jobs_dev, in.active, in.n_active, in.prefix, C->min_tiles,
-                                    2LL * C->cap * C->max_tiles, C->n_dim, C->kind, C->bf16, C->mb,
+                                    most_items, C->n_dim, C->kind, C->bf16, C->mb,
                                     C->grid_mult * S->sms, s);
       else
-        e = fa::launch_eval(C->jobs_dev, C->cap, C->max_tiles, C->n_dim, C->kind, C->bf16, s, false);
+        e = fa::launch_eval(C->jobs_dev, C->bound, C->max_tiles, C->n_dim, C->kind, C->bf16, s, false);
       if (e == cudaSuccess)
-        e = fa::launch_solve(C->jobs_dev, C->cap, C->max_nD, C->n_dim, s, in.active, in.n_active, &out,
-                             reinterpret_cast<unsigned*>(C->next + 1), false);
+        e = fa::launch_solve(C->jobs_dev, C->bound, C->max_nD, C->n_dim, s, in.active, in.n_active, &out,
+                             reinterpret_cast<unsigned*>(C->next + 1), false, early);
     }
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(C->h_counts, C->counts, (size_t)(C->cap + 2) * sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -406,6 +409,10 @@ fa_status slot_create(fa_server* S, SrvAcq* q, SrvSlot** out) {
   sl->index = C->free_idx.back();
   C->free_idx.pop_back();
   C->owner[sl->index] = sl;
+  if (sl->index >= C->bound) {  // the next launch's graph covers the entry (entries fill from 0)
+    while (C->bound <= sl->index) C->bound = std::min(2 * C->bound, C->cap);
+    C->dirty = true;
+  }
   // The entry is visible to every launch of the class from now on: its state starts as done, so the
   // frame stays out of the active list until it is activated.
   FA_CU(cudaMemcpyAsync(sl->F->state, C->dummy, sizeof(fa::FrameState), cudaMemcpyDeviceToDevice, C->stream));

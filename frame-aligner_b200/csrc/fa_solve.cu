@@ -715,6 +715,8 @@ __device__ __forceinline__ int solve_step(const Job* job_src, double* s_dyn) {
     }
     if (pair) __syncthreads();  // p is loaded before the rigid point's gradient replaces it
   }
+  cudaGridDependencySynchronize();  // the fused pass's partial sums (everything above is older)
+  cudaTriggerProgrammaticLaunchCompletion();  // the next pass may come in and wait for this launch's end
   reduce_partials(R, job.partials, &s_f, gt);
   // paired start: the rigid point's sums, its gradient into p (free until the first step)
   if (pair) reduce_partials(R, job.partials2, &s_f2, p);
@@ -756,6 +758,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const Job* __re
                                                                  unsigned* finished, int end_of_round) {
   extern __shared__ double s_dyn[];
   __shared__ bool s_last;
+  // Started early, everything read before the step's wait is older than the pass: the pass waited for the
+  // launch before it, and lets this one start only then.
   int na = 1, mine = blockIdx.x;
   if (active != nullptr) {
     na = *n_active;
@@ -764,6 +768,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const Job* __re
     if ((int)blockIdx.x >= (finished != nullptr ? max(na, 1) : na)) return;
   }
   const int items = na > 0 ? solve_step<ND, STAGED>(jobs + mine, s_dyn) : 0;
+  cudaGridDependencySynchronize();  // (a CTA without a step: the launch never ends before the pass)
   if (finished == nullptr) return;
   if (na > 1 || next.busy != nullptr) {
     __syncthreads();
@@ -800,29 +805,29 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const Job* __re
 namespace {
 template <int ND>
 cudaError_t launch_solve_nd(const Job* jobs_dev, int n_jobs, int max_nD, cudaStream_t s, const int* active,
-                            const int* n_active, const ActiveOut& next, unsigned* finished, int end_of_round) {
+                            const int* n_active, const ActiveOut& next, unsigned* finished, int end_of_round,
+                            bool early) {
   constexpr long long kCapBytes = 200 * 1024;
   const long long need = solve_smem_doubles(max_nD, ND) * (long long)sizeof(double);
-  if (need > kCapBytes) {  // every frame of the launch works in global memory
-    solve_kernel<ND, false><<<n_jobs, kSolveThreads, 0, s>>>(jobs_dev, active, n_active, next, finished, end_of_round);
-    return cudaGetLastError();
-  }
+  if (need > kCapBytes)  // every frame of the launch works in global memory
+    return launch_early(solve_kernel<ND, false>, dim3(n_jobs), dim3(kSolveThreads), 0, s, early, jobs_dev, active,
+                        n_active, next, finished, end_of_round);
   if (need > 40 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(solve_kernel<ND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
     if (e != cudaSuccess) return e;
   }
-  solve_kernel<ND, true><<<n_jobs, kSolveThreads, (size_t)need, s>>>(jobs_dev, active, n_active, next, finished,
-                                                                     end_of_round);
-  return cudaGetLastError();
+  return launch_early(solve_kernel<ND, true>, dim3(n_jobs), dim3(kSolveThreads), (size_t)need, s, early, jobs_dev,
+                      active, n_active, next, finished, end_of_round);
 }
 }  // namespace
 
 cudaError_t launch_solve(const Job* jobs_dev, int n_jobs, int max_nD, int n_dim, cudaStream_t s, const int* active,
-                         const int* n_active, const ActiveOut* next, unsigned* finished, bool end_of_round) {
+                         const int* n_active, const ActiveOut* next, unsigned* finished, bool end_of_round, bool early) {
   const ActiveOut out = next ? *next : ActiveOut{};
   unsigned* count = next ? finished : nullptr;
-  return n_dim == 3 ? launch_solve_nd<3>(jobs_dev, n_jobs, max_nD, s, active, n_active, out, count, end_of_round)
-                    : launch_solve_nd<2>(jobs_dev, n_jobs, max_nD, s, active, n_active, out, count, end_of_round);
+  const int end = end_of_round ? 1 : 0;
+  return n_dim == 3 ? launch_solve_nd<3>(jobs_dev, n_jobs, max_nD, s, active, n_active, out, count, end, early)
+                    : launch_solve_nd<2>(jobs_dev, n_jobs, max_nD, s, active, n_active, out, count, end, early);
 }
 
 // The factor of H itself, once per reference: one block brings the blocks of H into shared memory (when
