@@ -759,10 +759,7 @@ fa_status frame_alloc(fa_reference* R, int kind, fa_frame** out) {
   auto cleanup = [&](fa_status st) {
     std::string keep = g_err;
     if (F->stream) cudaStreamDestroy(F->stream);
-    if (F->h_result) cudaFreeHost(F->h_result);
-    if (F->h_dparams) cudaFreeHost(F->h_dparams);
-    if (F->h_x) cudaFreeHost(F->h_x);
-    if (F->h_state) cudaFreeHost(F->h_state);
+    if (F->h_pin) cudaFreeHost(F->h_pin);
     dfree_all(ctx, F->allocs);
     delete F;
     g_err = keep;
@@ -797,23 +794,35 @@ fa_status frame_alloc(fa_reference* R, int kind, fa_frame** out) {
   j.partials2 = j.partials + (size_t)R->G.n_tiles * fa::kPartialDoubles;
   if ((st = dalloc_t(ctx, 1, &F->state, F->allocs)) != FA_OK) return cleanup(st);
   double* pool;
-  size_t nd = 4 * P + work_doubles(R) + 1 + P;
+  size_t nd = 4 * P + work_doubles(R);
   if ((st = dalloc_t(ctx, nd, &pool, F->allocs)) != FA_OK) return cleanup(st);
   j.x = pool;
   j.g = pool + P;
   j.p = pool + 2 * P;
   j.gt = pool + 3 * P;
   j.work = pool + 4 * P;
-  j.result = j.work + work_doubles(R);
   j.state = nullptr;
-  if ((st = dalloc_t(ctx, 1, &F->job_dev, F->allocs)) != FA_OK) return cleanup(st);
-  if (cudaMallocHost(&F->h_result, (1 + P) * sizeof(double)) != cudaSuccess ||
-      cudaMallocHost(&F->h_dparams, (size_t)R->nD * fa::kDParamF4 * sizeof(float4)) != cudaSuccess ||
-      cudaMallocHost(&F->h_x, P * sizeof(double)) != cudaSuccess ||
-      cudaMallocHost(&F->h_state, sizeof(fa::FrameState)) != cudaSuccess)
-    return cleanup(fail(FA_ERR_OOM, "cudaMallocHost failed"));
-  if (cudaMemcpyAsync(F->job_dev, &F->job, sizeof(Job), cudaMemcpyHostToDevice, F->stream) != cudaSuccess)
-    return cleanup(fail(FA_ERR_CUDA, "job upload failed"));
+  if ((st = dalloc_t(ctx, 2, &F->job_dev, F->allocs)) != FA_OK) return cleanup(st);
+  {
+    const size_t o_dp = ((1 + P) * sizeof(double) + 63) / 64 * 64,
+                 o_state = o_dp + ((size_t)R->nD * fa::kDParamF4 * sizeof(float4) + 63) / 64 * 64;
+    void *hp = nullptr, *dp = nullptr;
+    if (cudaMallocHost(&hp, o_state + fa::kReportHeaderBytes + P * sizeof(double)) != cudaSuccess)
+      return cleanup(fail(FA_ERR_OOM, "cudaMallocHost failed"));
+    F->h_pin = static_cast<char*>(hp);
+    F->h_result = reinterpret_cast<double*>(F->h_pin);
+    F->h_dparams = reinterpret_cast<float4*>(F->h_pin + o_dp);
+    F->h_state = reinterpret_cast<fa::FrameState*>(F->h_pin + o_state);
+    F->h_x = reinterpret_cast<double*>(F->h_pin + o_state + fa::kReportHeaderBytes);
+    if (cudaHostGetDevicePointer(&dp, hp, 0) != cudaSuccess)
+      return cleanup(fail(FA_ERR_CUDA, "cudaHostGetDevicePointer failed"));
+    j.result = static_cast<double*>(dp);
+    Job js[2] = {j, j};
+    js[1].state = F->state;
+    js[1].report = static_cast<char*>(dp) + o_state;
+    if (cudaMemcpyAsync(F->job_dev, js, sizeof(js), cudaMemcpyHostToDevice, F->stream) != cudaSuccess)
+      return cleanup(fail(FA_ERR_CUDA, "job upload failed"));
+  }
   R->n_frames++;
   *out = F;
   return FA_OK;
@@ -891,10 +900,7 @@ extern "C" fa_status fa_deregister_frame(fa_frame* F) {
     cudaStreamSynchronize(F->stream);
     cudaStreamDestroy(F->stream);
   }
-  if (F->h_result) cudaFreeHost(F->h_result);
-  if (F->h_dparams) cudaFreeHost(F->h_dparams);
-  if (F->h_x) cudaFreeHost(F->h_x);
-  if (F->h_state) cudaFreeHost(F->h_state);
+  if (F->h_pin) cudaFreeHost(F->h_pin);
   F->ref->n_frames--;
   dfree_all(F->ref->ctx, F->allocs);
   delete F;
@@ -914,9 +920,8 @@ fa_status evaluate(fa_frame* F, const double* D) {
   FA_CU(cudaMemcpyAsync(F->job.dparams, F->h_dparams, np, cudaMemcpyHostToDevice, F->stream));
   FA_CU(fa::launch_eval(F->job_dev, 1, R->G.n_tiles, R->n_dim, F->kind, R->prec == FA_PREC_MIXED, F->stream,
                           R->nx % 4 == 0, R->host.tune_mb_small));
-  FA_CU(fa::launch_reduce(F->job_dev, R->host, F->stream));
+  FA_CU(fa::launch_reduce(F->job_dev, F->stream, R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles)));
   g_launches += 2;
-  FA_CU(cudaMemcpyAsync(F->h_result, F->job.result, (1 + R->P) * sizeof(double), cudaMemcpyDeviceToHost, F->stream));
   FA_CU(cudaStreamSynchronize(F->stream));
   F->last_f = F->h_result[0];
   F->last_g.assign(F->h_result + 1, F->h_result + 1 + R->P);
@@ -1042,27 +1047,27 @@ extern "C" fa_status fa_align_frame(fa_frame* F, const double* rigid_shift, int 
   std::lock_guard<std::mutex> lk(F->mu);
   fa_reference* R = F->ref;
   FA_CU(cudaSetDevice(R->ctx->device));
-  FA_TRY(init_solve(F, rigid_shift, max_iterations, false));
-  Job j = F->job;
-  j.state = F->state;
-  FA_CU(cudaMemcpyAsync(F->job_dev, &j, sizeof(Job), cudaMemcpyHostToDevice, F->stream));
-  const int max_steps = (max_iterations > 0 ? max_iterations : 100) + 4;
-  int phase = fa::kPhaseStartZero;
-  for (int step = 0; step < max_steps && phase != fa::kPhaseDone; step++) {
-    FA_CU(fa::launch_eval(F->job_dev, 1, R->G.n_tiles, R->n_dim, F->kind, R->prec == FA_PREC_MIXED, F->stream,
-                          R->nx % 4 == 0, R->host.tune_mb_small));
-    FA_CU(fa::launch_solve(F->job_dev, 1, R->nD, R->n_dim, F->stream, nullptr, nullptr, nullptr, nullptr, false,
-                           R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles)));
-    g_launches += 2;
-    FA_CU(cudaMemcpyAsync(&F->h_state->phase, &F->state->phase, sizeof(int), cudaMemcpyDeviceToHost, F->stream));
-    FA_CU(cudaStreamSynchronize(F->stream));
-    phase = F->h_state->phase;
-  }
+  // The host drives the iterations in bursts: a step that finds the frame done leaves at once (about 4 us),
+  // a round trip to the host costs three times that.
+  const int max_iter = max_iterations > 0 ? max_iterations : 100;
+  constexpr int kBurst = 4;
+  const bool early = R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles);
+  const fa::Job* job = F->job_dev + 1;
   F->have_last = false;
-  FA_TRY(finish_solve(F, D_out, stats));
-  Job j0 = F->job;
-  FA_CU(cudaMemcpyAsync(F->job_dev, &j0, sizeof(Job), cudaMemcpyHostToDevice, F->stream));
-  FA_CU(cudaStreamSynchronize(F->stream));
+  F->h_state->phase = fa::kPhaseStartZero;  // until the step that finishes the solve reports
+  FA_CU(fa::launch_start(job, rigid_shift, max_iter, F->stream));
+  g_launches += 1;
+  for (int step = 0; step < max_iter + 4 && F->h_state->phase != fa::kPhaseDone; step += kBurst) {
+    for (int i = 0; i < kBurst; i++) {
+      FA_CU(fa::launch_eval(job, 1, R->G.n_tiles, R->n_dim, F->kind, R->prec == FA_PREC_MIXED, F->stream, R->nx % 4 == 0,
+                            R->host.tune_mb_small));
+      FA_CU(fa::launch_solve(job, 1, R->nD, R->n_dim, F->stream, nullptr, nullptr, nullptr, nullptr, false, early));
+      g_launches += 2;
+    }
+    FA_CU(cudaStreamSynchronize(F->stream));
+  }
+  if (F->h_state->phase != fa::kPhaseDone) return finish_solve(F, D_out, stats);  // where the solve stands
+  finish_solve_read(F, F->h_x, *F->h_state, D_out, stats);
   return FA_OK;
 }
 
@@ -1114,10 +1119,10 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     FA_TRY(dalloc_t(ctx, 2 * (size_t)n + fa::kListSlack, &bc->d_list, bc->allocs));
     FA_TRY(dalloc_t(ctx, 2 * (size_t)n + 1 + fa::kListSlack, &bc->d_prefix, bc->allocs));
     void* hp = nullptr;
-    if (cudaHostAlloc(&hp, out_bytes, cudaHostAllocMapped) != cudaSuccess) {
+    if (cudaMallocHost(&hp, out_bytes) != cudaSuccess) {  // (pinned memory is mapped)
       cudaGetLastError();
       batch_cache_release(ctx, bc);
-      return fail(FA_ERR_OOM, "cudaHostAlloc failed");
+      return fail(FA_ERR_OOM, "cudaMallocHost failed");
     }
     bc->h_out = static_cast<char*>(hp);
     bc->out_bytes = out_bytes;

@@ -559,13 +559,13 @@ cudaError_t launch_eval(const Job* jobs_dev, int n_jobs, int max_tiles, int n_di
 __global__ void __launch_bounds__(kSolveThreads) reduce_kernel(const Job* __restrict__ job) {
   const RefDev& R = job->R;
   __shared__ double s_f;
+  cudaGridDependencySynchronize();  // the pass's partial sums
   reduce_partials(R, job->partials, &s_f, job->result + 1);
   if (threadIdx.x == 0) job->result[0] = s_f;
 }
 
-cudaError_t launch_reduce(const Job* job_dev, const RefDev&, cudaStream_t s) {
-  reduce_kernel<<<1, kSolveThreads, 0, s>>>(job_dev);
-  return cudaGetLastError();
+cudaError_t launch_reduce(const Job* job_dev, cudaStream_t s, bool early) {
+  return launch_early(reduce_kernel, dim3(1), dim3(kSolveThreads), 0, s, early, job_dev);
 }
 
 // ------------------------------------------------------------------ warped image -----------------
@@ -863,6 +863,36 @@ cudaError_t launch_activate_peaks(const Job* jobs_dev, int n, const long long* p
                                   int binning, int max_iter, bool pair, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   activate_peaks_kernel<<<n, 128, 0, s>>>(jobs_dev, peaks, cnx, cny, cnz, binning, max_iter, pair ? 1 : 0);
+  return cudaGetLastError();
+}
+
+// The zero start of one frame's own solve (kPhaseStartZero, then the rigid shift if it is not zero).
+struct RigidShift {
+  double v[3];
+};
+__global__ void start_kernel(const Job* __restrict__ job, RigidShift rigid, int max_iter) {
+  const Job& j = *job;
+  const RefDev& R = j.R;
+  for (int i = threadIdx.x; i < R.P; i += blockDim.x) {
+    j.x[i] = 0.0;
+    j.g[i] = 0.0;
+    j.p[i] = 0.0;
+    j.gt[i] = 0.0;
+  }
+  for (int i = threadIdx.x; i < R.nD * kDParamF4; i += blockDim.x) j.dparams[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (threadIdx.x == 0) {
+    FrameState S{};
+    S.phase = kPhaseStartZero;
+    S.max_iter = max_iter;
+    for (int c = 0; c < 3; c++) S.rigid[c] = c < R.n_dim ? rigid.v[c] : 0.0;
+    *j.state = S;
+  }
+}
+
+cudaError_t launch_start(const Job* job_dev, const double* rigid, int max_iter, cudaStream_t s) {
+  RigidShift r{{0.0, 0.0, 0.0}};
+  for (int c = 0; c < 3 && rigid; c++) r.v[c] = rigid[c];
+  start_kernel<<<1, 128, 0, s>>>(job_dev, r, max_iter);
   return cudaGetLastError();
 }
 

@@ -116,8 +116,11 @@ cudaError_t launch_activate_peaks(const Job* jobs_dev, int n, const long long* p
 // Initialises the solve state of n frames (zero start, optional rigid and warm starts) and marks them busy.
 cudaError_t launch_activate(const Job* jobs_dev, const Activation* recs, int n, int* busy, cudaStream_t s);
 
-// Reduces one job's tile partials into result = [f, g(P)] (deterministic order).
-cudaError_t launch_reduce(const Job* job_dev, const RefDev& ref_host, cudaStream_t s);
+// Reduces one job's tile partials into result = [f, g(P)] (deterministic order). early: directly after a
+// few-tile pass, may start before the pass ends.
+cudaError_t launch_reduce(const Job* job_dev, cudaStream_t s, bool early = false);
+// Zero start of one frame's own solve (rigid: 3 doubles or null).
+cudaError_t launch_start(const Job* job_dev, const double* rigid, int max_iter, cudaStream_t s);
 
 // Warped image (CpuFrameWarper::warpImageInterpolated semantics) for one frame.
 cudaError_t launch_warp(const RefDev* ref_dev, const RefDev& ref_host, const void* frame, long long fplane, int fpitch,

@@ -89,12 +89,15 @@ struct fa_frame {
   int kind = fa::kFrameF32;
   cudaStream_t stream = nullptr;
   fa::Job job{};
-  fa::Job* job_dev = nullptr;
+  fa::Job* job_dev = nullptr;   // [0]: bare evaluations; [1]: the single-frame solve (with state and report)
   fa::FrameState* state = nullptr;
-  double* h_result = nullptr;  // pinned: [f, g(P)]
-  float4* h_dparams = nullptr;  // pinned: nD * 3
-  double* h_x = nullptr;        // pinned: P
-  fa::FrameState* h_state = nullptr;  // pinned
+  // One pinned, host-mapped block: the result [f, g(P)] of a bare evaluation (written by the reduction),
+  // the control-point parameters on their way up, and the report of a finished solve (state, then x).
+  char* h_pin = nullptr;
+  double* h_result = nullptr;
+  float4* h_dparams = nullptr;  // nD * 3
+  fa::FrameState* h_state = nullptr;
+  double* h_x = nullptr;        // P, kReportHeaderBytes after h_state
   float* warp_out = nullptr;
   std::vector<double> lastD;
   std::vector<double> last_g;
