@@ -920,7 +920,7 @@ fa_status evaluate(fa_frame* F, const double* D) {
   FA_CU(cudaMemcpyAsync(F->job.dparams, F->h_dparams, np, cudaMemcpyHostToDevice, F->stream));
   FA_CU(fa::launch_eval(F->job_dev, 1, R->G.n_tiles, R->n_dim, F->kind, R->prec == FA_PREC_MIXED, F->stream,
                           R->nx % 4 == 0, R->host.tune_mb_small));
-  FA_CU(fa::launch_reduce(F->job_dev, F->stream, R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles)));
+  FA_CU(fa::launch_reduce(F->job_dev, R->G.n_tiles, R->nD, F->stream, R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles)));
   g_launches += 2;
   FA_CU(cudaStreamSynchronize(F->stream));
   F->last_f = F->h_result[0];
@@ -1051,7 +1051,7 @@ extern "C" fa_status fa_align_frame(fa_frame* F, const double* rigid_shift, int 
   // a round trip to the host costs three times that.
   const int max_iter = max_iterations > 0 ? max_iterations : 100;
   constexpr int kBurst = 4;
-  const bool early = R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles);
+  const bool overlap = R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles);
   const fa::Job* job = F->job_dev + 1;
   F->have_last = false;
   F->h_state->phase = fa::kPhaseStartZero;  // until the step that finishes the solve reports
@@ -1061,7 +1061,8 @@ extern "C" fa_status fa_align_frame(fa_frame* F, const double* rigid_shift, int 
     for (int i = 0; i < kBurst; i++) {
       FA_CU(fa::launch_eval(job, 1, R->G.n_tiles, R->n_dim, F->kind, R->prec == FA_PREC_MIXED, F->stream, R->nx % 4 == 0,
                             R->host.tune_mb_small));
-      FA_CU(fa::launch_solve(job, 1, R->nD, R->n_dim, F->stream, nullptr, nullptr, nullptr, nullptr, false, early));
+      if (fa::wide_reduction(R->G.n_tiles)) FA_CU(fa::launch_wide_reduce(job, 1, R->nD, F->stream));
+      FA_CU(fa::launch_solve(job, 1, R->nD, R->n_dim, F->stream, nullptr, nullptr, nullptr, nullptr, false, overlap));
       g_launches += 2;
     }
     FA_CU(cudaStreamSynchronize(F->stream));
@@ -1087,14 +1088,15 @@ struct PeakStart {
 // caller's align_batch_finish waits for it. frame_data (optional) replaces each frame's own device
 // data pointer for this call. bc keeps the buffers and the graph for the next call on the same
 // frames. With `peak_start` the rigid starts come from device peaks (rigid_shifts is ignored) and the
-// states are set up on the device, so the host neither waits for the peaks nor copies a state.
+// states are set up on the device, so the host neither waits for the peaks nor copies a state. alone: no
+// other solve of the caller competes with it.
 //
 // The graph holds one while-conditional node whose body is kGraphIters x (fused pass, solve step): the
 // last CTA of a step builds the next active list, the last step also controls the loop, and the body
 // repeats on the device until no frame is active or the iteration limit is reached, with no host round
 // trip between rounds.
 fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigid_shifts, int max_iterations,
-                              const void* const* frame_data, BatchCache* bc, const PeakStart* peak_start) {
+                              const void* const* frame_data, BatchCache* bc, const PeakStart* peak_start, bool alone) {
   if (!frames || n <= 0 || !bc) return fail(FA_ERR_BAD_ARG, "bad arguments");
   for (int i = 0; i < n; i++)
     if (!frames[i]) return fail(FA_ERR_BAD_ARG, "NULL frame");
@@ -1191,7 +1193,8 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   // the register budget tuned for launches of many frames, or of a few
   const int mb = n >= kManyFrames ? R0->host.tune_mb : R0->host.tune_mb_small;
-  const long long key[7] = {n, most_items, max_nD, (vec4 ? 1 : 0) + 2 * frames[0]->kind, mb, least_items, max_rounds};
+  const long long key[7] = {n, most_items, max_nD, (vec4 ? 1 : 0) + 2 * frames[0]->kind + (alone ? 16 : 0), mb, least_items,
+                            max_rounds};
   const bool reuse = bc->exec && bc->frames.size() == (size_t)n &&
                      std::equal(bc->frames.begin(), bc->frames.end(), frames) && std::equal(key, key + 7, bc->key);
   if (!reuse) {
@@ -1214,20 +1217,22 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
     }
     if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      const bool early = vec4 && fa::eval4_few_only(most_items);
+      const bool overlap = alone && vec4 && fa::eval4_few_only(most_items);
       for (int it = 0; it < kGraphIters && e == cudaSuccess; it++) {
         const fa::ActiveOut in = list_out(it & 1);
         fa::ActiveOut out = list_out(1 - (it & 1));
         out.loop = loop;
         if (vec4)
           e = fa::launch_eval4_active(bc->jobs_dev, in.active, in.n_active, in.prefix, least_items, most_items,
-                                      R0->n_dim, frames[0]->kind, R0->prec == FA_PREC_MIXED, mb, mb * sms, s);
+                                      R0->n_dim, frames[0]->kind, R0->prec == FA_PREC_MIXED, mb, mb * sms, s, overlap);
         else
           e = fa::launch_eval(bc->jobs_dev, n, max_tiles, R0->n_dim, frames[0]->kind, R0->prec == FA_PREC_MIXED, s,
                               false);
+        if (e == cudaSuccess && fa::wide_reduction(max_tiles))
+          e = fa::launch_wide_reduce(bc->jobs_dev, n, max_nD, s, in.active, in.n_active);
         if (e == cudaSuccess)
           e = fa::launch_solve(bc->jobs_dev, n, max_nD, R0->n_dim, s, in.active, in.n_active, &out,
-                               reinterpret_cast<unsigned*>(bc->d_active + 3), it == kGraphIters - 1, early);
+                               reinterpret_cast<unsigned*>(bc->d_active + 3), it == kGraphIters - 1, overlap);
       }
       cudaGraph_t captured = nullptr;
       const cudaError_t e2 = cudaStreamEndCapture(s, &captured);
@@ -1284,7 +1289,7 @@ fa_status align_batch_impl(fa_frame* const* frames, int n, const double* rigid_s
   for (int i = 0; i < n; i++) locks.emplace_back(frames[i]->mu);
   BatchCache local;
   BatchCache* bc = cache ? cache : &local;
-  fa_status r = align_batch_enqueue(frames, n, rigid_shifts, max_iterations, frame_data, bc, nullptr);
+  fa_status r = align_batch_enqueue(frames, n, rigid_shifts, max_iterations, frame_data, bc, nullptr, true);
   if (r == FA_OK) r = align_batch_finish(frames, n, bc, D_out, stats);
   std::string keep = g_err;
   cudaSetDevice(frames[0]->ref->ctx->device);
@@ -1987,13 +1992,15 @@ fa_status aligner_run(fa_aligner* A, const void* const* frames, fa_dtype dtype, 
   // group starts as soon as its peaks are there. The rigid starts are unravelled and scaled by the
   // binning on the device (FrameWarpAligner.cpp:181-190).
   std::vector<fa_frame*> batch(A->slots.begin(), A->slots.begin() + n);
+  // groups whose tiles all fit the device together do not take SMs from one another
+  const bool alone = n_groups == 1 || fa::eval4_few_only((long long)n * A->ref->G.n_tiles);
   fa_status r = FA_OK;
   int queued = 0;
   for (int g = 0; g < n_groups && r == FA_OK; g++) {
     const int g0 = gb[g], g1 = gb[g + 1];
     const PeakStart ps{C->d_idx + g0, C->nx, C->ny, C->nz, A->prm.spatial_binning, A->group_ev[g]};
     r = align_batch_enqueue(batch.data() + g0, g1 - g0, nullptr, A->prm.max_iterations, nullptr, &A->batch_cache[g],
-                            &ps);
+                            &ps, alone);
     // the last group's stream also holds whatever its failed enqueue left queued
     queued = g + 1;
   }

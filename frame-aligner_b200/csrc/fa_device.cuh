@@ -176,6 +176,10 @@ __device__ __forceinline__ void reduce_partials(const RefDev& R, const double* _
   __syncthreads();
 }
 
+// Frames of more tiles than this are reduced by a launch of their own over many CTAs (wide_reduce) before
+// the solve step; see launch_wide_reduce.
+constexpr int kWideTiles = 2048;
+
 // Control-point parameters (kDParamF4 float4 per control point) of the trial point D = x + p; control
 // points k = t0, t0 + stride, ...
 __device__ __forceinline__ void write_trial_dparams(float4* dparams, const double* x, const double* p, int nD, int nd,

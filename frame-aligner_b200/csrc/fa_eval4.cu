@@ -963,7 +963,7 @@ __global__ void __launch_bounds__(kEvalThreads, 2) eval4_active_cta_kernel(const
                                                                         const int* __restrict__ tile_prefix, int few) {
   extern __shared__ float4 s_cta[];
   auto& sm = *reinterpret_cast<CtaTileSmem<NDIM, RT>*>(s_cta);
-  cudaGridDependencySynchronize();            // the step before this pass
+  cudaGridDependencySynchronize();  // the step before this pass
   cudaTriggerProgrammaticLaunchCompletion();  // the one after it may come in and wait for this pass's end
   // (the lists have room for kListSlack entries more than jobs, so these loads need not wait for na)
   const int lane = threadIdx.x & 31;
@@ -1012,7 +1012,7 @@ cudaError_t launch_eval4(const Job* jobs_dev, int n_jobs, int max_tiles, int n_d
       auto kernel = eval4_cta_kernel<C::nd, typename C::F, typename C::R>;
       const cudaError_t e = allow_smem(kernel, smem);
       if (e != cudaSuccess) return e;
-      return launch_early(kernel, dim3(max_tiles, n_jobs), dim3(kEvalThreads), smem, s, true, jobs_dev);
+      return launch_overlapped(kernel, dim3(max_tiles, n_jobs), dim3(kEvalThreads), smem, s, true, jobs_dev);
     });
   const dim3 grid((max_tiles + kEvalWarps - 1) / kEvalWarps, n_jobs);
   return dispatch_cfg(n_dim, frame_kind, ref_bf16, [&](auto c) {
@@ -1041,7 +1041,7 @@ size_t eval4_active_local_bytes(int n_dim, int frame_kind, bool ref_bf16, int mb
 
 cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const int* n_active, const int* tile_prefix,
                                 long long least_items, long long most_items, int n_dim, int frame_kind, bool ref_bf16,
-                                int mb, int grid, cudaStream_t s) {
+                                int mb, int grid, cudaStream_t s, bool overlap) {
   return dispatch_cfg(n_dim, frame_kind, ref_bf16, [&](auto c) {
     using C = decltype(c);
     const bool few = least_items <= kCtaTiles, many = most_items > kCtaTiles;
@@ -1051,8 +1051,8 @@ cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const in
       auto kernel = eval4_active_cta_kernel<C::nd, typename C::F, typename C::R>;
       cudaError_t e = allow_smem(kernel, smem);
       if (e != cudaSuccess) return e;
-      e = launch_early(kernel, dim3((unsigned)std::max<long long>(1, ctas)), dim3(kEvalThreads), smem, s, !many, jobs_dev,
-                       active, n_active, tile_prefix, (int)kCtaTiles);
+      e = launch_overlapped(kernel, dim3((unsigned)std::max<long long>(1, ctas)), dim3(kEvalThreads), smem, s, overlap && !many,
+                            jobs_dev, active, n_active, tile_prefix, (int)kCtaTiles);
       if (e != cudaSuccess || !many) return e;
     }
     const long long most_ctas = (most_items + kEvalWarps - 1) / kEvalWarps;

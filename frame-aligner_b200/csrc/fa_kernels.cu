@@ -422,7 +422,8 @@ cudaError_t launch_downsample(const void* in, fa_dtype in_type, int nz, int ny, 
 
 // ------------------------------------------------------------------ fused evaluation -------------
 
-template <int NDIM, typename FT, typename RT>
+// RUNS: the form for few tiles, where what a lane's voxels cost is the latency of their loads.
+template <int NDIM, typename FT, typename RT, bool RUNS>
 __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const Job* __restrict__ jobs) {
   const Job& job = jobs[blockIdx.y];
   if (job.state != nullptr && (job.state->phase == kPhaseDone || job.state->phase == kPhaseWaitWarm)) return;
@@ -464,42 +465,155 @@ __global__ void __launch_bounds__(kEvalThreads) eval_kernel(const Job* __restric
     for (int k = 0; k < NDIM; k++) ag[s][k] = 0.0f;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int row = row_begin + warp; row < row_end; row += kEvalWarps) {
+  // One voxel of the general form: any interval, range and position.
+  const bool padded = job.fpad != 0;
+  auto general = [&](const RowDesc& rd, bool flip, int x, long long p) {
+    const VoxelModel vm = voxel_model(rd, x, nx, flip, bidir, dq);
+    // the host geometry guarantees c0-1 <= di <= c0+2; the clamp only keeps the shared-memory
+    // window in bounds
+    const int wi = min(max(vm.di - cw, 0), kWin - 2);
+    const float v = sample<NDIM, FT>(fr, job.fplane, job.fpitch, sD + wi * kDParamF4, vm.f, x, rd.y, rd.z, nx, ny, nz);
+    const float t = refgrad(0, p);
+    // include iff the interpolated value is positive: CPU rule px == 0 -> -1, then wimg >= 0
+    // (FrameWarper.cpp:67, 16-25)
+    const float e = (v > 0.0f) ? v - t : 0.0f;
+    af = fmaf(e, e, af);
+    if (!vm.last) {
+      const float e1 = e * vm.f;           // weight of control r+1: Df
+      const float e0 = e * (1.0f - vm.f);  // weight of control r:   1 - Df
+      float gk[NDIM];
+#pragma unroll
+      for (int k = 0; k < NDIM; k++) gk[k] = refgrad(k + 1, p);
+      if (vm.r == c0) {
+#pragma unroll
+        for (int k = 0; k < NDIM; k++) {
+          ag[0][k] = fmaf(gk[k], e0, ag[0][k]);
+          ag[1][k] = fmaf(gk[k], e1, ag[1][k]);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < NDIM; k++) {
+          ag[1][k] = fmaf(gk[k], e0, ag[1][k]);
+          ag[2][k] = fmaf(gk[k], e1, ag[2][k]);
+        }
+      }
+    }
+  };
+  if (!RUNS) {
+    for (int row = row_begin + warp; row < row_end; row += kEvalWarps) {
+      const RowDesc rd = R.rows[row];
+      const bool flip = bidir && (rd.y & 1);
+      for (int x = lane; x < nx; x += 32) general(rd, flip, x, (long long)row * nx + x);
+    }
+  }
+  // Most of a row has one interval, one range and one integer offset of the sample position: a run. Its
+  // parameters and tap rows stay in registers, and kTogether steps of 32 voxels have their loads in flight
+  // together; a step that leaves the run (by a vote on every voxel's own values) takes the general form
+  // and starts the next one. The values are the general form's, bit for bit.
+  constexpr int kTogether = 4;
+  for (int row = row_begin + warp; RUNS && row < row_end; row += kEvalWarps) {
     const RowDesc rd = R.rows[row];
-    const int z = row / ny;
-    const int y = row - z * ny;
-    const bool flip = bidir && (y & 1);
+    const bool flip = bidir && (rd.y & 1);
     const long long rowoff = (long long)row * nx;
-    for (int x = lane; x < nx; x += 32) {
+    int di = -1, r = 0, y_first = 0, z_first = 0, ox = 0;
+    float3 fl = make_float3(0.f, 0.f, 0.f);
+    float4 ph, dd;
+    bool run = false;
+    auto start = [&](int x) {  // the run that voxel x (the same for every lane) is in
       const VoxelModel vm = voxel_model(rd, x, nx, flip, bidir, dq);
-      // the host geometry guarantees c0-1 <= di <= c0+2; the clamp only keeps the shared-memory
-      // window in bounds
-      const int wi = min(max(vm.di - cw, 0), kWin - 2);
-      const float v = sample<NDIM, FT>(fr, job.fplane, job.fpitch, sD + wi * kDParamF4, vm.f, x, y, z, nx, ny, nz);
-      const long long p = rowoff + x;
-      const float t = refgrad(0, p);
-      // include iff the interpolated value is positive: CPU rule px == 0 -> -1, then wimg >= 0
-      // (FrameWarper.cpp:67, 16-25)
-      const float e = (v > 0.0f) ? v - t : 0.0f;
-      af = fmaf(e, e, af);
-      if (!vm.last) {
-        const float e1 = e * vm.f;           // weight of control r+1: Df
-        const float e0 = e * (1.0f - vm.f);  // weight of control r:   1 - Df
-        float gk[NDIM];
-        gk[0] = refgrad(1, p);
-        gk[1] = refgrad(2, p);
-        if (NDIM == 3) gk[NDIM - 1] = refgrad(3, p);
-        if (vm.r == c0) {
+      di = vm.di;
+      r = vm.r;
+      const float4* P = sD + min(max(di - cw, 0), kWin - 2) * kDParamF4;
+      const float4 n = P[0];
+      ph = P[1];
+      dd = P[2];
+      fl.x = floorf(fmaf(vm.f, dd.x, ph.x));
+      fl.y = floorf(fmaf(vm.f, dd.y, ph.y));
+      fl.z = NDIM == 3 ? floorf(fmaf(vm.f, dd.z, ph.z)) : 0.0f;
+      ox = (int)n.x + (int)fl.x;
+      y_first = min(max(rd.y + (int)n.y + (int)fl.y, -kHaloY), ny + kHaloY - 2);
+      z_first = NDIM == 3 ? min(max(rd.z + (int)n.z + (int)fl.z, -kHaloZ), nz + kHaloZ - 2) : 0;
+      // the taps x + ox, x + ox + 1 of every voxel of the row inside the halo
+      run = padded && ox >= -kHaloX && ox <= kHaloX - 1;
+    };
+    start(0);
+    for (int xb = 0; xb < nx; xb += 32 * kTogether) {
+      float f[kTogether], w[kTogether][NDIM];
+      bool same = run;
 #pragma unroll
-          for (int k = 0; k < NDIM; k++) {
-            ag[0][k] = fmaf(gk[k], e0, ag[0][k]);
-            ag[1][k] = fmaf(gk[k], e1, ag[1][k]);
-          }
-        } else {
+      for (int u = 0; u < kTogether; u++) {
+        const int x = min(xb + 32 * u + lane, nx - 1);
+        const VoxelModel vm = voxel_model(rd, x, nx, flip, bidir, dq);
+        f[u] = vm.f;
+        const float tx = fmaf(vm.f, dd.x, ph.x), ty = fmaf(vm.f, dd.y, ph.y);
+        w[u][0] = tx - fl.x;
+        w[u][1] = ty - fl.y;
+        same = same && vm.di == di && vm.r == r && !vm.last && floorf(tx) == fl.x && floorf(ty) == fl.y;
+        if (NDIM == 3) {
+          const float tz = fmaf(vm.f, dd.z, ph.z);
+          w[u][NDIM - 1] = tz - fl.z;
+          same = same && floorf(tz) == fl.z;
+        }
+      }
+      if (!__all_sync(0xffffffffu, same)) {
+#pragma unroll 1
+        for (int u = 0; u < kTogether; u++) {
+          const int x = xb + 32 * u + lane;
+          if (x < nx) general(rd, flip, x, rowoff + x);
+        }
+        __syncwarp();
+        start(min(xb + 32 * kTogether, nx - 1));
+        continue;
+      }
+      float v[kTogether][NDIM == 3 ? 8 : 4], t[kTogether], gk[kTogether][NDIM];
 #pragma unroll
-          for (int k = 0; k < NDIM; k++) {
-            ag[1][k] = fmaf(gk[k], e0, ag[1][k]);
-            ag[2][k] = fmaf(gk[k], e1, ag[2][k]);
+      for (int u = 0; u < kTogether; u++) {
+        const int x = min(xb + 32 * u + lane, nx - 1);
+        const FT* p = fr + ((long long)z_first * job.fplane + (long long)y_first * job.fpitch + (x + ox));
+        v[u][0] = ldf(p);
+        v[u][1] = ldf(p + 1);
+        v[u][2] = ldf(p + job.fpitch);
+        v[u][3] = ldf(p + job.fpitch + 1);
+        if (NDIM == 3) {
+          const FT* q = p + job.fplane;
+          v[u][NDIM == 3 ? 4 : 0] = ldf(q);
+          v[u][NDIM == 3 ? 5 : 0] = ldf(q + 1);
+          v[u][NDIM == 3 ? 6 : 0] = ldf(q + job.fpitch);
+          v[u][NDIM == 3 ? 7 : 0] = ldf(q + job.fpitch + 1);
+        }
+        t[u] = refgrad(0, rowoff + x);
+#pragma unroll
+        for (int k = 0; k < NDIM; k++) gk[u][k] = refgrad(k + 1, rowoff + x);
+      }
+#pragma unroll
+      for (int u = 0; u < kTogether; u++) {
+        const float c00 = fmaf(w[u][0], v[u][1] - v[u][0], v[u][0]);
+        const float c01 = fmaf(w[u][0], v[u][3] - v[u][2], v[u][2]);
+        float val = fmaf(w[u][1], c01 - c00, c00);
+        if (NDIM == 3) {
+          const float* h = v[u] + (NDIM == 3 ? 4 : 0);
+          const float c10 = fmaf(w[u][0], h[1] - h[0], h[0]);
+          const float c11 = fmaf(w[u][0], h[3] - h[2], h[2]);
+          const float c1 = fmaf(w[u][1], c11 - c10, c10);
+          val = fmaf(w[u][NDIM - 1], c1 - val, val);
+        }
+        if (xb + 32 * u + lane < nx) {
+          const float e = (val > 0.0f) ? val - t[u] : 0.0f;
+          af = fmaf(e, e, af);
+          const float e1 = e * f[u];
+          const float e0 = e * (1.0f - f[u]);
+          if (r == c0) {
+#pragma unroll
+            for (int k = 0; k < NDIM; k++) {
+              ag[0][k] = fmaf(gk[u][k], e0, ag[0][k]);
+              ag[1][k] = fmaf(gk[u][k], e1, ag[1][k]);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < NDIM; k++) {
+              ag[1][k] = fmaf(gk[u][k], e0, ag[1][k]);
+              ag[2][k] = fmaf(gk[u][k], e1, ag[2][k]);
+            }
           }
         }
       }
@@ -545,11 +659,18 @@ cudaError_t launch_eval4(const Job* jobs_dev, int n_jobs, int max_tiles, int n_d
 
 cudaError_t launch_eval(const Job* jobs_dev, int n_jobs, int max_tiles, int n_dim, int frame_kind, bool ref_bf16,
                         cudaStream_t s, bool rows_multiple_of_4, int mb) {
+  // One tile per CTA either way. Up to two tiles per SM a tile's latency counts: 168 tiles of 423 x 301 x 5
+  // (FP32) 23.8 us in the general form, 16.1 in runs; beyond, the run form's registers halve the resident
+  // warps: 4 FP32 frames of 511 x 511 x 16 168 us against 250 (8 mixed ones 302 against 288).
+  constexpr long long kScalarFew = 296;
   if (rows_multiple_of_4) return launch_eval4(jobs_dev, n_jobs, max_tiles, n_dim, frame_kind, ref_bf16, mb, s);
   const dim3 grid(max_tiles, n_jobs);
   return dispatch_cfg(n_dim, frame_kind, ref_bf16, [&](auto c) {
     using C = decltype(c);
-    eval_kernel<C::nd, typename C::F, typename C::R><<<grid, kEvalThreads, 0, s>>>(jobs_dev);
+    if ((long long)max_tiles * n_jobs <= kScalarFew)
+      eval_kernel<C::nd, typename C::F, typename C::R, true><<<grid, kEvalThreads, 0, s>>>(jobs_dev);
+    else
+      eval_kernel<C::nd, typename C::F, typename C::R, false><<<grid, kEvalThreads, 0, s>>>(jobs_dev);
     return cudaGetLastError();
   });
 }
@@ -564,8 +685,92 @@ __global__ void __launch_bounds__(kSolveThreads) reduce_kernel(const Job* __rest
   if (threadIdx.x == 0) job->result[0] = s_f;
 }
 
-cudaError_t launch_reduce(const Job* job_dev, cudaStream_t s, bool early) {
-  return launch_early(reduce_kernel, dim3(1), dim3(kSolveThreads), 0, s, early, job_dev);
+// reduce_partials for frames of many tiles, spread over CTAs: CTA c < nD of a frame takes control point c (its
+// tiles' sums are brought into shared memory by all threads and added in tile order by one thread per
+// component), CTA nD takes f. One CTA for everything waited for its own loads: 74 us of a step for
+// 1024 x 1024 x 64 (16384 tiles, 512 to 768 of them per control point). f goes to *f_out, g to g_out.
+constexpr int kWideThreads = 128, kWideStage = 512;
+static_assert(kWideThreads == kReduceRuns, "f runs");
+__device__ __forceinline__ void wide_reduce(const RefDev& R, const double* __restrict__ parts, double* f_out,
+                                            double* g_out, double* stage) {
+  const int tid = threadIdx.x;
+  if ((int)blockIdx.x == R.nD) {
+    double acc = 0.0;
+    for (int t = tid; t < R.n_tiles; t += kReduceRuns * kReduceDepth) {
+      double v[kReduceDepth];
+#pragma unroll
+      for (int u = 0; u < kReduceDepth; u++) {
+        const int tt = t + u * kReduceRuns;
+        v[u] = tt < R.n_tiles ? parts[(long long)tt * kPartialDoubles] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < kReduceDepth; u++) acc += v[u];
+    }
+    stage[tid] = acc;
+    __syncthreads();
+    if (tid < 32) {  // the tree of reduce_partials
+      double a = (stage[tid] + stage[tid + 64]) + (stage[tid + 32] + stage[tid + 96]);
+#pragma unroll
+      for (int w = 16; w > 0; w >>= 1) a += __shfl_down_sync(0xffffffffu, a, w);
+      if (tid == 0) *f_out = a;
+    }
+    __syncthreads();
+    return;
+  }
+  const int c = blockIdx.x, nd = R.n_dim;
+  const int4 tr = R.ctrl_tiles[c];
+  double a = 0.0;
+  for (int t0 = tr.x; t0 < tr.w; t0 += kWideStage) {
+    const int n = min(kWideStage, tr.w - t0);
+    __syncthreads();
+    for (int i = tid; i < n; i += kWideThreads) {
+      const int t = t0 + i, s = t < tr.y ? 2 : (t < tr.z ? 1 : 0);
+      const double* p = parts + (long long)t * kPartialDoubles + 2 + s * 3;
+      for (int k = 0; k < 3; k++) stage[k * kWideStage + i] = p[k];
+    }
+    __syncthreads();
+    if (tid < nd) {
+#pragma unroll 8
+      for (int i = 0; i < n; i++) a += stage[tid * kWideStage + i];
+    }
+  }
+  if (tid < nd) g_out[c * nd + tid] = a;
+  __syncthreads();
+}
+
+// The frames of a step: f to work[0] (and of the paired start's rigid point to work[1]), g to gt (and p).
+__global__ void __launch_bounds__(kWideThreads) wide_reduce_kernel(const Job* __restrict__ jobs,
+                                                                   const int* __restrict__ active,
+                                                                   const int* __restrict__ n_active, int bare) {
+  __shared__ double stage[3 * kWideStage];
+  if (active != nullptr && (int)blockIdx.y >= *n_active) return;
+  const Job& job = jobs[active != nullptr ? active[blockIdx.y] : blockIdx.y];
+  const RefDev& R = job.R;
+  if ((int)blockIdx.x > R.nD || R.n_tiles <= kWideTiles) return;
+  if (bare) {
+    wide_reduce(R, job.partials, job.result, job.result + 1, stage);
+    return;
+  }
+  const int phase = job.state->phase;
+  if (phase == kPhaseDone || phase == kPhaseWaitWarm) return;
+  wide_reduce(R, job.partials, job.work, job.gt, stage);
+  if (phase == kPhaseStartPair) wide_reduce(R, job.partials2, job.work + 1, job.p, stage);
+}
+
+bool wide_reduction(int n_tiles) { return n_tiles > kWideTiles; }
+
+cudaError_t launch_wide_reduce(const Job* jobs_dev, int n_jobs, int max_nD, cudaStream_t s, const int* active,
+                               const int* n_active) {
+  wide_reduce_kernel<<<dim3(max_nD + 1, n_jobs), kWideThreads, 0, s>>>(jobs_dev, active, n_active, 0);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_reduce(const Job* job_dev, int n_tiles, int nD, cudaStream_t s, bool overlap) {
+  if (n_tiles > kWideTiles) {
+    wide_reduce_kernel<<<dim3(nD + 1, 1), kWideThreads, 0, s>>>(job_dev, nullptr, nullptr, 1);
+    return cudaGetLastError();
+  }
+  return launch_overlapped(reduce_kernel, dim3(1), dim3(kSolveThreads), 0, s, overlap, job_dev);
 }
 
 // ------------------------------------------------------------------ warped image -----------------

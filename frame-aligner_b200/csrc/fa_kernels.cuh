@@ -14,6 +14,28 @@ constexpr int kEvalWarps = kEvalThreads / 32;
 constexpr int kReduceRuns = 128;
 constexpr int kSolveThreads = 256;
 
+// Passes and steps of few tiles may start while their predecessor on the stream still runs (programmatic
+// dependent launch): the kernel itself waits (cudaGridDependencySynchronize) before it touches what the
+// predecessor writes. A kernel that waits holds SMs (a step's CTA a whole one), so this is for solves that
+// have the device to themselves. One B200, a single-frame solve of an FP32 512 plane: 235 us without, 202
+// with; 20 frames of 256 x 256 (two groups that fit the device together) 717 and 657 us; 42 of 256 x 64 x 8
+// (five groups that do not) 594 and 681 (600 when the successor is let in late).
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool overlap,
+                                A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Exact float Sobel3d (Sobel3d.cpp:60-85) of an FP32 volume; with q16 also the BF16 groups of
 // launch_to_quad16.
 cudaError_t launch_sobel(const float* m, int nz, int ny, int nx, float* gx, float* gy, float* gz, __nv_bfloat16* q16,
@@ -62,10 +84,10 @@ cudaError_t launch_eval(const Job* jobs_dev, int n_jobs, int max_tiles, int n_di
 // launch can meet.
 cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const int* n_active, const int* tile_prefix,
                                 long long least_items, long long most_items, int n_dim, int frame_kind, bool ref_bf16,
-                                int mb, int grid, cudaStream_t s);
+                                int mb, int grid, cudaStream_t s, bool overlap = false);
 
 // Whether every pass of a solve of at most most_items items takes the form for few tiles: then its passes
-// and steps may overlap (the `early` of launch_solve).
+// and steps may overlap.
 bool eval4_few_only(long long most_items);
 
 // Thread-local (spill) bytes of that kernel's instantiation for a register budget of mb CTAs per SM.
@@ -77,25 +99,6 @@ size_t eval4_active_local_bytes(int n_dim, int frame_kind, bool ref_bf16, int mb
 // done_list[*n_done ...] (busy is cleared). A frame waiting for a warm start that has been written is
 // resumed. In a device-side loop (rounds non-null) the list that ends a round also counts it and repeats
 // the loop while a frame is active and fewer than max_rounds rounds ran.
-// Launches whose kernels may start while their predecessor on the stream still runs (programmatic
-// dependent launch): the kernel itself waits (cudaGridDependencySynchronize) before it touches what the
-// predecessor writes. Used where an iteration is short; a kernel that waits early holds its SMs.
-template <typename... P, typename... A>
-inline cudaError_t launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool early,
-                                A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = early ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
-
 constexpr int kListSlack = 32;  // entries that active and prefix have room for beyond n_jobs (+ 1)
 struct ActiveOut {
   int n_jobs;
@@ -116,9 +119,14 @@ cudaError_t launch_activate_peaks(const Job* jobs_dev, int n, const long long* p
 // Initialises the solve state of n frames (zero start, optional rigid and warm starts) and marks them busy.
 cudaError_t launch_activate(const Job* jobs_dev, const Activation* recs, int n, int* busy, cudaStream_t s);
 
-// Reduces one job's tile partials into result = [f, g(P)] (deterministic order). early: directly after a
-// few-tile pass, may start before the pass ends.
-cudaError_t launch_reduce(const Job* job_dev, cudaStream_t s, bool early = false);
+// Reduces one job's tile partials into result = [f, g(P)] (deterministic order). overlap: directly after
+// a few-tile pass.
+cudaError_t launch_reduce(const Job* job_dev, int n_tiles, int nD, cudaStream_t s, bool overlap = false);
+// Before launch_solve (same arguments) when a frame of it has many tiles (wide_reduction): those frames'
+// tile partials into the places where the step takes them from.
+bool wide_reduction(int n_tiles);
+cudaError_t launch_wide_reduce(const Job* jobs_dev, int n_jobs, int max_nD, cudaStream_t s, const int* active = nullptr,
+                               const int* n_active = nullptr);
 // Zero start of one frame's own solve (rigid: 3 doubles or null).
 cudaError_t launch_start(const Job* job_dev, const double* rigid, int max_iter, cudaStream_t s);
 
@@ -133,10 +141,10 @@ cudaError_t launch_warp(const RefDev* ref_dev, const RefDev& ref_host, const voi
 // above about 200 KB work in global memory). With `next`, the last CTA to finish builds the next active
 // list there (its list and length must not be `active` and `n_active`, which the launch's other CTAs may
 // still read; `finished` counts them and is zero between launches), and with end_of_round it also
-// controls the loop. early: the launch directly after a few-tile pass may start before the pass ends.
+// controls the loop. overlap: of a step directly after a pass of the same overlap.
 cudaError_t launch_solve(const Job* jobs_dev, int n_jobs, int max_nD, int n_dim, cudaStream_t s,
                          const int* active = nullptr, const int* n_active = nullptr, const ActiveOut* next = nullptr,
-                         unsigned* finished = nullptr, bool end_of_round = false, bool early = false);
+                         unsigned* finished = nullptr, bool end_of_round = false, bool overlap = false);
 
 // Test hook: the device trust-region subproblem on given dense H (P x P) and g.
 // The band Cholesky factor of H (lambda = 0) into L0 (nD * nd rows of 2 * nd) and inv0 (nD * nd); *ok

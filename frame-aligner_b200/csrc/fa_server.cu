@@ -300,7 +300,6 @@ fa_status class_capture(fa_server* S, SrvClass* C) {
   C->graph = nullptr;
   cudaStream_t s = C->stream;
   const long long most_items = 2LL * C->bound * C->max_tiles;
-  const bool early = C->vec4 && fa::eval4_few_only(most_items);
   // the steps alternate between two lists; the list before the first step is list 0
   auto list_out = [&](int which) {
     fa::ActiveOut o{};
@@ -322,12 +321,14 @@ fa_status class_capture(fa_server* S, SrvClass* C) {
       if (C->vec4)
         e = fa::launch_eval4_active(C->jobs_dev, in.active, in.n_active, in.prefix, C->min_tiles,
                                     most_items, C->n_dim, C->kind, C->bf16, C->mb,
-                                    C->grid_mult * S->sms, s);
+                                    C->grid_mult * S->sms, s);  // (classes run beside one another: no overlap)
       else
         e = fa::launch_eval(C->jobs_dev, C->bound, C->max_tiles, C->n_dim, C->kind, C->bf16, s, false);
+      if (e == cudaSuccess && fa::wide_reduction(C->max_tiles))
+        e = fa::launch_wide_reduce(C->jobs_dev, C->bound, C->max_nD, s, in.active, in.n_active);
       if (e == cudaSuccess)
         e = fa::launch_solve(C->jobs_dev, C->bound, C->max_nD, C->n_dim, s, in.active, in.n_active, &out,
-                             reinterpret_cast<unsigned*>(C->next + 1), false, early);
+                             reinterpret_cast<unsigned*>(C->next + 1));
     }
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(C->h_counts, C->counts, (size_t)(C->cap + 2) * sizeof(int), cudaMemcpyDeviceToHost, s);

@@ -717,9 +717,19 @@ __device__ __forceinline__ int solve_step(const Job* job_src, double* s_dyn) {
   }
   cudaGridDependencySynchronize();  // the fused pass's partial sums (everything above is older)
   cudaTriggerProgrammaticLaunchCompletion();  // the next pass may come in and wait for this launch's end
-  reduce_partials(R, job.partials, &s_f, gt);
-  // paired start: the rigid point's sums, its gradient into p (free until the first step)
-  if (pair) reduce_partials(R, job.partials2, &s_f2, p);
+  if (R.n_tiles > kWideTiles) {  // reduced by the launch before this one (p, too, in the paired start)
+    if (threadIdx.x == 0) {
+      s_f = job.work[0];
+      s_f2 = job.work[1];
+    }
+    if constexpr (STAGED)
+      for (int i = threadIdx.x; i < P; i += blockDim.x) gt[i] = job.gt[i];
+    __syncthreads();
+  } else {
+    reduce_partials(R, job.partials, &s_f, gt);
+    // paired start: the rigid point's sums, its gradient into p (free until the first step)
+    if (pair) reduce_partials(R, job.partials2, &s_f2, p);
+  }
   state_step<ND>(S, B, x, g, p, gt, work, s_f, pair ? s_f2 : 0.0, s_red, &s_flag);
   if constexpr (STAGED) {
     for (int i = threadIdx.x; i < P; i += blockDim.x) {
@@ -806,28 +816,28 @@ namespace {
 template <int ND>
 cudaError_t launch_solve_nd(const Job* jobs_dev, int n_jobs, int max_nD, cudaStream_t s, const int* active,
                             const int* n_active, const ActiveOut& next, unsigned* finished, int end_of_round,
-                            bool early) {
+                            bool overlap) {
   constexpr long long kCapBytes = 200 * 1024;
   const long long need = solve_smem_doubles(max_nD, ND) * (long long)sizeof(double);
   if (need > kCapBytes)  // every frame of the launch works in global memory
-    return launch_early(solve_kernel<ND, false>, dim3(n_jobs), dim3(kSolveThreads), 0, s, early, jobs_dev, active,
-                        n_active, next, finished, end_of_round);
+    return launch_overlapped(solve_kernel<ND, false>, dim3(n_jobs), dim3(kSolveThreads), 0, s, overlap, jobs_dev, active,
+                             n_active, next, finished, end_of_round);
   if (need > 40 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(solve_kernel<ND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
     if (e != cudaSuccess) return e;
   }
-  return launch_early(solve_kernel<ND, true>, dim3(n_jobs), dim3(kSolveThreads), (size_t)need, s, early, jobs_dev,
-                      active, n_active, next, finished, end_of_round);
+  return launch_overlapped(solve_kernel<ND, true>, dim3(n_jobs), dim3(kSolveThreads), (size_t)need, s, overlap, jobs_dev,
+                           active, n_active, next, finished, end_of_round);
 }
 }  // namespace
 
 cudaError_t launch_solve(const Job* jobs_dev, int n_jobs, int max_nD, int n_dim, cudaStream_t s, const int* active,
-                         const int* n_active, const ActiveOut* next, unsigned* finished, bool end_of_round, bool early) {
+                         const int* n_active, const ActiveOut* next, unsigned* finished, bool end_of_round, bool overlap) {
   const ActiveOut out = next ? *next : ActiveOut{};
   unsigned* count = next ? finished : nullptr;
   const int end = end_of_round ? 1 : 0;
-  return n_dim == 3 ? launch_solve_nd<3>(jobs_dev, n_jobs, max_nD, s, active, n_active, out, count, end, early)
-                    : launch_solve_nd<2>(jobs_dev, n_jobs, max_nD, s, active, n_active, out, count, end, early);
+  return n_dim == 3 ? launch_solve_nd<3>(jobs_dev, n_jobs, max_nD, s, active, n_active, out, count, end, overlap)
+                    : launch_solve_nd<2>(jobs_dev, n_jobs, max_nD, s, active, n_active, out, count, end, overlap);
 }
 
 // The factor of H itself, once per reference: one block brings the blocks of H into shared memory (when

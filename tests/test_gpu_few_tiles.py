@@ -1,6 +1,7 @@
-"""GPU: the fused pass's form for few tiles (csrc/fa_eval4.cu, eval4_tile_cta: one tile per CTA, errors
-by all warps, then the summation chains) at the edges of its range, and against the one-warp-per-tile
-form, whose partial sums it has to reproduce bit for bit.
+"""GPU: the fused pass's forms for few tiles (csrc/fa_eval4.cu, eval4_tile_cta: one tile per CTA, errors
+by all warps, then the summation chains; csrc/fa_kernels.cu, eval_kernel in runs, for rows that are no
+multiple of four voxels) at the edges of their range, and the first against the one-warp-per-tile form,
+whose partial sums it has to reproduce bit for bit.
 
 Tolerances, against the FP64 statement of one evaluation on the values the device stores
 (oracle_py.fp64_error_jacobian): the summation bounds of test_gpu_mixed.py, f relative 5e-6 and J^T e
@@ -34,7 +35,9 @@ def _acq(shape, nD, n_frames=1):
 # more than 32 segments (narrow rows: several batches), of fewer than 32 (short volumes, one warp's
 # worth), a last tile that is cut, one range per tile and two
 SHAPES = [((1, 64, 4), 4), ((1, 700, 8), 5), ((1, 96, 128), 6), ((1, 70, 132), 5), ((1, 33, 1028), 4),
-          ((2, 40, 64), 6), ((5, 61, 100), 10), ((3, 37, 256), 7), ((16, 24, 384), 32)]
+          ((2, 40, 64), 6), ((5, 61, 100), 10), ((3, 37, 256), 7), ((16, 24, 384), 32),
+          # rows that are no multiple of four: shorter than a step of 32 voxels, of one, of four and a little more
+          ((1, 64, 5), 4), ((1, 300, 33), 5), ((1, 70, 127), 6), ((1, 90, 129), 6), ((5, 61, 103), 10), ((3, 37, 257), 7)]
 
 
 @pytest.mark.parametrize("precision", [fa.PREC_F32, fa.PREC_MIXED], ids=["f32", "mixed"])
