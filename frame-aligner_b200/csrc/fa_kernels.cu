@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(kWideThreads) wide_reduce_kernel(const Job* __
   if (active != nullptr && (int)blockIdx.y >= *n_active) return;
   const Job& job = jobs[active != nullptr ? active[blockIdx.y] : blockIdx.y];
   const RefDev& R = job.R;
-  if ((int)blockIdx.x > R.nD || R.n_tiles <= kWideTiles) return;
+  if ((int)blockIdx.x > R.nD || (R.n_tiles <= kWideTiles && !bare)) return;
   if (bare) {
     wide_reduce(R, job.partials, job.result, job.result + 1, stage);
     return;
@@ -766,7 +766,10 @@ cudaError_t launch_wide_reduce(const Job* jobs_dev, int n_jobs, int max_nD, cuda
 }
 
 cudaError_t launch_reduce(const Job* job_dev, int n_tiles, int nD, cudaStream_t s, bool overlap) {
-  if (n_tiles > kWideTiles) {
+  // A bare evaluation's reduction is a launch of its own either way: 1024 tiles (512 x 512 x 16) 65 us a call
+  // with one CTA, 59 with many; a step's would be one launch more (271 -> 299 us a solve there).
+  constexpr int kBareWideTiles = 768;
+  if (n_tiles > kBareWideTiles) {
     wide_reduce_kernel<<<dim3(nD + 1, 1), kWideThreads, 0, s>>>(job_dev, nullptr, nullptr, 1);
     return cudaGetLastError();
   }
