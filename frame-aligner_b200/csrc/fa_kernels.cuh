@@ -188,7 +188,7 @@ cudaError_t launch_phase_argmax_final(const double* block_val, const long long* 
 struct PlaneDims {
   int nz, ny, nx, rows;      // rows = nz * ny
   int log2M, log2ny, log2G;  // M = nx / 2; G rows per row CTA
-  int PP;                    // planes per plane CTA (one-kernel (z, y) pass); 0 when split
+  int PP;                    // planes in 8192 points, two CTAs' (one-kernel (z, y) pass); 0 when split
   int n_twx, tw_x_post;      // x twiddles: stage table of the nx/2-point DFT, then W_nx^k (k <= nx/2)
   int n_twy;                 // y twiddles: stage table of the ny-point DFT
   long long n_complex, n_el;

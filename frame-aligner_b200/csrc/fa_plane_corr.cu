@@ -16,7 +16,7 @@
 //                           an nx/2-point complex inverse DFT) and the first maximum of the real
 //                           surface in flat (z, y, x) order, per CTA; then phase_argmax_final
 //
-// Planes too large for one CTA (nz * ny > 8192 or nz > 16, power-of-two nz >= 8) split the middle
+// Planes too large for a pair of CTAs (nz * ny > 8192 or nz > 16, power-of-two nz >= 8) split the middle
 // pass in three: plane_y_kernel (DFT of y lines, in place), plane_z_kernel (per kx plane and block of
 // y columns: DFT along z, cross-power with the reference, inverse DFT along z) and plane_y_kernel
 // again (inverse), so every volume of these dimensions stays off cuFFT.
@@ -267,8 +267,14 @@ namespace {
 
 constexpr int kRowThreads = 256;
 constexpr int kRowEPT = 8;      // G * nx/2 <= 2048 points per row CTA
-constexpr int kPlaneThreads = 512;
-constexpr int kPlaneEPT = 16;   // PP * nz * ny <= 8192 points per plane CTA
+// CTAs of the (z, y) pass hold 4096 points with 256 threads, two to an SM (128 registers a thread, about 74
+// KB of shared memory each), so that one loads or stores while the other computes, and small batches
+// have twice the CTAs. The whole correlation, before (8192 points with 512 threads, one to an SM) and
+// after: two frames of 1024 x 1024 x 64 4242 -> 3719 us, eight of 512 x 512 x 8 306 -> 284, 16 of 256 x 256
+// 107 -> 91.
+constexpr int kPlaneThreads = 256;
+constexpr int kPlaneEPT = 16;
+constexpr int kPlanePoints = kPlaneThreads * kPlaneEPT;
 
 // Global -> shared staging in 16-byte chunks: chunk i is read from src_of(i) and written to
 // dst_of(i), with K loads of each thread in flight before the first store. Published by the
@@ -375,21 +381,27 @@ __device__ __forceinline__ double2 cross_power(double2 a, double2 b) {
   return make_double2(re * r, im * r);
 }
 
-// Planes p0 .. p0 + PP - 1 of the batch's plane array (frame-major, nx/2 + 1 planes per frame).
-// REF: out = conj(forward DFT over (z, y)); otherwise out = inverse(normalised forward * ref_conj).
-// Shared memory: PP * NZ lines of S = ny + 1 points, then the ny twiddles W_ny^m.
+// Planes p0 .. p0 + pp - 1 of the batch's plane array (frame-major, nx/2 + 1 planes per frame), pp =
+// planes_of_cta. REF: out = conj(forward DFT over (z, y)); otherwise out = inverse(normalised forward *
+// ref_conj). Shared memory: pp * NZ lines of S = ny + 1 points, then the ny twiddles W_ny^m.
+__host__ __device__ inline int planes_of_cta(int nz, int ny) {
+  const int points = nz * ny;  // at most kPlanePoints (larger planes: a pair of CTAs, or the split pass)
+  return points < kPlanePoints ? kPlanePoints / points : 1;
+}
+
 template <int NZ, bool REF>
-__global__ void __launch_bounds__(kPlaneThreads, 1) plane_yz_kernel(const double2* in, double2* out,
+__global__ void __launch_bounds__(kPlaneThreads, 2) plane_yz_kernel(const double2* in, double2* out,
                                                                     const double2* __restrict__ ref_conj,
                                                                     const double2* __restrict__ tw_y, PlaneDims d,
                                                                     long long n_planes) {
   extern __shared__ double2 sm[];
   const int ny = d.ny, S = ny + 1;
   const int plane = NZ * ny;
-  const long long p0 = (long long)blockIdx.x * d.PP;
-  const int pp = (int)min((long long)d.PP, n_planes - p0);
+  const int most = planes_of_cta(NZ, ny);
+  const long long p0 = (long long)blockIdx.x * most;
+  const int pp = (int)min((long long)most, n_planes - p0);
   const int E = pp * plane;
-  double2* tws = sm + d.PP * NZ * S;
+  double2* tws = sm + most * NZ * S;
   const double2* src = in + p0 * plane;
   stage16<4>(
       d.n_twy, [&](int i) { return reinterpret_cast<const uint4*>(tw_y) + i; },
@@ -536,7 +548,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 2)
 // memory and the last writes it (ny >= 16: at least two stages, so a CTA reads all its lines before
 // it writes any). Shared memory: LY lines of S = ny + 1 points, then the ny twiddle slots.
 template <bool INV>
-__global__ void __launch_bounds__(kPlaneThreads, 1) plane_y_kernel(double2* spec, const double2* __restrict__ tw_y,
+__global__ void __launch_bounds__(kPlaneThreads, 2) plane_y_kernel(double2* spec, const double2* __restrict__ tw_y,
                                                                    PlaneDims d, long long n_lines) {
   extern __shared__ double2 sm[];
   const int ny = d.ny, S = ny + 1;
@@ -558,7 +570,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) plane_y_kernel(double2* spec
 // the reference, conjugated and written to ref_out), transformed back and stored along y.
 // Shared memory: YB lines of S = nz + 1 points, then the nz twiddle slots.
 template <bool REF>
-__global__ void __launch_bounds__(kPlaneThreads, 1) plane_z_kernel(double2* spec, double2* ref_out,
+__global__ void __launch_bounds__(kPlaneThreads, 2) plane_z_kernel(double2* spec, double2* ref_out,
                                                                    const double2* __restrict__ ref_conj,
                                                                    const double2* __restrict__ tw_z, PlaneDims d) {
   extern __shared__ double2 sm[];
@@ -769,13 +781,13 @@ void plane_twiddles(const PlaneDims& d, std::vector<double2>* tw_x, std::vector<
 
 bool plane_dims(int nz, int ny, int nx, PlaneDims* d) {
   if (!pow2(nz) || !pow2(ny) || !pow2(nx) || ny < 8 || ny > 2048 || nx < 16 || nx > 4096) return false;
-  const bool fits = nz <= 16 && (long long)nz * ny <= kPlaneThreads * kPlaneEPT;
-  // split pass: z columns of 8 .. 1024 points (at least 8 columns per CTA), y lines of >= 16 points
+  const bool fits = nz <= 16 && (long long)nz * ny <= 2 * kPlanePoints;
+  // split pass: z columns of 8 .. 1024 points (at least 4 columns per CTA), y lines of >= 16 points
   if (!fits && (nz < 8 || nz > 1024 || ny < 16)) return false;
   d->split = !fits;
   d->log2nz = ilog2(nz);
-  d->LY = std::max(1, (kPlaneThreads * kPlaneEPT) / ny);
-  d->log2YB = ilog2(std::min<long long>(ny, (kPlaneThreads * kPlaneEPT) / nz));
+  d->LY = std::max(1, kPlanePoints / ny);
+  d->log2YB = ilog2(std::min<long long>(ny, kPlanePoints / nz));
   d->n_twz = d->split ? stage_count(nz) : 0;
   d->nz = nz;
   d->ny = ny;
@@ -786,7 +798,7 @@ bool plane_dims(int nz, int ny, int nx, PlaneDims* d) {
   int G = 8;
   while (G > 1 && ((long long)G * (nx / 2) > (long long)kRowThreads * kRowEPT || G > d->rows)) G >>= 1;
   d->log2G = ilog2(G);
-  d->PP = d->split ? 0 : std::max(1, (kPlaneThreads * kPlaneEPT) / (nz * ny));
+  d->PP = d->split ? 0 : std::max(1, 2 * kPlanePoints / (nz * ny));
   d->n_complex = (long long)(nx / 2 + 1) * d->rows;
   d->n_el = (long long)nx * d->rows;
   d->tw_x_post = stage_count(nx / 2);
@@ -839,10 +851,12 @@ cudaError_t launch_yz(const PlaneDims& d, const double2* in, double2* out, const
       return cudaGetLastError();
     }
   }
-  const size_t smem = ((size_t)d.PP * NZ * (d.ny + 1) + d.ny) * sizeof(double2);
+  const int pp = planes_of_cta(NZ, d.ny);
+  if (pp * NZ * d.ny > kPlanePoints) return cudaErrorInvalidValue;
+  const size_t smem = ((size_t)pp * NZ * (d.ny + 1) + d.ny) * sizeof(double2);
   cudaError_t e = allow_smem(plane_yz_kernel<NZ, REF>, smem);
   if (e != cudaSuccess) return e;
-  const long long grid = (n_planes + d.PP - 1) / d.PP;
+  const long long grid = (n_planes + pp - 1) / pp;
   plane_yz_kernel<NZ, REF><<<(unsigned)grid, kPlaneThreads, smem, s>>>(in, out, ref_conj, tw_y, d, n_planes);
   return cudaGetLastError();
 }
