@@ -1327,61 +1327,43 @@ extern "C" fa_status fa_align_batch(fa_frame* const* frames, int n, const double
 
 namespace fa_rt {
 
-// Pointer staging for a batch of n inputs (pinned host + device arrays), grown on demand.
+// Peak slots of a batch of n inputs, grown on demand.
 fa_status correlator_reserve(fa_correlator* C, int n) {
-  if (n <= C->ptr_cap) return FA_OK;
+  if (n <= C->idx_cap) return FA_OK;
   FA_CU(cudaStreamSynchronize(C->stream));
-  dfree_all(C->ctx, C->ptr_allocs);
-  if (C->h_ptrs) cudaFreeHost(C->h_ptrs);
-  if (C->h_idx) cudaFreeHost(C->h_idx);
-  C->h_ptrs = nullptr;
-  C->h_idx = nullptr;
-  C->ptr_cap = 0;
-  FA_TRY(dalloc_t(C->ctx, 2 * (size_t)n, &C->d_ptrs, C->ptr_allocs));
-  FA_TRY(dalloc_t(C->ctx, (size_t)n, &C->d_idx, C->ptr_allocs));
-  if (cudaMallocHost(&C->h_ptrs, 2 * (size_t)n * sizeof(void*)) != cudaSuccess ||
-      cudaMallocHost(&C->h_idx, (size_t)n * sizeof(long long)) != cudaSuccess)
+  dfree_all(C->ctx, C->idx_allocs);
+  C->idx_cap = 0;
+  FA_TRY(dalloc_t(C->ctx, (size_t)n, &C->d_idx, C->idx_allocs));
+  if (!C->h_idx && cudaMallocHost(&C->h_idx, sizeof(long long)) != cudaSuccess)
     return fail(FA_ERR_OOM, "cudaMallocHost failed");
-  C->ptr_cap = n;
+  C->idx_cap = n;
   return FA_OK;
 }
 
 // Window, forward DFT, cross-power normalisation, inverse DFT and first-maximum argmax for n volumes
-// (device pointers, FP32 or raw uint16) in batches of C->cap; peak indices to C->d_idx[first ..].
+// (device pointers, FP32 or raw uint16) in batches of C->cap; peak indices to peaks,
+// or to C->d_idx[first ..].
 fa_status correlator_enqueue(fa_correlator* C, const void* const* vols, int in_kind, int n, double* surface,
                              bool planes, int first, void* const* slots, int slot_kind, int slot_pitch,
-                             long long slot_plane, bool* slots_written) {
+                             long long slot_plane, bool* slots_written, long long* peaks, bool alone) {
   if (slots_written) *slots_written = false;
-  if (first > 0 && first + n > C->ptr_cap) return fail(FA_ERR_STATE, "correlator slots not reserved");
+  if (first > 0 && first + n > C->idx_cap) return fail(FA_ERR_STATE, "correlator slots not reserved");
   FA_TRY(correlator_reserve(C, first + n));
   // the fused passes stage frames in 16-byte chunks: 16-byte aligned frames only
-  for (int i = 0; i < n; i++) {
-    C->h_ptrs[first + i] = vols[i];
+  for (int i = 0; i < n; i++)
     if (reinterpret_cast<uintptr_t>(vols[i]) % 16) planes = false;
-  }
   planes = planes && C->planes;
-  FA_CU(cudaMemcpyAsync(C->d_ptrs + first, C->h_ptrs + first, (size_t)n * sizeof(void*), cudaMemcpyHostToDevice,
-                        C->stream));
-  const void* const* d_ptrs = C->d_ptrs + first;
   // slots filled by the first pass: 16-byte aligned rows, and a raw uint16 slot only from uint16 frames
   const size_t slot_esz = slot_kind == fa::kFrameF32 ? 4 : 2;
   const bool fill = planes && slots && (slot_kind != fa::kFrameRawU16 || in_kind == FA_U16) &&
                     ((size_t)slot_pitch * slot_esz) % 16 == 0 && ((size_t)slot_plane * slot_esz) % 16 == 0 &&
                     C->nx % 8 == 0;
   bool fill_ok = fill;
-  if (fill) {
-    for (int i = 0; i < n; i++) {
-      C->h_ptrs[C->ptr_cap + first + i] = slots[i];
-      if (reinterpret_cast<uintptr_t>(slots[i]) % 16) fill_ok = false;
-    }
-  }
-  fa::SlotOut slot_out{};
-  if (fill_ok) {
-    FA_CU(cudaMemcpyAsync(C->d_ptrs + C->ptr_cap + first, C->h_ptrs + C->ptr_cap + first, (size_t)n * sizeof(void*),
-                          cudaMemcpyHostToDevice, C->stream));
-    slot_out = fa::SlotOut{C->d_ptrs + C->ptr_cap + first, slot_kind, slot_pitch, slot_plane};
-  }
-  long long* d_idx = C->d_idx + first;
+  for (int i = 0; fill && i < n; i++)
+    if (reinterpret_cast<uintptr_t>(slots[i]) % 16) fill_ok = false;
+  fa::FramePtrs in{};
+  fa::SlotOut slot_out{{}, slot_kind, slot_pitch, slot_plane};
+  if (!peaks) peaks = C->d_idx + first;
   if (!planes && C->planes && !C->ref_conj_rows) {  // a plane-path correlator falling back to cuFFT
     FA_CU(cudaStreamSynchronize(C->stream));
     FA_TRY(dalloc_t(C->ctx, (size_t)C->n_el * C->cap, &C->real, C->allocs));
@@ -1393,30 +1375,31 @@ fa_status correlator_enqueue(fa_correlator* C, const void* const* vols, int in_k
     int m = C->cap;  // the largest power-of-two batch that fits the rest
     while (m > n - c0) m >>= 1;
     double* surf = surface ? surface + (size_t)c0 * C->n_el : nullptr;
+    for (int i = 0; i < m; i++) {
+      in.p[i] = vols[c0 + i];
+      if (fill_ok) slot_out.p[i] = slots[c0 + i];
+    }
     if (planes) {
       const int nb = fa::plane_blocks_per_frame(C->pd);
-      fa::SlotOut so = slot_out;
-      if (fill_ok) so.ptrs += c0;
-      FA_CU(fa::launch_plane_rows_fwd(C->pd, d_ptrs + c0, in_kind, m, C->wy, C->wx, C->tw_x, C->spec, C->stream,
-                                      fill_ok ? &so : nullptr));
+      FA_CU(fa::launch_plane_rows_fwd(C->pd, in, in_kind, m, C->wy, C->wx, C->tw_x, C->spec, C->stream,
+                                      fill_ok ? &slot_out : nullptr));
       if (C->pd.split)
-        FA_CU(fa::launch_plane_yz_split(C->pd, C->spec, C->ref_conj, C->tw_y, C->tw_z, m, false, C->stream));
+        FA_CU(fa::launch_plane_yz_split(C->pd, C->spec, C->ref_conj, C->tw_y, C->tw_z, m, false, C->stream, alone));
       else
-        FA_CU(fa::launch_plane_yz(C->pd, C->spec, C->spec, C->ref_conj, C->tw_y, m, false, C->stream));
-      FA_CU(fa::launch_plane_rows_inv_argmax(C->pd, C->spec, m, C->tw_x, C->bval, C->bidx, surf, C->stream));
-      FA_CU(fa::launch_phase_argmax_final(C->bval, C->bidx, nb, m, d_idx + c0, C->stream));
+        FA_CU(fa::launch_plane_yz(C->pd, C->spec, C->spec, C->ref_conj, C->tw_y, m, false, C->stream, alone));
+      FA_CU(fa::launch_plane_rows_inv_argmax(C->pd, C->spec, m, C->tw_x, C->bval, C->bidx, surf, C->stream, alone));
+      FA_CU(fa::launch_phase_argmax_final(C->bval, C->bidx, nb, m, peaks + c0, C->stream, alone));
       g_launches += C->pd.split ? 6 : 4;
     } else {
       cufftHandle fwd, inv;
       FA_TRY(correlator_plans(C, m, &fwd, &inv));
-      FA_CU(fa::launch_phase_window(d_ptrs + c0, in_kind, C->wy, C->wx, C->ny, C->nx, C->n_el, m, C->real,
-                                    C->stream));
+      FA_CU(fa::launch_phase_window(in, in_kind, C->wy, C->wx, C->ny, C->nx, C->n_el, m, C->real, C->stream));
       if (cufftExecD2Z(fwd, C->real, reinterpret_cast<cufftDoubleComplex*>(C->spec)) != CUFFT_SUCCESS)
         return fail(FA_ERR_CUDA, "cufftExecD2Z failed");
       FA_CU(fa::launch_phase_normalise(C->spec, ref_rows, C->n_complex, m, C->stream));
       if (cufftExecZ2D(inv, reinterpret_cast<cufftDoubleComplex*>(C->spec), C->real) != CUFFT_SUCCESS)
         return fail(FA_ERR_CUDA, "cufftExecZ2D failed");
-      FA_CU(fa::launch_phase_argmax(C->real, C->n_el, m, C->bval, C->bidx, C->n_blocks, d_idx + c0, C->stream));
+      FA_CU(fa::launch_phase_argmax(C->real, C->n_el, m, C->bval, C->bidx, C->n_blocks, peaks + c0, C->stream));
       if (surf)
         FA_CU(cudaMemcpyAsync(surf, C->real, (size_t)m * C->n_el * sizeof(double), cudaMemcpyDeviceToDevice,
                               C->stream));
@@ -1449,10 +1432,11 @@ void unravel_shift(const fa_correlator* C, long long idx, double* shift) {
 
 namespace {
 
-fa_status correlator_read(fa_correlator* C, int n, double* shifts) {
-  FA_CU(cudaMemcpyAsync(C->h_idx, C->d_idx, (size_t)n * sizeof(long long), cudaMemcpyDeviceToHost, C->stream));
+// One volume's shift: the last pass writes the peak index to host memory, with no copy behind it.
+fa_status correlator_shift_one(fa_correlator* C, const void* volume, double* shift) {
+  FA_TRY(correlator_enqueue(C, &volume, FA_F32, 1, nullptr, true, 0, nullptr, 0, 0, 0, nullptr, C->h_idx, true));
   FA_CU(cudaStreamSynchronize(C->stream));
-  for (int i = 0; i < n; i++) unravel_shift(C, C->h_idx[i], shifts + 3 * i);
+  unravel_shift(C, *C->h_idx, shift);
   return FA_OK;
 }
 
@@ -1576,9 +1560,8 @@ fa_status correlator_create_impl(fa_context* ctx, const void* reference, bool re
                       ref_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, C->stream) != cudaSuccess)
     return cleanup(fail(FA_ERR_CUDA, "reference upload"));
   if ((st = correlator_reserve(C, 1)) != FA_OK) return cleanup(st);
-  C->h_ptrs[0] = C->vol;
-  if (cudaMemcpyAsync(C->d_ptrs, C->h_ptrs, sizeof(void*), cudaMemcpyHostToDevice, C->stream) != cudaSuccess)
-    return cleanup(fail(FA_ERR_CUDA, "pointer upload"));
+  fa::FramePtrs ref_ptr{};
+  ref_ptr.p[0] = C->vol;
   if (C->planes) {
     std::vector<double2> tx, ty, tz;
     fa::plane_twiddles(C->pd, &tx, &ty, &tz);
@@ -1591,7 +1574,7 @@ fa_status correlator_create_impl(fa_context* ctx, const void* reference, bool re
          cudaMemcpy(C->tw_z, tz.data(), tz.size() * sizeof(double2), cudaMemcpyHostToDevice) != cudaSuccess))
       return cleanup(fail(FA_ERR_CUDA, "twiddle upload"));
     const cudaError_t e_fwd =
-        fa::launch_plane_rows_fwd(C->pd, C->d_ptrs, FA_F32, 1, C->wy, C->wx, C->tw_x, C->spec, C->stream);
+        fa::launch_plane_rows_fwd(C->pd, ref_ptr, FA_F32, 1, C->wy, C->wx, C->tw_x, C->spec, C->stream);
     const cudaError_t e_yz =
         e_fwd != cudaSuccess ? e_fwd
         : C->pd.split
@@ -1601,7 +1584,7 @@ fa_status correlator_create_impl(fa_context* ctx, const void* reference, bool re
   } else {
     cufftHandle fwd1, inv1;
     if ((st = correlator_plans(C, 1, &fwd1, &inv1)) != FA_OK) return cleanup(st);
-    if (fa::launch_phase_window(C->d_ptrs, FA_F32, C->wy, C->wx, ny, nx, C->n_el, 1, C->real, C->stream) !=
+    if (fa::launch_phase_window(ref_ptr, FA_F32, C->wy, C->wx, ny, nx, C->n_el, 1, C->real, C->stream) !=
         cudaSuccess)
       return cleanup(fail(FA_ERR_CUDA, "window kernel"));
     if (cufftExecD2Z(fwd1, C->real, reinterpret_cast<cufftDoubleComplex*>(C->spec)) != CUFFT_SUCCESS)
@@ -1635,10 +1618,9 @@ extern "C" fa_status fa_correlator_destroy(fa_correlator* C) {
   }
   C->plans.clear();
   dfree_all(C->ctx, C->work_allocs);
-  if (C->h_ptrs) cudaFreeHost(C->h_ptrs);
   if (C->h_idx) cudaFreeHost(C->h_idx);
   if (C->stream) cudaStreamDestroy(C->stream);
-  dfree_all(C->ctx, C->ptr_allocs);
+  dfree_all(C->ctx, C->idx_allocs);
   dfree_all(C->ctx, C->allocs);
   delete C;
   return FA_OK;
@@ -1649,18 +1631,14 @@ extern "C" fa_status fa_correlator_shift(fa_correlator* C, const float* volume, 
   std::lock_guard<std::mutex> lk(C->mu);
   FA_CU(cudaSetDevice(C->ctx->device));
   FA_CU(cudaMemcpyAsync(C->vol, volume, (size_t)C->n_el * sizeof(float), cudaMemcpyHostToDevice, C->stream));
-  const void* v = C->vol;
-  FA_TRY(correlator_enqueue(C, &v, FA_F32, 1));
-  return correlator_read(C, 1, shift);
+  return correlator_shift_one(C, C->vol, shift);
 }
 
 extern "C" fa_status fa_correlator_shift_device(fa_correlator* C, const float* volume_device, double* shift) {
   if (!C || !volume_device || !shift) return fail(FA_ERR_BAD_ARG, "NULL argument");
   std::lock_guard<std::mutex> lk(C->mu);
   FA_CU(cudaSetDevice(C->ctx->device));
-  const void* v = volume_device;
-  FA_TRY(correlator_enqueue(C, &v, FA_F32, 1));
-  return correlator_read(C, 1, shift);
+  return correlator_shift_one(C, volume_device, shift);
 }
 
 // ================================================================== test hooks ====================
@@ -2142,7 +2120,7 @@ extern "C" fa_status fa_aligner_set_reference(fa_aligner* A, const void* referen
   FA_CU(fa::launch_downsample(raw, dtype, nz, ny, nx, b, static_cast<float*>(down), A->stream));
   FA_CU(cudaStreamSynchronize(A->stream));
   // Frames go through the correlator in batched cuFFT plans of up to 64 frames (less for large volumes).
-  fa_status st = correlator_create_impl(A->ctx, down, true, A->dz, A->dy, A->dx, 64, &A->corr);
+  fa_status st = correlator_create_impl(A->ctx, down, true, A->dz, A->dy, A->dx, fa::kCorrFrames, &A->corr);
   if (st == FA_OK)
     st = fa_set_reference_device(A->ctx, static_cast<const float*>(plus1), nz, ny, nx, A->nD, scan, A->prm.precision,
                                  &A->ref);

@@ -171,16 +171,23 @@ cudaError_t launch_shift_points(const RefDev* ref_dev, const double* scan4, cons
 // convertTo(CV_16U) of num (or num / den).
 cudaError_t launch_to_u16(const float* num, const float* den, long long n, unsigned short* out, cudaStream_t s);
 
-// Phase correlation kernels (fa_phase.cu), each over a batch of frames.
-cudaError_t launch_phase_window(const void* const* vols, int in_kind, const double* wy, const double* wx, int ny,
+// Phase correlation kernels (fa_phase.cu), each over a batch of frames. A batch holds at most
+// kCorrFrames frames, so that its frames' pointers (device memory) travel as a kernel argument:
+// copying them to the device first put a copy and its gap, about 4 us, before every batch.
+constexpr int kCorrFrames = 64;
+struct FramePtrs {
+  const void* p[kCorrFrames];
+};
+cudaError_t launch_phase_window(const FramePtrs& vols, int in_kind, const double* wy, const double* wx, int ny,
                                 int nx, long long n_el, int batch, double* out, cudaStream_t s);
 cudaError_t launch_phase_normalise(double2* spec, const double2* ref_conj, long long n, int batch, cudaStream_t s);
 cudaError_t launch_phase_argmax(const double* surf, long long n, int batch, double* block_val, long long* block_idx,
                                 int blocks_per_frame, long long* out_idx, cudaStream_t s);
 cudaError_t launch_phase_conj(const double2* in, double2* out, long long n, cudaStream_t s);
-// Second argmax stage alone: the first maximum of nb (value, index) pairs per frame.
+// Second argmax stage alone: the first maximum of nb (value, index) pairs per frame. out_idx may be
+// page-locked host memory. `overlap`: see launch_plane_yz.
 cudaError_t launch_phase_argmax_final(const double* block_val, const long long* block_idx, int nb, int batch,
-                                      long long* out_idx, cudaStream_t s);
+                                      long long* out_idx, cudaStream_t s, bool overlap = false);
 
 // Phase correlation as three fused passes over kx planes (fa_plane_corr.cu), for power-of-two
 // volumes with nz <= 16, 8 <= ny <= 2048, 16 <= nx <= 4096 and nz * ny <= 8192 (plane_dims is false
@@ -208,34 +215,38 @@ void plane_twiddles(const PlaneDims& d, std::vector<double2>* tw_x, std::vector<
 // CTAs (argmax partials) per frame of the last pass.
 int plane_blocks_per_frame(const PlaneDims& d);
 // Frame slots the first pass may fill while it reads the frames: frame i's value + 1 (the slot
-// conversion, stored as `kind`: raw uint16 saturated, FP16 or FP32) at ptrs[i] + z * plane +
+// conversion, stored as `kind`: raw uint16 saturated, FP16 or FP32) at p[i] + z * plane +
 // y * pitch + x (16-byte aligned rows).
 struct SlotOut {
-  const void* const* ptrs;  // device array, one interior pointer per frame of the batch (writable slots)
-  int kind;           // FrameKind
+  void* p[kCorrFrames];  // one interior pointer per frame of the batch
+  int kind;              // FrameKind
   int pitch;
   long long plane;
 };
 // Window + real DFT along x of each frame (dense FP32 or uint16, in_kind an fa_dtype) into spec
 // (batch * n_complex); with `slot` (optional) also the frames' slots.
-cudaError_t launch_plane_rows_fwd(const PlaneDims& d, const void* const* vols, int in_kind, int batch,
+cudaError_t launch_plane_rows_fwd(const PlaneDims& d, const FramePtrs& vols, int in_kind, int batch,
                                   const double* wy, const double* wx, const double2* tw_x, double2* spec,
                                   cudaStream_t s, const SlotOut* slot = nullptr);
 // Per plane: forward DFT over (z, y), then either out = conj (reference) or, in place,
-// out = inverse DFT of the normalised cross-power spectrum with ref_conj.
+// out = inverse DFT of the normalised cross-power spectrum with ref_conj. With `overlap` each pass
+// stages its twiddles while the pass before it in the stream drains (that pass has to be one of
+// these); for calls that have the device to themselves.
 cudaError_t launch_plane_yz(const PlaneDims& d, const double2* in, double2* out, const double2* ref_conj,
-                            const double2* tw_y, int batch, bool reference, cudaStream_t s);
+                            const double2* tw_y, int batch, bool reference, cudaStream_t s, bool overlap = false);
 // The same for split dimensions (d.split), in place in spec: forward DFT of every y line, then per
 // z column the forward z DFT and either conj (reference: written to ref_conj instead) or the
 // normalised cross-power with ref_conj and the inverse z DFT, then the inverse DFT of every y line
 // (not for the reference).
 cudaError_t launch_plane_yz_split(const PlaneDims& d, double2* spec, double2* ref_conj, const double2* tw_y,
-                                  const double2* tw_z, int batch, bool reference, cudaStream_t s);
+                                  const double2* tw_z, int batch, bool reference, cudaStream_t s,
+                                  bool overlap = false);
 // One frame's half-spectrum from planes spec[kx][z][y] to cuFFT's order [z][y][kx].
 cudaError_t launch_plane_to_rows(const PlaneDims& d, const double2* in, double2* out, cudaStream_t s);
 // Inverse real DFT along x and the per-CTA first maximum (bval / bidx: batch * plane_blocks_per_frame);
 // surface (batch * n_el doubles) receives the real surface when not null.
 cudaError_t launch_plane_rows_inv_argmax(const PlaneDims& d, const double2* spec, int batch, const double2* tw_x,
-                                         double* bval, long long* bidx, double* surface, cudaStream_t s);
+                                         double* bval, long long* bidx, double* surface, cudaStream_t s,
+                                         bool overlap = false);
 
 }  // namespace fa

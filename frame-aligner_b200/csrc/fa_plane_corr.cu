@@ -304,17 +304,18 @@ __host__ __device__ inline size_t rows_smem_bytes(const PlaneDims& d) {
 
 // SLOT: -1, or the FrameKind of the slots written from the same loads (SlotOut).
 template <bool U16, int SLOT>
-__global__ void __launch_bounds__(kRowThreads) plane_rows_fwd_kernel(const void* const* __restrict__ vols,
+__global__ void __launch_bounds__(kRowThreads) plane_rows_fwd_kernel(const __grid_constant__ FramePtrs vols,
                                                                      const double* __restrict__ wy,
                                                                      const double* __restrict__ wx,
                                                                      const double2* __restrict__ tw_x, PlaneDims d,
-                                                                     double2* __restrict__ spec, SlotOut slot) {
+                                                                     double2* __restrict__ spec, const __grid_constant__ SlotOut slot) {
+  cudaTriggerProgrammaticLaunchCompletion();
   extern __shared__ double2 sm[];
   const int M = d.nx >> 1, S = M + 1, G = 1 << d.log2G;
   double2* tws = sm + G * S;
   const int r0 = blockIdx.x << d.log2G;
-  const void* vol = vols[blockIdx.y];
-  void* const slot_base = SLOT >= 0 ? const_cast<void*>(slot.ptrs[blockIdx.y]) : nullptr;
+  const void* vol = vols.p[blockIdx.y];
+  void* const slot_base = SLOT >= 0 ? slot.p[blockIdx.y] : nullptr;
   // the twiddles (published by the first stage's closing barrier; the first stage needs none)
   stage16<4>(
       d.n_twx, [&](int i) { return reinterpret_cast<const uint4*>(tw_x) + i; },
@@ -394,6 +395,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2) plane_yz_kernel(const double
                                                                     const double2* __restrict__ ref_conj,
                                                                     const double2* __restrict__ tw_y, PlaneDims d,
                                                                     long long n_planes) {
+  cudaTriggerProgrammaticLaunchCompletion();
   extern __shared__ double2 sm[];
   const int ny = d.ny, S = ny + 1;
   const int plane = NZ * ny;
@@ -406,6 +408,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2) plane_yz_kernel(const double
   stage16<4>(
       d.n_twy, [&](int i) { return reinterpret_cast<const uint4*>(tw_y) + i; },
       [&](int i) { return reinterpret_cast<uint4*>(tws) + i; });
+  cudaGridDependencySynchronize();
   // the first stage reads the planes (in may be out: each CTA reads its own planes before it
   // writes them)
   auto first = [&](int l, int i) -> double2 { return src[l * ny + i]; };
@@ -472,6 +475,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 2)
     plane_yz_pair_kernel(const double2* in, double2* out, const double2* __restrict__ ref_conj,
                          const double2* __restrict__ tw_y, PlaneDims d) {
   namespace cg = cooperative_groups;
+  cudaTriggerProgrammaticLaunchCompletion();
   extern __shared__ double2 sm[];
   constexpr int H = NZ / 2;  // z lines per CTA
   cg::cluster_group cluster = cg::this_cluster();
@@ -483,6 +487,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 2)
   stage16<4>(
       d.n_twy, [&](int i) { return reinterpret_cast<const uint4*>(tw_y) + i; },
       [&](int i) { return reinterpret_cast<uint4*>(tws) + i; });
+  cudaGridDependencySynchronize();
   // this CTA's lines (in may be out: each CTA reads its own lines before it writes them)
   const double2* src = in + p * plane + (long long)r * H * ny;
   auto first = [&](int l, int i) -> double2 { return src[l * ny + i]; };
@@ -550,6 +555,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 2)
 template <bool INV>
 __global__ void __launch_bounds__(kPlaneThreads, 2) plane_y_kernel(double2* spec, const double2* __restrict__ tw_y,
                                                                    PlaneDims d, long long n_lines) {
+  cudaTriggerProgrammaticLaunchCompletion();
   extern __shared__ double2 sm[];
   const int ny = d.ny, S = ny + 1;
   const long long l0 = (long long)blockIdx.x * d.LY;
@@ -559,6 +565,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2) plane_y_kernel(double2* spec
   stage16<4>(
       d.n_twy, [&](int i) { return reinterpret_cast<const uint4*>(tw_y) + i; },
       [&](int i) { return reinterpret_cast<uint4*>(tws) + i; });
+  cudaGridDependencySynchronize();
   auto first = [&](int l, int i) -> double2 { return base[(long long)l * ny + i]; };
   auto last = [&](int l, int i, double2 v) { base[(long long)l * ny + i] = v; };
   fft_rows<INV, kPlaneEPT, kPlaneThreads, false, false>(sm, nl, d.log2ny, tws, first, last);
@@ -573,6 +580,7 @@ template <bool REF>
 __global__ void __launch_bounds__(kPlaneThreads, 2) plane_z_kernel(double2* spec, double2* ref_out,
                                                                    const double2* __restrict__ ref_conj,
                                                                    const double2* __restrict__ tw_z, PlaneDims d) {
+  cudaTriggerProgrammaticLaunchCompletion();
   extern __shared__ double2 sm[];
   const int nz = d.nz, ny = d.ny, S = nz + 1, YB = 1 << d.log2YB;
   const int yblocks = ny >> d.log2YB;
@@ -585,6 +593,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 2) plane_z_kernel(double2* spec
   stage16<4>(
       d.n_twz, [&](int i) { return reinterpret_cast<const uint4*>(tw_z) + i; },
       [&](int i) { return reinterpret_cast<uint4*>(tws) + i; });
+  cudaGridDependencySynchronize();
   for (int idx = threadIdx.x; idx < E; idx += blockDim.x) {
     const int z = idx >> d.log2YB, yy = idx & (YB - 1);
     sm[yy * S + swz(z)] = col[(long long)z * ny + yy];
@@ -638,6 +647,7 @@ __global__ void __launch_bounds__(kRowThreads) plane_rows_inv_argmax_kernel(cons
                                                                             PlaneDims d, double* __restrict__ bval,
                                                                             long long* __restrict__ bidx,
                                                                             double* __restrict__ surface) {
+  cudaTriggerProgrammaticLaunchCompletion();
   extern __shared__ double2 sm[];
   const int M = d.nx >> 1, S = M + 1, G = 1 << d.log2G, H = M >> 1;
   double2* tws = sm + G * S;
@@ -646,6 +656,7 @@ __global__ void __launch_bounds__(kRowThreads) plane_rows_inv_argmax_kernel(cons
   stage16<4>(
       d.n_twx, [&](int i) { return reinterpret_cast<const uint4*>(tw_x) + i; },
       [&](int i) { return reinterpret_cast<uint4*>(tws) + i; });
+  cudaGridDependencySynchronize();
   // Bins k and M - k of each row, folded as they arrive (the fold's twiddles from global memory, so
   // that it need not wait for the staged table): four pairs per thread in flight.
   {
@@ -811,7 +822,7 @@ int plane_blocks_per_frame(const PlaneDims& d) { return d.rows >> d.log2G; }
 
 namespace {
 template <bool U16, int SLOT>
-cudaError_t launch_rows_fwd(const PlaneDims& d, const void* const* vols, int batch, const double* wy,
+cudaError_t launch_rows_fwd(const PlaneDims& d, const FramePtrs& vols, int batch, const double* wy,
                             const double* wx, const double2* tw_x, double2* spec, cudaStream_t s, const SlotOut& so) {
   const size_t smem = rows_smem_bytes(d);
   cudaError_t e = allow_smem(plane_rows_fwd_kernel<U16, SLOT>, smem);
@@ -822,10 +833,10 @@ cudaError_t launch_rows_fwd(const PlaneDims& d, const void* const* vols, int bat
 }
 }  // namespace
 
-cudaError_t launch_plane_rows_fwd(const PlaneDims& d, const void* const* vols, int in_kind, int batch,
+cudaError_t launch_plane_rows_fwd(const PlaneDims& d, const FramePtrs& vols, int in_kind, int batch,
                                   const double* wy, const double* wx, const double2* tw_x, double2* spec,
                                   cudaStream_t s, const SlotOut* slot) {
-  const SlotOut so = slot ? *slot : SlotOut{nullptr, -1, 0, 0};
+  const SlotOut so = slot ? *slot : SlotOut{{}, -1, 0, 0};
   const int k = slot ? slot->kind : -1;
   if (in_kind == FA_U16) {
     if (k == kFrameRawU16) return launch_rows_fwd<true, kFrameRawU16>(d, vols, batch, wy, wx, tw_x, spec, s, so);
@@ -841,14 +852,14 @@ cudaError_t launch_plane_rows_fwd(const PlaneDims& d, const void* const* vols, i
 namespace {
 template <int NZ, bool REF>
 cudaError_t launch_yz(const PlaneDims& d, const double2* in, double2* out, const double2* ref_conj,
-                      const double2* tw_y, long long n_planes, cudaStream_t s) {
+                      const double2* tw_y, long long n_planes, cudaStream_t s, bool overlap) {
   if constexpr (NZ >= 4) {
     if ((long long)NZ * d.ny == 2LL * kPairThreads * kPairEPT) {  // one plane per pair of CTAs
       const size_t smem = ((size_t)(NZ / 2) * (d.ny + 1) + d.ny) * sizeof(double2);
       cudaError_t e = allow_smem(plane_yz_pair_kernel<NZ, REF>, smem);
       if (e != cudaSuccess) return e;
-      plane_yz_pair_kernel<NZ, REF><<<(unsigned)(2 * n_planes), kPairThreads, smem, s>>>(in, out, ref_conj, tw_y, d);
-      return cudaGetLastError();
+      return launch_overlapped(plane_yz_pair_kernel<NZ, REF>, dim3((unsigned)(2 * n_planes)), dim3(kPairThreads), smem, s,
+                               overlap, in, out, ref_conj, tw_y, d);
     }
   }
   const int pp = planes_of_cta(NZ, d.ny);
@@ -857,33 +868,34 @@ cudaError_t launch_yz(const PlaneDims& d, const double2* in, double2* out, const
   cudaError_t e = allow_smem(plane_yz_kernel<NZ, REF>, smem);
   if (e != cudaSuccess) return e;
   const long long grid = (n_planes + pp - 1) / pp;
-  plane_yz_kernel<NZ, REF><<<(unsigned)grid, kPlaneThreads, smem, s>>>(in, out, ref_conj, tw_y, d, n_planes);
-  return cudaGetLastError();
+  return launch_overlapped(plane_yz_kernel<NZ, REF>, dim3((unsigned)grid), dim3(kPlaneThreads), smem, s, overlap, in, out,
+                           ref_conj, tw_y, d, n_planes);
 }
 
 template <bool REF>
 cudaError_t launch_yz_nz(const PlaneDims& d, const double2* in, double2* out, const double2* ref_conj,
-                         const double2* tw_y, long long n_planes, cudaStream_t s) {
+                         const double2* tw_y, long long n_planes, cudaStream_t s, bool overlap) {
   switch (d.nz) {
-    case 1: return launch_yz<1, REF>(d, in, out, ref_conj, tw_y, n_planes, s);
-    case 2: return launch_yz<2, REF>(d, in, out, ref_conj, tw_y, n_planes, s);
-    case 4: return launch_yz<4, REF>(d, in, out, ref_conj, tw_y, n_planes, s);
-    case 8: return launch_yz<8, REF>(d, in, out, ref_conj, tw_y, n_planes, s);
-    case 16: return launch_yz<16, REF>(d, in, out, ref_conj, tw_y, n_planes, s);
+    case 1: return launch_yz<1, REF>(d, in, out, ref_conj, tw_y, n_planes, s, overlap);
+    case 2: return launch_yz<2, REF>(d, in, out, ref_conj, tw_y, n_planes, s, overlap);
+    case 4: return launch_yz<4, REF>(d, in, out, ref_conj, tw_y, n_planes, s, overlap);
+    case 8: return launch_yz<8, REF>(d, in, out, ref_conj, tw_y, n_planes, s, overlap);
+    case 16: return launch_yz<16, REF>(d, in, out, ref_conj, tw_y, n_planes, s, overlap);
     default: return cudaErrorInvalidValue;
   }
 }
 }  // namespace
 
 cudaError_t launch_plane_yz(const PlaneDims& d, const double2* in, double2* out, const double2* ref_conj,
-                            const double2* tw_y, int batch, bool reference, cudaStream_t s) {
+                            const double2* tw_y, int batch, bool reference, cudaStream_t s, bool overlap) {
   const long long n_planes = (long long)batch * ((d.nx >> 1) + 1);
-  return reference ? launch_yz_nz<true>(d, in, out, nullptr, tw_y, n_planes, s)
-                   : launch_yz_nz<false>(d, in, out, ref_conj, tw_y, n_planes, s);
+  return reference ? launch_yz_nz<true>(d, in, out, nullptr, tw_y, n_planes, s, overlap)
+                   : launch_yz_nz<false>(d, in, out, ref_conj, tw_y, n_planes, s, overlap);
 }
 
 cudaError_t launch_plane_yz_split(const PlaneDims& d, double2* spec, double2* ref_conj, const double2* tw_y,
-                                  const double2* tw_z, int batch, bool reference, cudaStream_t s) {
+                                  const double2* tw_z, int batch, bool reference, cudaStream_t s,
+                                  bool overlap) {
   if (!d.split) return cudaErrorInvalidValue;
   const long long n_planes = (long long)batch * ((d.nx >> 1) + 1);
   const long long n_lines = n_planes * d.nz;
@@ -896,14 +908,14 @@ cudaError_t launch_plane_yz_split(const PlaneDims& d, double2* spec, double2* re
   if (e == cudaSuccess) e = allow_smem(plane_z_kernel<false>, smem_z);
   if (e == cudaSuccess) e = allow_smem(plane_z_kernel<true>, smem_z);
   if (e != cudaSuccess) return e;
-  plane_y_kernel<false><<<(unsigned)grid_y, kPlaneThreads, smem_y, s>>>(spec, tw_y, d, n_lines);
-  if (reference) {
-    plane_z_kernel<true><<<(unsigned)grid_z, kPlaneThreads, smem_z, s>>>(spec, ref_conj, nullptr, tw_z, d);
-    return cudaGetLastError();
-  }
-  plane_z_kernel<false><<<(unsigned)grid_z, kPlaneThreads, smem_z, s>>>(spec, nullptr, ref_conj, tw_z, d);
-  plane_y_kernel<true><<<(unsigned)grid_y, kPlaneThreads, smem_y, s>>>(spec, tw_y, d, n_lines);
-  return cudaGetLastError();
+  const dim3 gy((unsigned)grid_y), gz((unsigned)grid_z), threads(kPlaneThreads);
+  e = launch_overlapped(plane_y_kernel<false>, gy, threads, smem_y, s, overlap, spec, tw_y, d, n_lines);
+  if (e != cudaSuccess) return e;
+  if (reference)
+    return launch_overlapped(plane_z_kernel<true>, gz, threads, smem_z, s, overlap, spec, ref_conj, nullptr, tw_z, d);
+  e = launch_overlapped(plane_z_kernel<false>, gz, threads, smem_z, s, overlap, spec, nullptr, ref_conj, tw_z, d);
+  if (e != cudaSuccess) return e;
+  return launch_overlapped(plane_y_kernel<true>, gy, threads, smem_y, s, overlap, spec, tw_y, d, n_lines);
 }
 
 cudaError_t launch_plane_to_rows(const PlaneDims& d, const double2* in, double2* out, cudaStream_t s) {
@@ -913,13 +925,13 @@ cudaError_t launch_plane_to_rows(const PlaneDims& d, const double2* in, double2*
 }
 
 cudaError_t launch_plane_rows_inv_argmax(const PlaneDims& d, const double2* spec, int batch, const double2* tw_x,
-                                         double* bval, long long* bidx, double* surface, cudaStream_t s) {
+                                         double* bval, long long* bidx, double* surface, cudaStream_t s,
+                                         bool overlap) {
   const size_t smem = rows_smem_bytes(d);
   cudaError_t e = allow_smem(plane_rows_inv_argmax_kernel, smem);
   if (e != cudaSuccess) return e;
-  plane_rows_inv_argmax_kernel<<<dim3(d.rows >> d.log2G, batch), kRowThreads, smem, s>>>(spec, tw_x, d, bval, bidx,
-                                                                                         surface);
-  return cudaGetLastError();
+  return launch_overlapped(plane_rows_inv_argmax_kernel, dim3(d.rows >> d.log2G, batch), dim3(kRowThreads), smem, s,
+                           overlap, spec, tw_x, d, bval, bidx, surface);
 }
 
 }  // namespace fa

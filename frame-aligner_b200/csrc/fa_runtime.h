@@ -132,17 +132,15 @@ struct fa_correlator {
   double2* ref_conj = nullptr;          // n_complex (planes [kx][z][y] when `planes`, else cuFFT's order)
   double2* ref_conj_rows = nullptr;     // cuFFT's order, made when a plane-path correlator falls back
   float* vol = nullptr;                 // one host-uploaded volume
-  const void** d_ptrs = nullptr;        // device array of input pointers, then (from ptr_cap) slot pointers
-  const void** h_ptrs = nullptr;        // pinned staging of the same
-  int ptr_cap = 0;
+  int idx_cap = 0;
   double* bval = nullptr;
   long long* bidx = nullptr;
-  long long* d_idx = nullptr;           // one peak index per frame (ptr_cap)
-  long long* h_idx = nullptr;
+  long long* d_idx = nullptr;           // one peak index per frame (idx_cap)
+  long long* h_idx = nullptr;           // page-locked, the peak index of a single-frame call
   int n_blocks = 0;                     // argmax blocks per frame (cuFFT path)
   std::mutex mu;
   std::vector<fa_rt::Alloc> allocs;
-  std::vector<fa_rt::Alloc> ptr_allocs;
+  std::vector<fa_rt::Alloc> idx_allocs;
 };
 
 namespace fa_rt {
@@ -254,18 +252,20 @@ int slot_kind_for(const fa_aligner* A, fa_dtype dtype);
 // The correlator's D2Z / Z2D plans for a batch size (made and cached on first use).
 fa_status correlator_plans(fa_correlator* C, int batch, cufftHandle* fwd, cufftHandle* inv);
 // Window, forward DFT, normalisation, inverse DFT and argmax for n device volumes; peak indices to
-// C->d_idx[first .. first + n). surface (n * n_el doubles, optional) receives the correlation
+// peaks[0 .. n), by default C->d_idx[first .. first + n). surface (n * n_el doubles, optional) receives the correlation
 // surfaces; planes selects the fused kx-plane passes (when C->planes) or cuFFT. Calls with
-// first > 0 use pointer and result slots reserved before (correlator_reserve(C, first + n)), so
-// that consecutive calls queue on the stream without waiting for one another.
+// first > 0 use peak slots reserved before (correlator_reserve(C, first + n)), so that consecutive
+// calls queue on the stream without waiting for one another.
 // With `slots` (n interior pointers of frame slots of `slot_kind` with the given pitch and plane),
 // the plane path also writes each frame + 1 into its slot as it reads it (*slots_written = true);
-// on the cuFFT path it does not, and the caller converts the frames itself.
+// on the cuFFT path it does not, and the caller converts the frames itself. peaks may be page-locked
+// host memory. alone: nothing else uses the device, so the passes may overlap their launches.
 fa_status correlator_enqueue(fa_correlator* C, const void* const* vols, int in_kind, int n,
                              double* surface = nullptr, bool planes = true, int first = 0,
                              void* const* slots = nullptr, int slot_kind = 0, int slot_pitch = 0,
-                             long long slot_plane = 0, bool* slots_written = nullptr);
-// Pointer staging and peak slots for n volumes (grows with a stream synchronisation).
+                             long long slot_plane = 0, bool* slots_written = nullptr,
+                             long long* peaks = nullptr, bool alone = false);
+// Peak slots for n volumes (grows with a stream synchronisation).
 fa_status correlator_reserve(fa_correlator* C, int n);
 // Peak index -> signed integer shift (x, y, z).
 void unravel_shift(const fa_correlator* C, long long idx, double* shift);

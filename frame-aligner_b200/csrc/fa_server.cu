@@ -543,8 +543,7 @@ fa_status intake(fa_server* S, SrvAcq* q, std::vector<SrvSlot*>& batch) {
       cin[i] = src;
     }
   }
-  FA_TRY(correlator_enqueue(A->corr, cin.data(), cin_kind, m));
-  FA_CU(cudaMemcpyAsync(q->h_idx, A->corr->d_idx, (size_t)m * sizeof(long long), cudaMemcpyDeviceToHost, s));
+  FA_TRY(correlator_enqueue(A->corr, cin.data(), cin_kind, m, nullptr, true, 0, nullptr, 0, 0, 0, nullptr, q->h_idx));
   FA_CU(cudaEventRecord(q->corr_ev, s));
   FA_CU(cudaLaunchHostFunc(s, wake_worker, S));
   q->corr_busy = true;
