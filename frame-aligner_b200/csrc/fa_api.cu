@@ -1837,6 +1837,19 @@ fa_status aligner_grow(fa_aligner* A, int n, int kind, size_t staging_need) {
   return FA_OK;
 }
 
+// Frames of a solve group (and of an upload) from host frames of raw_bytes each. While frames upload, the
+// solves of those before them have the device to themselves, so a group need not fill it and a long
+// upload is better cut finer: groups are the frames of a 32 MiB upload, 2 to 8 of them. Groups of 8 / 4 / 2,
+// ms a call: 50 frames of 16 x 512 x 512 (8.4 MB) 10.07 / 9.72 / 9.38, 16 of them 3.55 / 3.22 / 3.21; 8 of
+// 32 x 512 x 512 (16.8 MB) 4.97 / 4.91 / 4.32; 4 of 64 x 1024 x 1024 (134 MB) 43.4 / 38.3 / 38.5; 24 of 8 x 512 x
+// 512 (4.2 MB) 2.49 / 2.42 / 2.44; 32 of 4 x 512 x 512 (2.1 MB) 1.87 / 1.89 / 2.00; 40 of 2 x 512 x 512 1.51 / 1.56 /
+// 1.79. (Half that upload, 2 frames of 8.4 MB, would make an aligner's first call instantiate 25 graphs for
+// 50 frames.) Frames in device memory: 7.19 ms in groups of 8, 7.34 in groups of 4.
+int host_group_frames(size_t raw_bytes) {
+  constexpr size_t kUpload = (size_t)32 << 20;
+  return (int)std::min<size_t>(8, std::max<size_t>(2, kUpload / std::max<size_t>(raw_bytes, 1)));
+}
+
 // Solve groups of one call, as frame boundaries {0, ..., n}: groups of `chunk` frames (a last
 // remainder under chunk / 2 joins the group before it). Every group's solve is queued on its own
 // stream behind its own peaks, so the solves of the first groups run while the later groups upload
@@ -1878,14 +1891,14 @@ fa_status aligner_run(fa_aligner* A, const void* const* frames, fa_dtype dtype, 
     FA_CU(cudaEventCreate(&A->ev_corr));
   }
   FA_CU(cudaEventRecord(A->ev0, s));
-  // Host frames upload on a copy stream in chunks of kChunk; each chunk's conversion and phase
+  // Host frames upload on a copy stream in chunks of a solve group; each chunk's conversion and phase
   // correlation wait only for its own uploads, so they overlap the uploads of the chunks after it.
-  constexpr int kChunk = 8;
-  const int chunk = device_src ? n : kChunk;
+  const int group = device_src ? 8 : host_group_frames(raw_bytes);
+  const int chunk = device_src ? n : group;
   if (!device_src) {
     if (!A->copy_stream) FA_CU(cudaStreamCreateWithFlags(&A->copy_stream, cudaStreamNonBlocking));
     // one event per upload chunk: chunks never straddle a solve group, so a group adds at most one
-    while ((int)A->copy_ev.size() < (n + chunk - 1) / chunk + (int)solve_groups(n, kChunk, raw_bytes).size()) {
+    while ((int)A->copy_ev.size() < (n + chunk - 1) / chunk + (int)solve_groups(n, group, raw_bytes).size()) {
       cudaEvent_t e;
       FA_CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       A->copy_ev.push_back(e);
@@ -1904,7 +1917,7 @@ fa_status aligner_run(fa_aligner* A, const void* const* frames, fa_dtype dtype, 
     }
   } drain{device_src ? nullptr : A->copy_stream};
   FA_TRY(correlator_reserve(A->corr, n));
-  const std::vector<int> gb = solve_groups(n, kChunk, device_src ? 0 : raw_bytes);  // group g: frames [gb[g], gb[g + 1])
+  const std::vector<int> gb = solve_groups(n, group, device_src ? 0 : raw_bytes);  // group g: frames [gb[g], gb[g + 1])
   const int n_groups = (int)gb.size() - 1;
   while ((int)A->batch_cache.size() < n_groups) A->batch_cache.emplace_back();
   while ((int)A->group_ev.size() < n_groups) {
