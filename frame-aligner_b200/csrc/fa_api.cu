@@ -301,6 +301,7 @@ extern "C" fa_status fa_create(const fa_config* cfg, fa_context** out) {
   FA_CU(cudaSetDevice(dev));
   size_t free_b = 0, total_b = 0;
   FA_CU(cudaMemGetInfo(&free_b, &total_b));
+  fa::smem_new_context(dev);
   fa_context* c = new fa_context;
   c->device = dev;
   c->budget = (cfg && cfg->memory_budget) ? cfg->memory_budget : (size_t)(0.9 * (double)free_b);

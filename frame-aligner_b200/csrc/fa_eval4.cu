@@ -997,20 +997,14 @@ inline cudaError_t dispatch_mb(int mb, Fn&& f) {
 
 bool eval4_few_only(long long most_items) { return most_items <= kCtaTiles; }
 
-template <typename K>
-cudaError_t allow_smem(K kernel, size_t bytes) {
-  return bytes <= 48 * 1024 ? cudaSuccess
-                            : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 cudaError_t launch_eval4(const Job* jobs_dev, int n_jobs, int max_tiles, int n_dim, int frame_kind, bool ref_bf16,
                          int mb, cudaStream_t s) {
   if ((long long)max_tiles * n_jobs <= kCtaTiles)
     return dispatch_cfg(n_dim, frame_kind, ref_bf16, [&](auto c) {
       using C = decltype(c);
       constexpr size_t smem = sizeof(CtaTileSmem<C::nd, typename C::R>);
-      auto kernel = eval4_cta_kernel<C::nd, typename C::F, typename C::R>;
-      const cudaError_t e = allow_smem(kernel, smem);
+      constexpr auto kernel = eval4_cta_kernel<C::nd, typename C::F, typename C::R>;
+      const cudaError_t e = allow_smem<kernel>(smem, smem);
       if (e != cudaSuccess) return e;
       return launch_overlapped(kernel, dim3(max_tiles, n_jobs), dim3(kEvalThreads), smem, s, true, jobs_dev);
     });
@@ -1048,8 +1042,8 @@ cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const in
     if (few) {
       const long long ctas = std::min<long long>(std::min<long long>(most_items, kCtaTiles), kCtaGrid);
       constexpr size_t smem = sizeof(CtaTileSmem<C::nd, typename C::R>);
-      auto kernel = eval4_active_cta_kernel<C::nd, typename C::F, typename C::R>;
-      cudaError_t e = allow_smem(kernel, smem);
+      constexpr auto kernel = eval4_active_cta_kernel<C::nd, typename C::F, typename C::R>;
+      cudaError_t e = allow_smem<kernel>(smem, smem);
       if (e != cudaSuccess) return e;
       e = launch_overlapped(kernel, dim3((unsigned)std::max<long long>(1, ctas)), dim3(kEvalThreads), smem, s, overlap && !many,
                             jobs_dev, active, n_active, tile_prefix, (int)kCtaTiles);

@@ -15,6 +15,17 @@
 
 namespace fa {
 
+namespace {
+std::atomic<unsigned> g_smem_epoch[kSmemDevices];
+}
+unsigned smem_epoch(int device) {
+  return device >= 0 && device < kSmemDevices ? g_smem_epoch[device].load(std::memory_order_acquire) : 0u;
+}
+void smem_new_context(int device) {
+  if (device < 0 || device >= kSmemDevices) return;
+  if (++g_smem_epoch[device] == 0u) ++g_smem_epoch[device];
+}
+
 // ------------------------------------------------------------------ Sobel3d ----------------------
 
 // One separable pass (Sobel3d.cpp:8-58) at a position of an axis from its neighbours: interior
@@ -803,6 +814,8 @@ __global__ void __launch_bounds__(256) warp_kernel(const RefDev* __restrict__ Rp
   }
 }
 
+constexpr size_t kMostSmem = 227 * 1024;  // all a CTA can have: 4842 control points
+
 cudaError_t launch_warp(const RefDev* ref_dev, const RefDev& R, const void* frame, long long fplane, int fpitch,
                         int frame_kind, const float4* dparams, float invalid_value, float* out, cudaStream_t s) {
   int blocks = (R.n_rows + 7) / 8;
@@ -810,11 +823,9 @@ cudaError_t launch_warp(const RefDev* ref_dev, const RefDev& R, const void* fram
   const size_t smem = (size_t)R.nD * kDParamF4 * sizeof(float4);
   return dispatch_cfg(R.n_dim, frame_kind, false, [&](auto c) {
     using C = decltype(c);
-    auto kern = warp_kernel<C::nd, typename C::F>;
-    if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
+    constexpr auto kern = warp_kernel<C::nd, typename C::F>;
+    const cudaError_t e = allow_smem<kern>(smem, kMostSmem);
+    if (e != cudaSuccess) return e;
     kern<<<blocks, 256, smem, s>>>(ref_dev, static_cast<const typename C::F*>(frame), fplane, fpitch, dparams,
                                    invalid_value, out);
     return cudaGetLastError();

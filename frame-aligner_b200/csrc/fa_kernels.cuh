@@ -1,6 +1,7 @@
 // fa_kernels.cuh -- kernel launch declarations (implemented in fa_kernels.cu, fa_solve.cu).
 #pragma once
 
+#include <atomic>
 #include <vector>
 
 #include "fa_internal.h"
@@ -34,6 +35,31 @@ inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block
   cfg.attrs = at;
   cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Lets Kernel take up to `most` bytes of dynamic shared memory, where a launch wants `bytes` of them (more
+// than 48 KB of shared memory have to be allowed, per kernel and device). The permission is the whole
+// process's: `most` is the kernel's constant, never a call's own size, so that no thread takes away
+// what another is about to launch with; and it is asked for once, because the call takes a lock that
+// the launches of all threads need (eight threads solving FP32 512 x 512 planes, one frame each: 17.5k solves/s
+// with the call in every launch, 56k without). smem_epoch changes with every context created on the
+// device, so a device that was reset is asked again.
+constexpr int kSmemDevices = 64;
+unsigned smem_epoch(int device);      // 0: no context yet, or a device beyond the table
+void smem_new_context(int device);
+template <auto Kernel>
+inline cudaError_t allow_smem(size_t bytes, size_t most, size_t free_bytes = 48 * 1024) {
+  static std::atomic<unsigned> allowed[kSmemDevices];
+  if (bytes > most) return cudaErrorInvalidValue;
+  if (bytes <= free_bytes) return cudaSuccess;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned epoch = smem_epoch(dev);
+  if (epoch != 0 && allowed[dev].load(std::memory_order_acquire) == epoch) return cudaSuccess;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  if (e == cudaSuccess && epoch != 0) allowed[dev].store(epoch, std::memory_order_release);
+  return e;
 }
 
 // Exact float Sobel3d (Sobel3d.cpp:60-85) of an FP32 volume; with q16 also the BF16 groups of

@@ -728,11 +728,10 @@ __global__ void plane_to_rows_kernel(const double2* __restrict__ in, double2* __
   }
 }
 
-template <typename K>
-cudaError_t allow_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
+// The most shared memory any pass takes, whatever the dimensions: lines of kPlanePoints points with a point
+// of padding per line and the twiddle slots of the longest line, 2048 (rows of 4096 voxels: 2049 points
+// and 4096 slots).
+constexpr size_t kPlaneSmem = (kPlanePoints + 2 + 2048) * sizeof(double2);
 
 int ilog2(long long v) {
   int l = 0;
@@ -825,7 +824,7 @@ template <bool U16, int SLOT>
 cudaError_t launch_rows_fwd(const PlaneDims& d, const FramePtrs& vols, int batch, const double* wy,
                             const double* wx, const double2* tw_x, double2* spec, cudaStream_t s, const SlotOut& so) {
   const size_t smem = rows_smem_bytes(d);
-  cudaError_t e = allow_smem(plane_rows_fwd_kernel<U16, SLOT>, smem);
+  cudaError_t e = allow_smem<plane_rows_fwd_kernel<U16, SLOT>>(smem, kPlaneSmem);
   if (e != cudaSuccess) return e;
   plane_rows_fwd_kernel<U16, SLOT><<<dim3(d.rows >> d.log2G, batch), kRowThreads, smem, s>>>(vols, wy, wx, tw_x, d,
                                                                                              spec, so);
@@ -856,7 +855,7 @@ cudaError_t launch_yz(const PlaneDims& d, const double2* in, double2* out, const
   if constexpr (NZ >= 4) {
     if ((long long)NZ * d.ny == 2LL * kPairThreads * kPairEPT) {  // one plane per pair of CTAs
       const size_t smem = ((size_t)(NZ / 2) * (d.ny + 1) + d.ny) * sizeof(double2);
-      cudaError_t e = allow_smem(plane_yz_pair_kernel<NZ, REF>, smem);
+      cudaError_t e = allow_smem<plane_yz_pair_kernel<NZ, REF>>(smem, kPlaneSmem);
       if (e != cudaSuccess) return e;
       return launch_overlapped(plane_yz_pair_kernel<NZ, REF>, dim3((unsigned)(2 * n_planes)), dim3(kPairThreads), smem, s,
                                overlap, in, out, ref_conj, tw_y, d);
@@ -865,7 +864,7 @@ cudaError_t launch_yz(const PlaneDims& d, const double2* in, double2* out, const
   const int pp = planes_of_cta(NZ, d.ny);
   if (pp * NZ * d.ny > kPlanePoints) return cudaErrorInvalidValue;
   const size_t smem = ((size_t)pp * NZ * (d.ny + 1) + d.ny) * sizeof(double2);
-  cudaError_t e = allow_smem(plane_yz_kernel<NZ, REF>, smem);
+  cudaError_t e = allow_smem<plane_yz_kernel<NZ, REF>>(smem, kPlaneSmem);
   if (e != cudaSuccess) return e;
   const long long grid = (n_planes + pp - 1) / pp;
   return launch_overlapped(plane_yz_kernel<NZ, REF>, dim3((unsigned)grid), dim3(kPlaneThreads), smem, s, overlap, in, out,
@@ -903,10 +902,10 @@ cudaError_t launch_plane_yz_split(const PlaneDims& d, double2* spec, double2* re
   const size_t smem_z = (((size_t)1 << d.log2YB) * (d.nz + 1) + d.nz) * sizeof(double2);
   const long long grid_y = (n_lines + d.LY - 1) / d.LY;
   const long long grid_z = n_planes * (d.ny >> d.log2YB);
-  cudaError_t e = allow_smem(plane_y_kernel<false>, smem_y);
-  if (e == cudaSuccess) e = allow_smem(plane_y_kernel<true>, smem_y);
-  if (e == cudaSuccess) e = allow_smem(plane_z_kernel<false>, smem_z);
-  if (e == cudaSuccess) e = allow_smem(plane_z_kernel<true>, smem_z);
+  cudaError_t e = allow_smem<plane_y_kernel<false>>(smem_y, kPlaneSmem);
+  if (e == cudaSuccess) e = allow_smem<plane_y_kernel<true>>(smem_y, kPlaneSmem);
+  if (e == cudaSuccess) e = allow_smem<plane_z_kernel<false>>(smem_z, kPlaneSmem);
+  if (e == cudaSuccess) e = allow_smem<plane_z_kernel<true>>(smem_z, kPlaneSmem);
   if (e != cudaSuccess) return e;
   const dim3 gy((unsigned)grid_y), gz((unsigned)grid_z), threads(kPlaneThreads);
   e = launch_overlapped(plane_y_kernel<false>, gy, threads, smem_y, s, overlap, spec, tw_y, d, n_lines);
@@ -928,7 +927,7 @@ cudaError_t launch_plane_rows_inv_argmax(const PlaneDims& d, const double2* spec
                                          double* bval, long long* bidx, double* surface, cudaStream_t s,
                                          bool overlap) {
   const size_t smem = rows_smem_bytes(d);
-  cudaError_t e = allow_smem(plane_rows_inv_argmax_kernel, smem);
+  cudaError_t e = allow_smem<plane_rows_inv_argmax_kernel>(smem, kPlaneSmem);
   if (e != cudaSuccess) return e;
   return launch_overlapped(plane_rows_inv_argmax_kernel, dim3(d.rows >> d.log2G, batch), dim3(kRowThreads), smem, s,
                            overlap, spec, tw_x, d, bval, bidx, surface);

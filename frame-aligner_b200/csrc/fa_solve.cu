@@ -822,10 +822,8 @@ cudaError_t launch_solve_nd(const Job* jobs_dev, int n_jobs, int max_nD, cudaStr
   if (need > kCapBytes)  // every frame of the launch works in global memory
     return launch_overlapped(solve_kernel<ND, false>, dim3(n_jobs), dim3(kSolveThreads), 0, s, overlap, jobs_dev, active,
                              n_active, next, finished, end_of_round);
-  if (need > 40 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(solve_kernel<ND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_smem<solve_kernel<ND, true>>((size_t)need, (size_t)kCapBytes, 40 * 1024);  // (8 KB are static)
+  if (e != cudaSuccess) return e;
   return launch_overlapped(solve_kernel<ND, true>, dim3(n_jobs), dim3(kSolveThreads), (size_t)need, s, overlap, jobs_dev,
                            active, n_active, next, finished, end_of_round);
 }
