@@ -25,6 +25,9 @@ std::atomic<long long> g_launches{0};
 
 fa_status fail(fa_status s, const std::string& msg) {
   g_err = msg;
+  // An error that CUDA has reported here stays the thread's last error, and the check after this thread's
+  // next launch would report it again for a call that is fine.
+  if (s == FA_ERR_CUDA || s == FA_ERR_OOM) cudaGetLastError();
   return s;
 }
 
