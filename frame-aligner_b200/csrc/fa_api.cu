@@ -1202,6 +1202,7 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
   const bool reuse = bc->exec && bc->frames.size() == (size_t)n &&
                      std::equal(bc->frames.begin(), bc->frames.end(), frames) && std::equal(key, key + 7, bc->key);
   if (!reuse) {
+    bc->captures++;
     if (bc->exec) cudaGraphExecDestroy(bc->exec);
     bc->exec = nullptr;
     bc->frames.clear();
@@ -1647,6 +1648,15 @@ extern "C" fa_status fa_correlator_shift_device(fa_correlator* C, const float* v
 
 // ================================================================== test hooks ====================
 
+extern "C" fa_status fa_test_aligner_graphs(fa_aligner* A, long long* captured, int* kept) {
+  if (!A || !captured || !kept) return fail(FA_ERR_BAD_ARG, "NULL argument");
+  std::lock_guard<std::mutex> lk(A->mu);
+  *captured = A->graphs_captured;
+  *kept = 0;
+  for (const BatchCache& c : A->batch_cache) *kept += c.exec != nullptr;
+  return FA_OK;
+}
+
 extern "C" fa_status fa_test_plane_tables(int nz, int ny, int nx, double* tw_x, int cap_x, int* n_x, int* x_post,
                                           double* tw_y, int cap_y, int* n_y, int* rows_per_cta, int* planes_per_cta) {
   if (!tw_x || !n_x || !x_post || !tw_y || !n_y || !rows_per_cta || !planes_per_cta)
@@ -1775,6 +1785,7 @@ namespace {
 void aligner_release_reference(fa_aligner* A) {
   aligner_release_results(A);
   for (auto& c : A->batch_cache) batch_cache_release(A->ctx, &c);
+  A->batch_cache.clear();
   dfree_all(A->ctx, A->smooth_allocs);
   A->smooth_kx = A->smooth_ky = A->smooth_tmp = A->smooth_out = nullptr;
   A->smooth_nkx = A->smooth_nky = 0;
@@ -1847,11 +1858,42 @@ fa_status aligner_grow(fa_aligner* A, int n, int kind, size_t staging_need) {
 // ms a call: 50 frames of 16 x 512 x 512 (8.4 MB) 10.07 / 9.72 / 9.38, 16 of them 3.55 / 3.22 / 3.21; 8 of
 // 32 x 512 x 512 (16.8 MB) 4.97 / 4.91 / 4.32; 4 of 64 x 1024 x 1024 (134 MB) 43.4 / 38.3 / 38.5; 24 of 8 x 512 x
 // 512 (4.2 MB) 2.49 / 2.42 / 2.44; 32 of 4 x 512 x 512 (2.1 MB) 1.87 / 1.89 / 2.00; 40 of 2 x 512 x 512 1.51 / 1.56 /
-// 1.79. (Half that upload, 2 frames of 8.4 MB, would make an aligner's first call instantiate 25 graphs for
-// 50 frames.) Frames in device memory: 7.19 ms in groups of 8, 7.34 in groups of 4.
-int host_group_frames(size_t raw_bytes) {
+// 1.79. Frames in device memory: 7.19 ms in groups of 8, 7.34 in groups of 4. Each group has a graph and buffers
+// of its own, made by the first call that has it (50 frames of 16.8 MB, 26 groups of up to 2: first call 46 ms, 51 in
+// groups of 8; the slots are most of it), so that there are at most kMostGroups, whatever the number of frames.
+int host_group_frames(size_t raw_bytes, int n) {
   constexpr size_t kUpload = (size_t)32 << 20;
-  return (int)std::min<size_t>(8, std::max<size_t>(2, kUpload / std::max<size_t>(raw_bytes, 1)));
+  constexpr int kMostGroups = 64;
+  const int group = (int)std::min<size_t>(8, std::max<size_t>(2, kUpload / std::max<size_t>(raw_bytes, 1)));
+  return std::max(group, (n + kMostGroups - 1) / kMostGroups);
+}
+
+// The buffers and graph kept for the solve of slots [first, first + n). They are looked up by that range,
+// because the groups of a call depend on its number of frames and on where they come from: an aligner that
+// takes host and device frames in turn, or now and then one frame fewer, keeps a graph for each (16 frames of
+// 8.4 MB from the host and from the device in turn, by the group's number instead: nearly every graph made
+// anew, 4.5 and 3.0 ms a call; so 3.3 and 2.3). Beyond kMostCaches the one unused for longest goes; its streams
+// are idle, as every call ends with a wait for all of its solves.
+BatchCache* aligner_batch_cache(fa_aligner* A, int first, int n) {
+  constexpr size_t kMostCaches = 128;
+  BatchCache* found = nullptr;
+  auto oldest = A->batch_cache.end();
+  for (auto it = A->batch_cache.begin(); it != A->batch_cache.end(); ++it) {
+    if (it->first == first && it->count == n) found = &*it;
+    if (it->used != A->calls && (oldest == A->batch_cache.end() || it->used < oldest->used)) oldest = it;
+  }
+  if (!found) {
+    if (A->batch_cache.size() >= kMostCaches && oldest != A->batch_cache.end()) {
+      batch_cache_release(A->ctx, &*oldest);
+      A->batch_cache.erase(oldest);
+    }
+    A->batch_cache.emplace_back();
+    found = &A->batch_cache.back();
+    found->first = first;
+    found->count = n;
+  }
+  found->used = A->calls;
+  return found;
 }
 
 // Solve groups of one call, as frame boundaries {0, ..., n}: groups of `chunk` frames (a last
@@ -1897,7 +1939,7 @@ fa_status aligner_run(fa_aligner* A, const void* const* frames, fa_dtype dtype, 
   FA_CU(cudaEventRecord(A->ev0, s));
   // Host frames upload on a copy stream in chunks of a solve group; each chunk's conversion and phase
   // correlation wait only for its own uploads, so they overlap the uploads of the chunks after it.
-  const int group = device_src ? 8 : host_group_frames(raw_bytes);
+  const int group = device_src ? 8 : host_group_frames(raw_bytes, n);
   const int chunk = device_src ? n : group;
   if (!device_src) {
     if (!A->copy_stream) FA_CU(cudaStreamCreateWithFlags(&A->copy_stream, cudaStreamNonBlocking));
@@ -1923,7 +1965,9 @@ fa_status aligner_run(fa_aligner* A, const void* const* frames, fa_dtype dtype, 
   FA_TRY(correlator_reserve(A->corr, n));
   const std::vector<int> gb = solve_groups(n, group, device_src ? 0 : raw_bytes);  // group g: frames [gb[g], gb[g + 1])
   const int n_groups = (int)gb.size() - 1;
-  while ((int)A->batch_cache.size() < n_groups) A->batch_cache.emplace_back();
+  A->calls++;
+  std::vector<BatchCache*> cache((size_t)n_groups);
+  for (int g = 0; g < n_groups; g++) cache[g] = aligner_batch_cache(A, gb[g], gb[g + 1] - gb[g]);
   while ((int)A->group_ev.size() < n_groups) {
     cudaEvent_t e;
     FA_CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1998,8 +2042,9 @@ fa_status aligner_run(fa_aligner* A, const void* const* frames, fa_dtype dtype, 
   for (int g = 0; g < n_groups && r == FA_OK; g++) {
     const int g0 = gb[g], g1 = gb[g + 1];
     const PeakStart ps{C->d_idx + g0, C->nx, C->ny, C->nz, A->prm.spatial_binning, A->group_ev[g]};
-    r = align_batch_enqueue(batch.data() + g0, g1 - g0, nullptr, A->prm.max_iterations, nullptr, &A->batch_cache[g],
-                            &ps, alone);
+    const int before = cache[g]->captures;
+    r = align_batch_enqueue(batch.data() + g0, g1 - g0, nullptr, A->prm.max_iterations, nullptr, cache[g], &ps, alone);
+    A->graphs_captured += cache[g]->captures - before;
     // the last group's stream also holds whatever its failed enqueue left queued
     queued = g + 1;
   }
@@ -2011,7 +2056,7 @@ fa_status aligner_run(fa_aligner* A, const void* const* frames, fa_dtype dtype, 
       g_err = keep;
       continue;
     }
-    r = align_batch_finish(batch.data() + g0, g1 - g0, &A->batch_cache[g], D_out + (size_t)g0 * 3 * A->ref->nD,
+    r = align_batch_finish(batch.data() + g0, g1 - g0, cache[g], D_out + (size_t)g0 * 3 * A->ref->nD,
                            stats ? stats + g0 : nullptr);
   }
   if (r != FA_OK) return r;

@@ -7,6 +7,7 @@
 
 #include <atomic>
 #include <deque>
+#include <list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -158,7 +159,11 @@ struct BatchCache {
   char* d_out = nullptr;    // its device address
   size_t out_bytes = 0;
   int per_round = 0;        // kernel launches per round
+  int captures = 0;         // graphs captured so far
   int cap = 0;
+  // an aligner's: the slots it is for, and the last call that used it
+  int first = 0, count = 0;
+  long long used = 0;
   cudaGraphExec_t exec = nullptr;
   std::vector<fa_frame*> frames;  // the frames the graph was captured for
   long long key[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -194,7 +199,9 @@ struct fa_aligner {
   cudaStream_t copy_stream = nullptr;
   std::vector<cudaEvent_t> copy_ev;
   std::vector<cudaEvent_t> group_ev;  // peaks of a group of frames read back
-  std::deque<fa_rt::BatchCache> batch_cache;  // the batched solve's buffers and graph per solve group
+  std::list<fa_rt::BatchCache> batch_cache;  // the batched solve's buffers and graph per range of slots
+  long long calls = 0;
+  long long graphs_captured = 0;
   // smoothStack (smoothing > 0): Gaussian weights along x and y, and two frame-sized work buffers
   // used one frame at a time in stream order
   float* smooth_kx = nullptr;

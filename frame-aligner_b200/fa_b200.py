@@ -182,6 +182,7 @@ SIGNATURES = {
     "fa_profile_eval": [_vp, C.c_int, _f64p, C.c_int, C.POINTER(C.c_double)],
     "fa_test_tr_subproblem": [_vp, C.c_int, C.c_int, _f64p, _f64p, C.c_double, _f64p, C.POINTER(C.c_int)],
     "fa_test_correlation_surface": [_vp, _f32p, C.c_int, _f64p],
+    "fa_test_aligner_graphs": [_vp, C.POINTER(C.c_longlong), C.POINTER(C.c_int)],
     "fa_test_downsample": [_vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _f32p],
     "fa_test_plane_tables": [C.c_int, C.c_int, C.c_int, _f64p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int),
                              _f64p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)],
@@ -524,6 +525,12 @@ class Aligner:
         ms = C.c_double()
         check(lib().fa_aligner_last_device_ms(self._h, C.byref(ms)))
         return ms.value
+
+    def graphs(self):
+        """Solve graphs captured so far and kept now (test hook)."""
+        captured, kept = C.c_longlong(), C.c_int()
+        check(lib().fa_test_aligner_graphs(self._h, C.byref(captured), C.byref(kept)))
+        return captured.value, kept.value
 
     def last_phase_ms(self):
         """(correlation ms, total ms) of the last add_frames call (fa_aligner_last_phase_ms)."""

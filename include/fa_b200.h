@@ -396,6 +396,11 @@ fa_status fa_test_downsample(fa_context* ctx, const void* volume, fa_dtype dtype
    cuFFT (use_planes = 0). Lets tests compare both with a CPU DFT. */
 fa_status fa_test_correlation_surface(fa_correlator* c, const float* volume, int use_planes, double* surface);
 
+/* Test hook (no reference counterpart): the solve graphs the aligner has captured since it was created, and
+   those that it keeps now. Lets tests see that calls of a kind the aligner has had before make no
+   new ones, and that the number kept is bounded. */
+fa_status fa_test_aligner_graphs(fa_aligner* a, long long* captured, int* kept);
+
 /* Test hook (no reference counterpart, host only: no device work): the tables and launch shape the
    fused kx-plane passes would use for an nz x ny x nx volume. tw_x receives n_x complex twiddles
    (interleaved re, im): the stage twiddles of the nx/2-point row DFT, then W_nx^k for k = 0..nx/2
