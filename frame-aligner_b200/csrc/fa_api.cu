@@ -1065,9 +1065,10 @@ extern "C" fa_status fa_align_frame(fa_frame* F, const double* rigid_shift, int 
     for (int i = 0; i < kBurst; i++) {
       FA_CU(fa::launch_eval(job, 1, R->G.n_tiles, R->n_dim, F->kind, R->prec == FA_PREC_MIXED, F->stream, R->nx % 4 == 0,
                             R->host.tune_mb_small));
-      if (fa::wide_reduction(R->G.n_tiles)) FA_CU(fa::launch_wide_reduce(job, 1, R->nD, F->stream));
+      const bool wide = fa::wide_reduction(R->G.n_tiles);
+      if (wide) FA_CU(fa::launch_wide_reduce(job, 1, R->nD, F->stream));
       FA_CU(fa::launch_solve(job, 1, R->nD, R->n_dim, F->stream, nullptr, nullptr, nullptr, nullptr, false, overlap));
-      g_launches += 2;
+      g_launches += wide ? 3 : 2;
     }
     FA_CU(cudaStreamSynchronize(F->stream));
   }
@@ -1254,7 +1255,8 @@ fa_status align_batch_enqueue(fa_frame* const* frames, int n, const double* rigi
   }
   e = cudaGraphLaunch(bc->exec, s);
   if (e != cudaSuccess) return fail(FA_ERR_CUDA, std::string("batch solve: ") + cudaGetErrorString(e));
-  bc->per_round = 2 * kGraphIters;
+  const int pass = vec4 ? fa::eval4_active_kernels(least_items, most_items) : 1;
+  bc->per_round = (pass + (fa::wide_reduction(max_tiles) ? 1 : 0) + 1) * kGraphIters;
   return FA_OK;
 }
 

@@ -997,6 +997,10 @@ inline cudaError_t dispatch_mb(int mb, Fn&& f) {
 
 bool eval4_few_only(long long most_items) { return most_items <= kCtaTiles; }
 
+int eval4_active_kernels(long long least_items, long long most_items) {
+  return (least_items <= kCtaTiles ? 1 : 0) + (most_items > kCtaTiles ? 1 : 0);
+}
+
 cudaError_t launch_eval4(const Job* jobs_dev, int n_jobs, int max_tiles, int n_dim, int frame_kind, bool ref_bf16,
                          int mb, cudaStream_t s) {
   if ((long long)max_tiles * n_jobs <= kCtaTiles)

@@ -116,6 +116,9 @@ cudaError_t launch_eval4_active(const Job* jobs_dev, const int* active, const in
 // and steps may overlap.
 bool eval4_few_only(long long most_items);
 
+// Kernels that launch_eval4_active queues for these bounds: one form, or both where the list may need either.
+int eval4_active_kernels(long long least_items, long long most_items);
+
 // Thread-local (spill) bytes of that kernel's instantiation for a register budget of mb CTAs per SM.
 size_t eval4_active_local_bytes(int n_dim, int frame_kind, bool ref_bf16, int mb);
 

@@ -6,7 +6,6 @@
 #include <cufft.h>
 
 #include <atomic>
-#include <deque>
 #include <list>
 #include <map>
 #include <mutex>

@@ -130,6 +130,7 @@ struct SrvClass {
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  int per_launch = 0;  // kernels in the graph
   bool dirty = true;
   cudaEvent_t ev = nullptr;
   bool running = false;
@@ -337,6 +338,8 @@ fa_status class_capture(fa_server* S, SrvClass* C) {
   }
   if (e == cudaSuccess) e = cudaGraphInstantiate(&C->exec, C->graph, 0);
   if (e != cudaSuccess) return fail(FA_ERR_CUDA, std::string("server graph: ") + cudaGetErrorString(e));
+  const int pass = C->vec4 ? fa::eval4_active_kernels(C->min_tiles, most_items) : 1;
+  C->per_launch = (pass + (fa::wide_reduction(C->max_tiles) ? 1 : 0) + 1) * S->cfg.iterations_per_launch + 1;
   C->dirty = false;
   return FA_OK;
 }
@@ -584,7 +587,7 @@ fa_status class_launch(fa_server* S, SrvClass* C, bool* launched) {
     g_launches += 1;
   }
   FA_CU(cudaGraphLaunch(C->exec, C->stream));
-  g_launches += 2 * S->cfg.iterations_per_launch + 1;
+  g_launches += C->per_launch;
   FA_CU(cudaEventRecord(C->ev, C->stream));
   FA_CU(cudaLaunchHostFunc(C->stream, wake_worker, S));
   C->in_solve += n_act;

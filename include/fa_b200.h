@@ -357,7 +357,9 @@ fa_status fa_get_error_jacobian_static(const fa_reference* ref, const void* fram
 
 /* ---------------------------------------------------------------- measurement ----------------- */
 
-/* Number of this library's kernels launched so far in the process (graph replays included). */
+/* Number of this library's kernels launched so far in the process by evaluations, warps, correlations,
+   solves and aligned or served frames (graph replays included; the kernels that set up a reference, a
+   registered frame or a correlator are not counted, nor are cuFFT's). */
 long long fa_kernel_launches(void);
 /* Device time (CUDA events on the library's streams) of the last fa_aligner_add_frames* call, ms. */
 fa_status fa_aligner_last_device_ms(const fa_aligner* a, double* ms);
