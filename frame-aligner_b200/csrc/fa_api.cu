@@ -98,6 +98,15 @@ struct ScanEval {
   }
 };
 
+// RefDev::ctrl_tiles of tiles that start at the ranges tile_c0.
+void control_tiles(const std::vector<int>& tile_c0, int nD, std::vector<int4>* out) {
+  out->resize(nD);
+  for (int c = 0; c < nD; c++) {
+    auto first_at_least = [&](int r) { return (int)(std::lower_bound(tile_c0.begin(), tile_c0.end(), r) - tile_c0.begin()); };
+    (*out)[c] = make_int4(first_at_least(c - 2), first_at_least(c - 1), first_at_least(c), first_at_least(c + 1));
+  }
+}
+
 // Tiles of whole rows, about target_tile_voxels each, never longer than the shortest storage range
 // (so a tile meets at most two ranges); per tile its first range, per control point its tile span.
 void assign_tiles(Geometry& G, int target_tile_voxels) {
@@ -108,13 +117,7 @@ void assign_tiles(Geometry& G, int target_tile_voxels) {
   G.n_tiles = (G.n_rows + tr - 1) / tr;
   G.tile_c0.resize(G.n_tiles);
   for (int t = 0; t < G.n_tiles; t++) G.tile_c0[t] = G.rows[(size_t)t * tr].r0;
-  G.ctrl_tiles.resize(nD);
-  for (int c = 0; c < nD; c++) {
-    auto first_at_least = [&](int r) {
-      return (int)(std::lower_bound(G.tile_c0.begin(), G.tile_c0.end(), r) - G.tile_c0.begin());
-    };
-    G.ctrl_tiles[c] = make_int4(first_at_least(c - 2), first_at_least(c - 1), first_at_least(c), first_at_least(c + 1));
-  }
+  control_tiles(G.tile_c0, nD, &G.ctrl_tiles);
 }
 
 fa_status build_geometry(const fa_scan_params& scan, int nz, int ny, int nx, int nD, int target_tile_voxels,
@@ -1777,6 +1780,48 @@ extern "C" fa_status fa_test_tr_subproblem(fa_context* ctx, int nD, int n_dim, c
   if (e == cudaSuccess) e = cudaMemcpy(p, dp, (size_t)P * sizeof(double), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(on_boundary, db, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return done(fail(FA_ERR_CUDA, std::string("subproblem: ") + cudaGetErrorString(e)));
+  return done(FA_OK);
+}
+
+extern "C" fa_status fa_test_reduce(fa_context* ctx, int nD, int n_dim, int n_tiles, const int* tile_c0,
+                                    const double* partials, int wide, double* result) {
+  if (!ctx || !tile_c0 || !partials || !result || nD < 2 || (n_dim != 2 && n_dim != 3) || n_tiles < 1)
+    return fail(FA_ERR_BAD_ARG, "bad arguments");
+  for (int t = 0; t < n_tiles; t++)
+    if (tile_c0[t] < (t ? tile_c0[t - 1] : 0) || tile_c0[t] > nD - 2)
+      return fail(FA_ERR_BAD_ARG, "tiles start at ascending ranges below nD - 1");
+  FA_CU(cudaSetDevice(ctx->device));
+  std::vector<int4> ctrl;
+  control_tiles(std::vector<int>(tile_c0, tile_c0 + n_tiles), nD, &ctrl);
+  const size_t np = (size_t)n_tiles * fa::kPartialDoubles, nr = (size_t)nD * n_dim + 1;
+  std::vector<Alloc> tmp;
+  double *parts = nullptr, *res = nullptr;
+  int4* dctrl = nullptr;
+  Job* dj = nullptr;
+  auto done = [&](fa_status st) {
+    std::string keep = g_err;
+    dfree_all(ctx, tmp);
+    g_err = keep;
+    return st;
+  };
+  fa_status st;
+  if ((st = dalloc_t(ctx, np, &parts, tmp)) != FA_OK || (st = dalloc_t(ctx, nr, &res, tmp)) != FA_OK ||
+      (st = dalloc_t(ctx, ctrl.size(), &dctrl, tmp)) != FA_OK || (st = dalloc_t(ctx, 1, &dj, tmp)) != FA_OK)
+    return done(st);
+  Job j{};
+  j.R.nD = nD;
+  j.R.n_dim = n_dim;
+  j.R.P = nD * n_dim;
+  j.R.n_tiles = n_tiles;
+  j.R.ctrl_tiles = dctrl;
+  j.partials = parts;
+  j.result = res;
+  cudaError_t e = cudaMemcpy(parts, partials, np * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dctrl, ctrl.data(), ctrl.size() * sizeof(int4), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dj, &j, sizeof(Job), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = fa::launch_reduce_form(dj, wide != 0, nD, 0);
+  if (e == cudaSuccess) e = cudaMemcpy(result, res, nr * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return done(fail(FA_ERR_CUDA, std::string("reduction: ") + cudaGetErrorString(e)));
   return done(FA_OK);
 }
 

@@ -780,7 +780,11 @@ cudaError_t launch_reduce(const Job* job_dev, int n_tiles, int nD, cudaStream_t 
   // A bare evaluation's reduction is a launch of its own either way: 1024 tiles (512 x 512 x 16) 65 us a call
   // with one CTA, 59 with many; a step's would be one launch more (271 -> 299 us a solve there).
   constexpr int kBareWideTiles = 768;
-  if (n_tiles > kBareWideTiles) {
+  return launch_reduce_form(job_dev, n_tiles > kBareWideTiles, nD, s, overlap);
+}
+
+cudaError_t launch_reduce_form(const Job* job_dev, bool wide, int nD, cudaStream_t s, bool overlap) {
+  if (wide) {
     wide_reduce_kernel<<<dim3(nD + 1, 1), kWideThreads, 0, s>>>(job_dev, nullptr, nullptr, 1);
     return cudaGetLastError();
   }

@@ -151,6 +151,8 @@ cudaError_t launch_activate(const Job* jobs_dev, const Activation* recs, int n, 
 // Reduces one job's tile partials into result = [f, g(P)] (deterministic order). overlap: directly after
 // a few-tile pass.
 cudaError_t launch_reduce(const Job* job_dev, int n_tiles, int nD, cudaStream_t s, bool overlap = false);
+// The same in a given form: over many CTAs (wide) or by one.
+cudaError_t launch_reduce_form(const Job* job_dev, bool wide, int nD, cudaStream_t s, bool overlap = false);
 // Before launch_solve (same arguments) when a frame of it has many tiles (wide_reduction): those frames'
 // tile partials into the places where the step takes them from.
 bool wide_reduction(int n_tiles);

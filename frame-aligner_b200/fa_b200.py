@@ -182,6 +182,7 @@ SIGNATURES = {
     "fa_profile_eval": [_vp, C.c_int, _f64p, C.c_int, C.POINTER(C.c_double)],
     "fa_test_tr_subproblem": [_vp, C.c_int, C.c_int, _f64p, _f64p, C.c_double, _f64p, C.POINTER(C.c_int)],
     "fa_test_correlation_surface": [_vp, _f32p, C.c_int, _f64p],
+    "fa_test_reduce": [_vp, C.c_int, C.c_int, C.c_int, _i32p, _f64p, C.c_int, _f64p],
     "fa_test_aligner_graphs": [_vp, C.POINTER(C.c_longlong), C.POINTER(C.c_int)],
     "fa_test_downsample": [_vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _f32p],
     "fa_test_plane_tables": [C.c_int, C.c_int, C.c_int, _f64p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int),
@@ -704,6 +705,14 @@ def test_tr_subproblem(ctx: Context, nD, n_dim, H, g, radius):
     b = C.c_int()
     check(lib().fa_test_tr_subproblem(ctx._h, nD, n_dim, _c64(H), _c64(g), radius, p, C.byref(b)))
     return p, bool(b.value)
+
+
+def test_reduce(ctx: Context, nD, n_dim, tile_c0, partials, wide):
+    """fa_test_reduce: [f, g] of tile sums (n_tiles x 12) by one CTA or over many."""
+    c0 = np.ascontiguousarray(tile_c0, np.int32)
+    out = np.empty(1 + nD * n_dim, np.float64)
+    check(lib().fa_test_reduce(ctx._h, nD, n_dim, c0.size, c0, _c64(partials), 1 if wide else 0, out))
+    return out
 
 
 def test_downsample(ctx: Context, volume, factor):

@@ -398,6 +398,13 @@ fa_status fa_test_downsample(fa_context* ctx, const void* volume, fa_dtype dtype
    cuFFT (use_planes = 0). Lets tests compare both with a CPU DFT. */
 fa_status fa_test_correlation_surface(fa_correlator* c, const float* volume, int use_planes, double* surface);
 
+/* Test hook (no reference counterpart): the reduction of one frame's tile sums. Tile t (12 doubles: f, an unused
+   one, 3 sums for each of the control points tile_c0[t], + 1 and + 2, an unused one) starts at range tile_c0[t], which
+   does not decrease; result is [f, g(nD * n_dim)], by one CTA or over many (wide). Lets tests compare both
+   forms with the order of summation they share. */
+fa_status fa_test_reduce(fa_context* ctx, int nD, int n_dim, int n_tiles, const int* tile_c0, const double* partials,
+                         int wide, double* result);
+
 /* Test hook (no reference counterpart): the solve graphs the aligner has captured since it was created, and
    those that it keeps now. Lets tests see that calls of a kind the aligner has had before make no
    new ones, and that the number kept is bounded. */
