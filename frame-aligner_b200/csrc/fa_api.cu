@@ -1684,7 +1684,20 @@ extern "C" fa_status fa_test_plane_tables(int nz, int ny, int nx, double* tw_x, 
   *x_post = d.tw_x_post;
   *n_y = d.n_twy;
   *rows_per_cta = 1 << d.log2G;
-  *planes_per_cta = d.PP;
+  *planes_per_cta = d.split ? 0 : std::max(1, 8192 / (nz * ny));
+  return FA_OK;
+}
+
+extern "C" fa_status fa_test_plane_launch(int nz, int ny, int nx, int batch, int* planes_per_cta, long long* ctas,
+                                          long long* smem_bytes) {
+  if (!planes_per_cta || !ctas || !smem_bytes || batch < 1) return fail(FA_ERR_BAD_ARG, "bad arguments");
+  fa::PlaneDims d{};
+  if (!fa::plane_dims(nz, ny, nx, &d) || d.split)
+    return fail(FA_ERR_UNSUPPORTED, "dimensions outside the one-kernel (z, y) pass");
+  const fa::PlaneLaunch l = fa::plane_yz_launch(nz, ny, (long long)batch * (nx / 2 + 1));
+  *planes_per_cta = l.planes;
+  *ctas = l.ctas;
+  *smem_bytes = (long long)l.smem;
   return FA_OK;
 }
 

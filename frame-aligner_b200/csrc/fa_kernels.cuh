@@ -226,7 +226,6 @@ cudaError_t launch_phase_argmax_final(const double* block_val, const long long* 
 struct PlaneDims {
   int nz, ny, nx, rows;      // rows = nz * ny
   int log2M, log2ny, log2G;  // M = nx / 2; G rows per row CTA
-  int PP;                    // planes in 8192 points, two CTAs' (one-kernel (z, y) pass); 0 when split
   int n_twx, tw_x_post;      // x twiddles: stage table of the nx/2-point DFT, then W_nx^k (k <= nx/2)
   int n_twy;                 // y twiddles: stage table of the ny-point DFT
   long long n_complex, n_el;
@@ -243,6 +242,14 @@ bool plane_dims(int nz, int ny, int nx, PlaneDims* d);
 // pass is split, else empty), computed in long double.
 void plane_twiddles(const PlaneDims& d, std::vector<double2>* tw_x, std::vector<double2>* tw_y,
                     std::vector<double2>* tw_z);
+// Launch of the one-kernel (z, y) pass over n_planes planes (not for split dimensions): CTAs of `planes` planes
+// each, or a pair of CTAs per plane (planes 0), and the shared memory of each CTA.
+struct PlaneLaunch {
+  int planes;
+  long long ctas;
+  size_t smem;
+};
+PlaneLaunch plane_yz_launch(int nz, int ny, long long n_planes);
 // CTAs (argmax partials) per frame of the last pass.
 int plane_blocks_per_frame(const PlaneDims& d);
 // Frame slots the first pass may fill while it reads the frames: frame i's value + 1 (the slot

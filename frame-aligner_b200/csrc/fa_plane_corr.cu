@@ -808,7 +808,6 @@ bool plane_dims(int nz, int ny, int nx, PlaneDims* d) {
   int G = 8;
   while (G > 1 && ((long long)G * (nx / 2) > (long long)kRowThreads * kRowEPT || G > d->rows)) G >>= 1;
   d->log2G = ilog2(G);
-  d->PP = d->split ? 0 : std::max(1, 2 * kPlanePoints / (nz * ny));
   d->n_complex = (long long)(nx / 2 + 1) * d->rows;
   d->n_el = (long long)nx * d->rows;
   d->tw_x_post = stage_count(nx / 2);
@@ -818,6 +817,14 @@ bool plane_dims(int nz, int ny, int nx, PlaneDims* d) {
 }
 
 int plane_blocks_per_frame(const PlaneDims& d) { return d.rows >> d.log2G; }
+
+PlaneLaunch plane_yz_launch(int nz, int ny, long long n_planes) {
+  static_assert(kPairThreads * kPairEPT == kPlanePoints, "half a plane per CTA of a pair");
+  if (nz >= 4 && nz * ny == 2 * kPlanePoints)  // half of the plane's z lines each
+    return PlaneLaunch{0, 2 * n_planes, ((size_t)(nz / 2) * (ny + 1) + ny) * sizeof(double2)};
+  const int pp = planes_of_cta(nz, ny);
+  return PlaneLaunch{pp, (n_planes + pp - 1) / pp, ((size_t)pp * nz * (ny + 1) + ny) * sizeof(double2)};
+}
 
 namespace {
 template <bool U16, int SLOT>
@@ -852,22 +859,19 @@ namespace {
 template <int NZ, bool REF>
 cudaError_t launch_yz(const PlaneDims& d, const double2* in, double2* out, const double2* ref_conj,
                       const double2* tw_y, long long n_planes, cudaStream_t s, bool overlap) {
+  const PlaneLaunch l = plane_yz_launch(NZ, d.ny, n_planes);
   if constexpr (NZ >= 4) {
-    if ((long long)NZ * d.ny == 2LL * kPairThreads * kPairEPT) {  // one plane per pair of CTAs
-      const size_t smem = ((size_t)(NZ / 2) * (d.ny + 1) + d.ny) * sizeof(double2);
-      cudaError_t e = allow_smem<plane_yz_pair_kernel<NZ, REF>>(smem, kPlaneSmem);
+    if (l.planes == 0) {
+      const cudaError_t e = allow_smem<plane_yz_pair_kernel<NZ, REF>>(l.smem, kPlaneSmem);
       if (e != cudaSuccess) return e;
-      return launch_overlapped(plane_yz_pair_kernel<NZ, REF>, dim3((unsigned)(2 * n_planes)), dim3(kPairThreads), smem, s,
-                               overlap, in, out, ref_conj, tw_y, d);
+      return launch_overlapped(plane_yz_pair_kernel<NZ, REF>, dim3((unsigned)l.ctas), dim3(kPairThreads), l.smem, s, overlap,
+                               in, out, ref_conj, tw_y, d);
     }
   }
-  const int pp = planes_of_cta(NZ, d.ny);
-  if (pp * NZ * d.ny > kPlanePoints) return cudaErrorInvalidValue;
-  const size_t smem = ((size_t)pp * NZ * (d.ny + 1) + d.ny) * sizeof(double2);
-  cudaError_t e = allow_smem<plane_yz_kernel<NZ, REF>>(smem, kPlaneSmem);
+  if (l.planes * NZ * d.ny > kPlanePoints) return cudaErrorInvalidValue;
+  const cudaError_t e = allow_smem<plane_yz_kernel<NZ, REF>>(l.smem, kPlaneSmem);
   if (e != cudaSuccess) return e;
-  const long long grid = (n_planes + pp - 1) / pp;
-  return launch_overlapped(plane_yz_kernel<NZ, REF>, dim3((unsigned)grid), dim3(kPlaneThreads), smem, s, overlap, in, out,
+  return launch_overlapped(plane_yz_kernel<NZ, REF>, dim3((unsigned)l.ctas), dim3(kPlaneThreads), l.smem, s, overlap, in, out,
                            ref_conj, tw_y, d, n_planes);
 }
 

@@ -187,6 +187,8 @@ SIGNATURES = {
     "fa_test_downsample": [_vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _f32p],
     "fa_test_plane_tables": [C.c_int, C.c_int, C.c_int, _f64p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int),
                              _f64p, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)],
+    "fa_test_plane_launch": [C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_longlong),
+                             C.POINTER(C.c_longlong)],
 }
 
 
@@ -738,6 +740,13 @@ def plane_tables(nz, ny, nx):
     as_c = lambda a, n: a[: 2 * n].reshape(n, 2) @ np.array([1.0, 1.0j])
     return {"tw_x": as_c(tx, n_x.value), "x_post": x_post.value, "tw_y": as_c(ty, n_y.value),
             "rows_per_cta": g.value, "planes_per_cta": pp.value}
+
+
+def plane_launch(nz, ny, nx, batch):
+    """Host-only test hook (fa_test_plane_launch): planes per CTA, CTAs and shared bytes per CTA."""
+    pp, ctas, smem = C.c_int(), C.c_longlong(), C.c_longlong()
+    check(lib().fa_test_plane_launch(nz, ny, nx, batch, C.byref(pp), C.byref(ctas), C.byref(smem)))
+    return pp.value, ctas.value, smem.value
 
 
 class B200FrameWarper:
