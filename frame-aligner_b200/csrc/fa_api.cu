@@ -1755,19 +1755,66 @@ extern "C" fa_status fa_test_downsample(fa_context* ctx, const void* volume, fa_
   return done(FA_OK);
 }
 
+namespace {
+
+// The diagonal and sub-diagonal blocks of a dense H (P x P).
+void band_blocks(const double* H, int nD, int n_dim, std::vector<double>* hd, std::vector<double>* hl) {
+  const int P = nD * n_dim, nn = n_dim * n_dim;
+  hd->assign((size_t)nD * nn, 0.0);
+  hl->assign((size_t)nD * nn, 0.0);
+  for (int b = 0; b < nD; b++)
+    for (int a = 0; a < n_dim; a++)
+      for (int c = 0; c < n_dim; c++) {
+        (*hd)[(size_t)b * nn + a * n_dim + c] = H[(size_t)(b * n_dim + a) * P + b * n_dim + c];
+        if (b > 0) (*hl)[(size_t)b * nn + a * n_dim + c] = H[(size_t)(b * n_dim + a) * P + (b - 1) * n_dim + c];
+      }
+}
+
+}  // namespace
+
+extern "C" fa_status fa_test_ratio(fa_context* ctx, int nD, int n_dim, const double* H, const double* g, const double* p,
+                                   const double* measured, int n, double* predicted, int* taken, int* ordered) {
+  if (!ctx || !H || !g || !p || !measured || !predicted || !taken || !ordered || n < 1 || nD < 1 || (n_dim != 2 && n_dim != 3))
+    return fail(FA_ERR_BAD_ARG, "bad arguments");
+  FA_CU(cudaSetDevice(ctx->device));
+  std::vector<double> hd, hl;
+  band_blocks(H, nD, n_dim, &hd, &hl);
+  const size_t P = (size_t)nD * n_dim;
+  std::vector<Alloc> tmp;
+  double* d = nullptr;
+  int* bits = nullptr;
+  auto done = [&](fa_status st) {
+    std::string keep = g_err;
+    dfree_all(ctx, tmp);
+    g_err = keep;
+    return st;
+  };
+  fa_status st;
+  if ((st = dalloc_t(ctx, hd.size() + hl.size() + 2 * P + n + 1, &d, tmp)) != FA_OK ||
+      (st = dalloc_t(ctx, 2 * (size_t)n, &bits, tmp)) != FA_OK)
+    return done(st);
+  double *dHd = d, *dHl = dHd + hd.size(), *dg = dHl + hl.size(), *dp = dg + P, *dm = dp + P, *dpred = dm + n;
+  cudaError_t e = cudaMemcpy(dHd, hd.data(), hd.size() * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dHl, hl.data(), hl.size() * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dg, g, P * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dp, p, P * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(dm, measured, (size_t)n * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = fa::launch_test_ratio(dHd, dHl, nD, n_dim, dg, dp, dm, n, dpred, bits, bits + n, 0);
+  if (e == cudaSuccess) e = cudaMemcpy(predicted, dpred, sizeof(double), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(taken, bits, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(ordered, bits + n, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess) return done(fail(FA_ERR_CUDA, std::string("ratio: ") + cudaGetErrorString(e)));
+  return done(FA_OK);
+}
+
 extern "C" fa_status fa_test_tr_subproblem(fa_context* ctx, int nD, int n_dim, const double* H, const double* g,
                                            double radius, double* p, int* on_boundary) {
   if (!ctx || !H || !g || !p || !on_boundary || nD < 1 || (n_dim != 2 && n_dim != 3))
     return fail(FA_ERR_BAD_ARG, "bad arguments");
   FA_CU(cudaSetDevice(ctx->device));
-  const int P = nD * n_dim, nn = n_dim * n_dim;
-  std::vector<double> hd((size_t)nD * nn, 0.0), hl((size_t)nD * nn, 0.0);
-  for (int b = 0; b < nD; b++)
-    for (int a = 0; a < n_dim; a++)
-      for (int c = 0; c < n_dim; c++) {
-        hd[(size_t)b * nn + a * n_dim + c] = H[(size_t)(b * n_dim + a) * P + b * n_dim + c];
-        if (b > 0) hl[(size_t)b * nn + a * n_dim + c] = H[(size_t)(b * n_dim + a) * P + (b - 1) * n_dim + c];
-      }
+  const int P = nD * n_dim;
+  std::vector<double> hd, hl;
+  band_blocks(H, nD, n_dim, &hd, &hl);
   std::vector<Alloc> tmp;
   double *dHd, *dHl, *dg, *dp, *work;
   int* db;

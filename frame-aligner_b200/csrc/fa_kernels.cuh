@@ -185,6 +185,9 @@ cudaError_t launch_chol0(const double* Hd, const double* Hl, int nD, int nd, dou
 cudaError_t launch_test_subproblem(const double* Hd, const double* Hl, int nD, int nd, double hinf, double mindiag,
                                    const double* g, double radius, double* p_out, int* boundary_out, double* work,
                                    cudaStream_t s);
+// Test hook: the ratio test of a step for n measured reductions, as the solver takes it and by the ordered sum.
+cudaError_t launch_test_ratio(const double* Hd, const double* Hl, int nD, int nd, const double* g, const double* p,
+                              const double* meas, int n, double* pred, int* taken, int* ordered, cudaStream_t s);
 
 // Outputs after the solve (fa_output.cu). scan4 = processed {pixel, interline, interframe, stack}.
 // Forward splat of a dense raw frame (FA_F32 / FA_U16) by D (device, nD x 3): coverage always, the

@@ -902,4 +902,32 @@ cudaError_t launch_test_subproblem(const double* Hd, const double* Hl, int nD, i
   return cudaGetLastError();
 }
 
+// The ratio test on given H, g and p for n measured reductions: as the solver takes it, and as the ordered
+// sum alone decides it. pred: the ordered predicted reduction.
+template <int ND>
+__global__ void __launch_bounds__(kSolveThreads) test_ratio_kernel(const double* Hd, const double* Hl, int nD, const double* g,
+                                                                   const double* p, const double* meas, int n, double* pred,
+                                                                   int* taken, int* ordered) {
+  __shared__ double s_red[3 * (kSolveThreads / 32)];
+  __shared__ int s_flag;
+  const Band<ND> B{Hd, Hl, nD, nD * ND, 0.0, 0.0};
+  for (int i = 0; i < n; i++) {
+    const int r = ratio_block<ND>(B, g, p, meas[i], s_red, &s_flag);
+    if (threadIdx.x == 0) {
+      taken[i] = r;
+      *pred = predicted<ND>(B, g, p);
+      ordered[i] = ratio_bits(*pred, meas[i]);
+    }
+  }
+}
+
+cudaError_t launch_test_ratio(const double* Hd, const double* Hl, int nD, int nd, const double* g, const double* p,
+                              const double* meas, int n, double* pred, int* taken, int* ordered, cudaStream_t s) {
+  if (nd == 3)
+    test_ratio_kernel<3><<<1, kSolveThreads, 0, s>>>(Hd, Hl, nD, g, p, meas, n, pred, taken, ordered);
+  else
+    test_ratio_kernel<2><<<1, kSolveThreads, 0, s>>>(Hd, Hl, nD, g, p, meas, n, pred, taken, ordered);
+  return cudaGetLastError();
+}
+
 }  // namespace fa

@@ -182,6 +182,7 @@ SIGNATURES = {
     "fa_profile_eval": [_vp, C.c_int, _f64p, C.c_int, C.POINTER(C.c_double)],
     "fa_test_tr_subproblem": [_vp, C.c_int, C.c_int, _f64p, _f64p, C.c_double, _f64p, C.POINTER(C.c_int)],
     "fa_test_correlation_surface": [_vp, _f32p, C.c_int, _f64p],
+    "fa_test_ratio": [_vp, C.c_int, C.c_int, _f64p, _f64p, _f64p, _f64p, C.c_int, C.POINTER(C.c_double), _i32p, _i32p],
     "fa_test_reduce": [_vp, C.c_int, C.c_int, C.c_int, _i32p, _f64p, C.c_int, _f64p],
     "fa_test_aligner_graphs": [_vp, C.POINTER(C.c_longlong), C.POINTER(C.c_int)],
     "fa_test_downsample": [_vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _f32p],
@@ -707,6 +708,14 @@ def test_tr_subproblem(ctx: Context, nD, n_dim, H, g, radius):
     b = C.c_int()
     check(lib().fa_test_tr_subproblem(ctx._h, nD, n_dim, _c64(H), _c64(g), radius, p, C.byref(b)))
     return p, bool(b.value)
+
+
+def test_ratio(ctx: Context, nD, n_dim, H, g, p, measured):
+    """fa_test_ratio: the predicted reduction and, per measured one, the solver's bits and the ordered sum's."""
+    m = _c64(measured)
+    pred, taken, ordered = C.c_double(), np.empty(m.size, np.int32), np.empty(m.size, np.int32)
+    check(lib().fa_test_ratio(ctx._h, nD, n_dim, _c64(H), _c64(g), _c64(p), m, m.size, C.byref(pred), taken, ordered))
+    return pred.value, taken, ordered
 
 
 def test_reduce(ctx: Context, nD, n_dim, tile_c0, partials, wide):

@@ -398,6 +398,12 @@ fa_status fa_test_downsample(fa_context* ctx, const void* volume, fa_dtype dtype
    cuFFT (use_planes = 0). Lets tests compare both with a CPU DFT. */
 fa_status fa_test_correlation_surface(fa_correlator* c, const float* volume, int use_planes, double* surface);
 
+/* Test hook (no reference counterpart): the ratio test of a step p on given H and g for n measured reductions.
+   predicted: the predicted reduction -(g.p + p.H.p / 2) by the ordered sum; taken[i]: the solver's answer,
+   ordered[i]: the ordered sum's (bits: 1 the solve ends, 2 ratio < 1/4, 4 ratio > 3/4, 8 ratio > 0). */
+fa_status fa_test_ratio(fa_context* ctx, int nD, int n_dim, const double* H, const double* g, const double* p,
+                        const double* measured, int n, double* predicted, int* taken, int* ordered);
+
 /* Test hook (no reference counterpart): the reduction of one frame's tile sums. Tile t (12 doubles: f, an unused
    one, 3 sums for each of the control points tile_c0[t], + 1 and + 2, an unused one) starts at range tile_c0[t], which
    does not decrease; result is [f, g(nD * n_dim)], by one CTA or over many (wide). Lets tests compare both
