@@ -830,6 +830,8 @@ fa_status frame_alloc(fa_reference* R, int kind, fa_frame** out) {
     if (cudaMemcpyAsync(F->job_dev, js, sizeof(js), cudaMemcpyHostToDevice, F->stream) != cudaSuccess)
       return cleanup(fail(FA_ERR_CUDA, "job upload failed"));
   }
+  // An aligner and a server fill the slot on streams of their own, which do not wait for the clearing above.
+  if (cudaStreamSynchronize(F->stream) != cudaSuccess) return cleanup(fail(FA_ERR_CUDA, "slot set-up"));
   R->n_frames++;
   *out = F;
   return FA_OK;

@@ -392,7 +392,6 @@ fa_status slot_create(fa_server* S, SrvAcq* q, SrvSlot** out) {
   };
   fa_status st = frame_alloc(R, q->kind, &sl->F);
   if (st != FA_OK) return undo(st);
-  if (cudaStreamSynchronize(sl->F->stream) != cudaSuccess) return undo(fail(FA_ERR_CUDA, "slot set-up"));
   if ((st = dalloc(S->ctx, q->raw_bytes, &sl->raw, sl->allocs)) != FA_OK) return undo(st);
   if (A->prm.spatial_binning > 1 &&
       (st = dalloc_t(S->ctx, (size_t)A->dz * A->dy * A->dx, &sl->vol, sl->allocs)) != FA_OK)
@@ -855,7 +854,8 @@ extern "C" fa_status fa_server_add_acquisition(fa_server* S, const fa_aligner_pa
     if ((st = dalloc_t(S->ctx, nw, &q->warm, q->allocs)) != FA_OK) return undo(st);
     if ((st = dalloc_t(S->ctx, (size_t)S->cfg.warm_start, &q->warm_seq, q->allocs)) != FA_OK) return undo(st);
     if (cudaMemset(q->warm, 0, nw * sizeof(double)) != cudaSuccess ||
-        cudaMemset(q->warm_seq, 0xff, (size_t)S->cfg.warm_start * sizeof(long long)) != cudaSuccess)  // -1: empty
+        cudaMemset(q->warm_seq, 0xff, (size_t)S->cfg.warm_start * sizeof(long long)) != cudaSuccess ||  // -1: empty
+        cudaStreamSynchronize(nullptr) != cudaSuccess)  // the class's stream does not wait for the default one
       return undo(fail(FA_ERR_CUDA, "cudaMemset failed"));
   }
   std::unique_lock<std::mutex> lk(S->mu);
