@@ -202,19 +202,6 @@ cudaError_t launch_sobel(const float* m, int nz, int ny, int nx, float* gx, floa
 
 // ------------------------------------------------------------------ conversions ------------------
 
-__global__ void to_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = __float2bfloat16_rn(in[i]);
-}
-
-cudaError_t launch_to_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t s) {
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  if (blocks < 1) blocks = 1;
-  to_bf16_kernel<<<blocks, 256, 0, s>>>(in, out, n);
-  return cudaGetLastError();
-}
-
 __global__ void to_quad16_kernel(const float* __restrict__ ref, const float* __restrict__ gx,
                                  const float* __restrict__ gy, const float* __restrict__ gz, long long n,
                                  __nv_bfloat16* __restrict__ q16) {
@@ -246,25 +233,6 @@ __device__ __forceinline__ float load_any(const void* in, int t, long long i) {
     case FA_BF16: return __bfloat162float(static_cast<const __nv_bfloat16*>(in)[i]);
     default: return (float)static_cast<const uint16_t*>(in)[i];
   }
-}
-
-__global__ void convert_kernel(const void* __restrict__ in, int in_t, void* __restrict__ out, int out_t, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    float v = load_any(in, in_t, i);
-    if (out_t == FA_F16)
-      static_cast<__half*>(out)[i] = __float2half_rn(v);
-    else
-      static_cast<float*>(out)[i] = v;
-  }
-}
-
-cudaError_t launch_convert(const void* in, fa_dtype in_type, void* out, fa_dtype out_type, long long n,
-                           cudaStream_t s) {
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 148 * 32) blocks = 148 * 32;
-  if (blocks < 1) blocks = 1;
-  convert_kernel<<<blocks, 256, 0, s>>>(in, (int)in_type, out, (int)out_type, n);
-  return cudaGetLastError();
 }
 
 // Raw frame (any dtype) -> warper storage with FrameWarpAligner's +1 offset

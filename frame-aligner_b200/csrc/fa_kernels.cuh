@@ -72,15 +72,10 @@ cudaError_t launch_sobel(const float* m, int nz, int ny, int nx, float* gx, floa
 cudaError_t launch_hessian(const RefDev* ref_dev, const RefDev& ref_host, const double* scan4, double* tile_parts,
                            double* Hd, double* Hl, cudaStream_t s);
 
-// FP32 -> BF16 copy.
-cudaError_t launch_to_bf16(const float* in, __nv_bfloat16* out, long long n, cudaStream_t s);
 // FP32 reference and gradient planes -> the interleaved BF16 groups of RefDev::q16 (ceil(n / 4) * 16
 // values; entries past the volume are zero).
 cudaError_t launch_to_quad16(const float* ref, const float* gx, const float* gy, const float* gz, long long n,
                              __nv_bfloat16* q16, cudaStream_t s);
-// Any input dtype -> FP32 or FP16 frame storage.
-cudaError_t launch_convert(const void* in, fa_dtype in_type, void* out, fa_dtype out_type, long long n,
-                           cudaStream_t s);
 
 // Dense frame (any dtype) -> a frame slot's interior (pitch / plane stride), optionally with +1.
 cudaError_t launch_to_slot(const void* in, fa_dtype in_type, void* out, int out_kind, int nz, int ny, int nx,
