@@ -1063,6 +1063,14 @@ extern "C" fa_status fa_align_frame(fa_frame* F, const double* rigid_shift, int 
   const bool overlap = R->nx % 4 == 0 && fa::eval4_few_only(R->G.n_tiles);
   const fa::Job* job = F->job_dev + 1;
   F->have_last = false;
+  // On an error no step stays in flight: its report would be taken for the next solve's.
+  struct Drain {
+    cudaStream_t s;
+    bool armed;
+    ~Drain() {
+      if (armed) cudaStreamSynchronize(s);
+    }
+  } drain{F->stream, true};
   F->h_state->phase = fa::kPhaseStartZero;  // until the step that finishes the solve reports
   FA_CU(fa::launch_start(job, rigid_shift, max_iter, F->stream));
   g_launches += 1;
@@ -1077,6 +1085,7 @@ extern "C" fa_status fa_align_frame(fa_frame* F, const double* rigid_shift, int 
     }
     FA_CU(cudaStreamSynchronize(F->stream));
   }
+  drain.armed = false;
   if (F->h_state->phase != fa::kPhaseDone) return finish_solve(F, D_out, stats);  // where the solve stands
   finish_solve_read(F, F->h_x, *F->h_state, D_out, stats);
   return FA_OK;
