@@ -251,7 +251,8 @@ void aligner_release_results(fa_aligner* A);
 std::vector<float> gaussian_kernel(double sigma);
 // smoothStack of one dense raw frame (device) into A->smooth_out on stream s (no-op without smoothing).
 fa_status aligner_smooth(fa_aligner* A, const void* raw, fa_dtype dtype, cudaStream_t s);
-// Frame slot (zero-halo storage of the given FrameKind + solve buffers + stream) for reference R.
+// Frame slot (zero-halo storage of the given FrameKind + solve buffers + stream) for reference R. The slot is
+// cleared on the frame's stream: wait for that before another stream fills it.
 fa_status frame_alloc(fa_reference* R, int kind, fa_frame** out);
 // Slot storage the aligner uses for frames of dtype (raw uint16 counts + 1, FP16 or FP32 values + 1).
 int slot_kind_for(const fa_aligner* A, fa_dtype dtype);

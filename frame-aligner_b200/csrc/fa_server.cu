@@ -392,6 +392,7 @@ fa_status slot_create(fa_server* S, SrvAcq* q, SrvSlot** out) {
   };
   fa_status st = frame_alloc(R, q->kind, &sl->F);
   if (st != FA_OK) return undo(st);
+  if (cudaStreamSynchronize(sl->F->stream) != cudaSuccess) return undo(fail(FA_ERR_CUDA, "slot set-up"));
   if ((st = dalloc(S->ctx, q->raw_bytes, &sl->raw, sl->allocs)) != FA_OK) return undo(st);
   if (A->prm.spatial_binning > 1 &&
       (st = dalloc_t(S->ctx, (size_t)A->dz * A->dy * A->dx, &sl->vol, sl->allocs)) != FA_OK)
