@@ -1979,7 +1979,7 @@ fa_status aligner_grow(fa_aligner* A, int n, int kind, size_t staging_need) {
 // 32 x 512 x 512 (16.8 MB) 4.97 / 4.91 / 4.32; 4 of 64 x 1024 x 1024 (134 MB) 43.4 / 38.3 / 38.5; 24 of 8 x 512 x
 // 512 (4.2 MB) 2.49 / 2.42 / 2.44; 32 of 4 x 512 x 512 (2.1 MB) 1.87 / 1.89 / 2.00; 40 of 2 x 512 x 512 1.51 / 1.56 /
 // 1.79. Frames in device memory: 7.19 ms in groups of 8, 7.34 in groups of 4. Each group has a graph and buffers
-// of its own, made by the first call that has it (50 frames of 16.8 MB, 26 groups of up to 2: first call 46 ms, 51 in
+// of its own, made by the first call that has it (50 frames of 16.8 MB, 26 groups of up to 2: first call 45 ms, 51 in
 // groups of 8; the slots are most of it), so that there are at most kMostGroups, whatever the number of frames.
 int host_group_frames(size_t raw_bytes, int n) {
   constexpr size_t kUpload = (size_t)32 << 20;

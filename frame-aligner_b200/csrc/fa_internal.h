@@ -48,7 +48,7 @@ enum Phase : int {
   kPhaseDone = 3,
   kPhaseStartLast = 4,   // trial = an earlier frame's solution (warm start)
   kPhaseWaitWarm = 5,    // cold starting points done; out of the passes until the warm-start vector
-                         // has been written (resumed by the compact pass)
+                         // has been written (resumed where the next active list is built)
   kPhaseStartPair = 6    // both cold starting points in one pass: zero (dparams, partials) and the
                          // rigid shift (dparams2, partials2); persistent fused pass only
 };

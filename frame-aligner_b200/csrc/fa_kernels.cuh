@@ -17,10 +17,14 @@ constexpr int kSolveThreads = 256;
 
 // Passes and steps of few tiles may start while their predecessor on the stream still runs (programmatic
 // dependent launch): the kernel itself waits (cudaGridDependencySynchronize) before it touches what the
-// predecessor writes. A kernel that waits holds SMs (a step's CTA a whole one), so this is for solves that
-// have the device to themselves. One B200, a single-frame solve of an FP32 512 plane: 235 us without, 202
-// with; 20 frames of 256 x 256 (two groups that fit the device together) 717 and 657 us; 42 of 256 x 64 x 8
-// (five groups that do not) 594 and 681 (600 when the successor is let in late).
+// predecessor writes. A kernel that waits holds SMs (a step's CTA a whole one). One B200, without / with:
+// - single-frame calls always do; it pays beside other threads' calls too. FP32 512 x 512 solves, a frame per
+//   thread: one thread 11.0k / 14.1k a second, three 23.3k / 31k, eight 45.5k / 57k; evaluations 35.5k / 38.5k
+//   and, with eight threads, 82k either way; correlations of 512 x 512 x 16 9.5k / 10.4k, with four 13.9k / 14.0k.
+// - a batch does where the groups of its call fit the device together: 20 frames of 256 x 256 (two groups) 717
+//   and 657 us; 42 of 256 x 64 x 8 (five groups that do not fit) 594 and 681 (600 when the successor is let in
+//   late). The rule does not know of other threads: one aligner with those 20 frames makes 3.3k / 3.5k calls a
+//   second, two at once 5.8k / 5.5k, four 9.7k / 8.4k.
 template <typename... P, typename... A>
 inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool overlap,
                                 A... args) {
@@ -163,8 +167,8 @@ cudaError_t launch_warp(const RefDev* ref_dev, const RefDev& ref_host, const voi
 
 // One trust-region step for each job (grid = n_jobs): reduce partials, advance the state machine,
 // solve the next subproblem, write the next trial point's dparams. With an active list, block b
-// serves jobs[active[b]] for b < *n_active. max_nD / n_dim size the shared-memory staging (frames
-// above about 200 KB work in global memory). With `next`, the last CTA to finish builds the next active
+// serves jobs[active[b]] for b < *n_active. max_nD / n_dim size the shared-memory staging (launches
+// whose largest frame wants more than 200 KB work in global memory). With `next`, the last CTA to finish builds the next active
 // list there (its list and length must not be `active` and `n_active`, which the launch's other CTAs may
 // still read; `finished` counts them and is zero between launches), and with end_of_round it also
 // controls the loop. overlap: of a step directly after a pass of the same overlap.
@@ -267,7 +271,7 @@ cudaError_t launch_plane_rows_fwd(const PlaneDims& d, const FramePtrs& vols, int
 // Per plane: forward DFT over (z, y), then either out = conj (reference) or, in place,
 // out = inverse DFT of the normalised cross-power spectrum with ref_conj. With `overlap` each pass
 // stages its twiddles while the pass before it in the stream drains (that pass has to be one of
-// these); for calls that have the device to themselves.
+// these); see launch_overlapped.
 cudaError_t launch_plane_yz(const PlaneDims& d, const double2* in, double2* out, const double2* ref_conj,
                             const double2* tw_y, int batch, bool reference, cudaStream_t s, bool overlap = false);
 // The same for split dimensions (d.split), in place in spec: forward DFT of every y line, then per

@@ -266,7 +266,7 @@ fa_status correlator_plans(fa_correlator* C, int batch, cufftHandle* fwd, cufftH
 // With `slots` (n interior pointers of frame slots of `slot_kind` with the given pitch and plane),
 // the plane path also writes each frame + 1 into its slot as it reads it (*slots_written = true);
 // on the cuFFT path it does not, and the caller converts the frames itself. peaks may be page-locked
-// host memory. alone: nothing else uses the device, so the passes may overlap their launches.
+// host memory. alone: the call's only work, so the passes overlap their launches (launch_overlapped).
 fa_status correlator_enqueue(fa_correlator* C, const void* const* vols, int in_kind, int n,
                              double* surface = nullptr, bool planes = true, int first = 0,
                              void* const* slots = nullptr, int slot_kind = 0, int slot_pitch = 0,

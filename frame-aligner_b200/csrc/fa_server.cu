@@ -7,8 +7,8 @@
 // slot memory fits the server's budget, then upload, convert (+1 offset) and phase-correlate on the
 // acquisition's own stream. Per class of frames that can share a kernel (dimensionality, slot
 // storage, reference precision, row width a multiple of 4): a job table of max_in_flight entries, a
-// CUDA graph of iterations_per_launch x (compact, fused pass, trust-region step) + compact, and a
-// stream. Between graph launches newly correlated frames are activated (device-side zero start),
+// CUDA graph (the active list, then iterations_per_launch x (fused pass, trust-region step), whose last
+// CTA builds the next list) and a stream. Between graph launches newly correlated frames are activated (device-side zero start),
 // finished frames are read from host-mapped reports and their slots reused; host callbacks on the
 // streams wake the worker, so uploads and correlations of new frames overlap the solves of others.
 //
