@@ -2016,6 +2016,20 @@ BatchCache* aligner_batch_cache(fa_aligner* A, int first, int n) {
   return found;
 }
 
+// Gives back what is kept for ranges that this call does not use; false when there is nothing.
+bool aligner_drop_unused(fa_aligner* A) {
+  const size_t had = A->batch_cache.size();
+  for (auto it = A->batch_cache.begin(); it != A->batch_cache.end();) {
+    if (it->used != A->calls) {
+      batch_cache_release(A->ctx, &*it);
+      it = A->batch_cache.erase(it);
+    } else {
+      ++it;
+    }
+  }
+  return A->batch_cache.size() < had;
+}
+
 // Solve groups of one call, as frame boundaries {0, ..., n}: groups of `chunk` frames (a last
 // remainder under chunk / 2 joins the group before it). Every group's solve is queued on its own
 // stream behind its own peaks, so the solves of the first groups run while the later groups upload
@@ -2164,6 +2178,8 @@ fa_status aligner_run(fa_aligner* A, const void* const* frames, fa_dtype dtype, 
     const PeakStart ps{C->d_idx + g0, C->nx, C->ny, C->nz, A->prm.spatial_binning, A->group_ev[g]};
     const int before = cache[g]->captures;
     r = align_batch_enqueue(batch.data() + g0, g1 - g0, nullptr, A->prm.max_iterations, nullptr, cache[g], &ps, alone);
+    if (r == FA_ERR_OOM && aligner_drop_unused(A))  // (its buffers are allocated before anything is queued)
+      r = align_batch_enqueue(batch.data() + g0, g1 - g0, nullptr, A->prm.max_iterations, nullptr, cache[g], &ps, alone);
     A->graphs_captured += cache[g]->captures - before;
     // the last group's stream also holds whatever its failed enqueue left queued
     queued = g + 1;

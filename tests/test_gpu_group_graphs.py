@@ -57,3 +57,43 @@ def test_graphs_kept_are_bounded():
     assert np.array_equal(device(200), want)
     assert al.graphs()[1] <= 128
     al.close()
+
+
+def test_kept_graphs_do_not_exhaust_the_budget():
+    """With the smallest memory budget that a call of 40 frames fits, calls of fewer frames fit too: what is
+    kept for other ranges is given back."""
+    import torch
+
+    shape, nD = (1, 32, 64), 4
+    acq = S.make_acquisition(shape, nD, 2, S.BlobSpec(40, (2.0, 6.0), (1.0, 2.0), mean=20.0),
+                             S.WalkSpec(1.0, 3.0, 0.0, 0.0), seed=73)
+    line, il, ifr = acq.scan
+    dev = torch.from_numpy(np.ascontiguousarray(acq.frames.astype(np.uint16)).view(np.int16)).to("cuda:0")
+    torch.cuda.synchronize()
+
+    def aligner(budget):
+        al = fa.Aligner(fa.Context(memory_budget=budget), nD=nD, precision=fa.PREC_MIXED)
+        al.set_reference(acq.reference, fa.scan_params(line, il, ifr, 64, 32, 1))
+        return al
+
+    def call(al, n):
+        return al.add_frames_device([dev[k % 2].data_ptr() for k in range(n)], fa.U16, n)[0]
+
+    def fits(budget):
+        try:
+            call(aligner(budget), 40)
+            return True
+        except fa.FaError as e:
+            assert e.status == fa.FA_ERR_OOM
+            return False
+
+    lo, hi = 1 << 12, 1 << 28
+    assert fits(hi)
+    while hi - lo > 64:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if fits(mid) else (mid, hi)
+    al = aligner(hi)
+    want = call(al, 40)
+    for n in (39, 36, 33, 20, 7, 1, 40, 12, 40):
+        assert np.array_equal(call(al, n), want[:n]), n
+    al.close()
